@@ -101,14 +101,16 @@ __global__ void __launch_bounds__(256) panel_i8_kernel(const float *__restrict__
 // blocks, four units a block and round, whose sums of squares meet in shared
 // memory.  (The row is read before the blocks meet and written after, by the
 // threads that read it: xout may be x.)  A single block per token took 13 us for
-// rows of 5120; a decoder layer with two norms became 16 us shorter.
+// rows of 5120; a decoder layer with two norms became 16 us shorter.  The cluster's
+// first meeting, which says that the peers run, has the row's loads between its halves.
 constexpr int NORM_CLUSTER = 8;
 template <int P>
 __global__ void __launch_bounds__(1024) normalize_i8_kernel(const float *x, const float *__restrict__ weight, float eps, float *xout,
                                                             size_t cols, int n, uint8_t *__restrict__ panels) {
+    const int t = blockIdx.y, rank = blockIdx.x, ranks = gridDim.x;
+    if (ranks > 1) cluster_arrive();
     griddep_launch();
     griddep_wait();
-    const int t = blockIdx.y, rank = blockIdx.x, ranks = gridDim.x;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, j = warp & 7, uu = tid >> 8;
     __shared__ float part[32];
     __shared__ float sums[NORM_CLUSTER];
@@ -124,6 +126,7 @@ __global__ void __launch_bounds__(1024) normalize_i8_kernel(const float *x, cons
     float total = warp_sum(part[lane]);
     if (ranks > 1) {
         // every block's sum to every block, added in rank order
+        cluster_wait();                     // all of them run
         if (warp == 0 && lane < ranks) st_cluster_f32(smem_u32(sums + rank), lane, total);
         cluster_sync();
         total = sums[0];

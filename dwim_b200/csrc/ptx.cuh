@@ -92,9 +92,15 @@ __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wa
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Thread-block clusters: all threads of the cluster meet (what they wrote to shared memory before is
-// visible to the others after), and loads and stores of another block's shared memory (`addr` as in this block).
+// visible to the others after), at once or in two halves; and loads and stores of another block's shared
+// memory (`addr` as in this block).  The blocks of a cluster are scheduled together, but a block may reach
+// into another only once that one has started, and only until it ends: the cluster meets before the first
+// access to a peer and after the last.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_arrive();
+    cluster_wait();
 }
 __device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, int rank) {
     uint32_t r;

@@ -1,0 +1,52 @@
+"""Rules of the hardware that the kernels' sources must keep, read from the sources.
+
+A breach of these is undefined behaviour that timing can hide on every run, so that no result shows it:
+they are checked where the code is, without a GPU.
+"""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "dwim_b200", "csrc")
+SOURCES = sorted(f for f in os.listdir(CSRC) if f.endswith(".cu"))
+
+# what reaches another block's shared memory, and what proves that the block is there (ptx.cuh)
+REMOTE = re.compile(r"\b(?:st_cluster_f32|ld_cluster_f32|cluster_addr)\s*\(")
+MET = re.compile(r"\b(?:cluster_sync|cluster_wait)\s*\(")
+
+
+def source(name):
+    """A source file without its comments."""
+    text = open(os.path.join(CSRC, name)).read()
+    return re.sub(r"//[^\n]*|/\*.*?\*/", "", text, flags=re.S)
+
+
+def kernels(text):
+    """(name, body) of every __global__ function."""
+    for m in re.finditer(r"__global__", text):
+        at = text.index("{", m.start())
+        name = re.findall(r"(\w+)\s*\(", text[m.start():at])[-1]
+        depth, end = 0, at
+        while True:
+            depth += {"{": 1, "}": -1}.get(text[end], 0)
+            end += 1
+            if depth == 0:
+                break
+        yield name, text[at:end]
+
+
+def test_every_kernel_is_found():
+    names = [name for f in SOURCES for name, _ in kernels(source(f))]
+    assert {"normalize_i8_kernel", "matmul_bf16_tile_kernel", "gemm_q4k_kernel", "gemm_dense_kernel", "dwim_smallm_kernel"} <= set(names)
+
+
+@pytest.mark.parametrize("name", SOURCES)
+def test_a_cluster_meets_before_its_blocks_reach_each_other(name):
+    """A block may touch another's shared memory once that block is known to run: after a barrier of the cluster
+    (being scheduled together is not having started)."""
+    for kernel, body in kernels(source(name)):
+        remote = REMOTE.search(body)
+        if remote:
+            met = MET.search(body)
+            assert met and met.start() < remote.start(), f"{kernel}: a remote access ahead of the cluster's first meeting"
