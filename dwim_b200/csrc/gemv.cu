@@ -149,9 +149,10 @@ __device__ __forceinline__ float lds32f(uint32_t a) {
 // of the MMA (8 columns each).  Tile p's column g is blob column
 // p*tile_stride + g, present when g < tile_cols.
 //   one and two tokens:  one tile, column = 4*token + plane, tile_cols = 4n
-//   three to five:       two tiles, the blob's 3n columns eight by eight (plane p of token t is column
-//                        p*n + t): a third fewer MMAs and multiplies than a tile per plane ([17408, 5120]
-//                        Q4_K by five tokens 25.0 us, 21.4 like this); a token's planes meet after the K-split sums
+//   three to five:       two tiles, the first eight of the blob's 3n columns and the last eight, so that
+//                        neither reads past them (plane p of token t is column p*n + t): a third fewer MMAs
+//                        and multiplies than a tile per plane ([17408, 5120] Q4_K by five tokens 25.0 us,
+//                        21.4 like this); a token's planes meet after the K-split sums
 //   six to eight:        a tile per plane, column g = token g, tile_stride = tile_cols = n
 // In all a lane's accumulators are (row a | row b) x (tile column 2c, 2c+1).
 // One token of Q6_K fills half a tile, so its columns 4..7 take a second scale group: B is block
@@ -162,9 +163,26 @@ struct I8Cols {
     int nc;           // columns in a unit's blob
     int tile_stride;
     int tile_cols;
-    // the column a lane's B fragment comes from: the sums of columns that are not there are not used
-    __device__ __forceinline__ int lane_col(int g) const { return g < tile_cols ? g : 0; }
+    // the column a lane's B fragment of tile 0 comes from: the sums of columns that are not there are not used
+    __host__ __device__ constexpr int lane_col(int g) const { return g < tile_cols ? g : 0; }
 };
+template <int NTILE> __host__ __device__ constexpr I8Cols i8_cols(int nc, int n_tokens) {
+    return I8Cols{nc, NTILE == 1 ? 0 : NTILE == 2 ? nc - 8 : n_tokens, NTILE == 1 ? nc : NTILE == 2 ? 8 : n_tokens};
+}
+// Column tiles of n tokens (of any format): one (4 planes x 1-2 tokens), two (3 planes x 3-5 tokens), one per plane.
+__host__ __device__ constexpr int i8_tiles(int n) { return n <= 2 ? 1 : n <= 5 ? 2 : 3; }
+// Every lane's column of every tile is one of the blob's.
+template <int NTILE> constexpr bool i8_columns_exist() {
+    for (int n = 1; n <= I8_MAX_TOKENS; n++) {
+        if (i8_tiles(n) != NTILE) continue;
+        const I8Cols X = i8_cols<NTILE>(i8_planes(n) * n, n);
+        for (int g = 0; g < 8; g++)
+            for (int p = 0; p < NTILE; p++)
+                if (X.lane_col(g) + p * X.tile_stride >= X.nc) return false;
+    }
+    return true;
+}
+static_assert(i8_columns_exist<1>() && i8_columns_exist<2>() && i8_columns_exist<3>(), "a lane reads past a unit's planes");
 
 // Q4_K.  Lane (g, c) owns bytes [8c, 8c+8) of each 32-byte group of its two rows: MMA
 // k-slots 4c..4c+3 and 16+4c..16+4c+3, matched by the same eight digits of the
@@ -233,7 +251,7 @@ __device__ __forceinline__ void unit_q4k_i8(const Lane &L, const I8Cols X, int u
                 uint4 t = make_uint4(0, 0, 0, 0);
                 float worth = 0.0f;
                 const int col = p * X.tile_stride + 2 * L.c + i;
-                if (NTILE == 2 ? col < X.nc : 2 * L.c + i < X.tile_cols) {
+                if (NTILE == 2 || 2 * L.c + i < X.tile_cols) {
                     t = lds128(blob + 256 * X.nc + col * 16);
                     worth = lds32f(blob + 272 * X.nc + 4 * col);
                 }
@@ -284,7 +302,7 @@ __device__ __forceinline__ void unit_q8_i8(const Lane &L, const I8Cols X, int ul
         for (int i = 0; i < 2; i++) {
             float worth = 0.0f;
             const int col = p * X.tile_stride + 2 * L.c + i;
-            if (NTILE == 2 ? col < X.nc : 2 * L.c + i < X.tile_cols) worth = lds32f(blob + 272 * X.nc + 4 * col);
+            if (NTILE == 2 || 2 * L.c + i < X.tile_cols) worth = lds32f(blob + 272 * X.nc + 4 * col);
             acc[(NTILE == 2 ? 4 * p : 0) + i] += worth * fs[p][i];
             acc[(NTILE == 2 ? 4 * p : 0) + 2 + i] += worth * fs[p][2 + i];
         }
@@ -395,7 +413,7 @@ __device__ __forceinline__ void unit_q6k_i8(const Lane &L, const I8Cols X, int u
         for (int i = 0; i < 2; i++) {
             float worth = 0.0f;
             const int col = p * X.tile_stride + 2 * L.c + i;
-            if (NTILE == 2 ? col < X.nc : 2 * L.c + i < X.tile_cols) worth = lds32f(blob + 272 * X.nc + 4 * col);
+            if (NTILE == 2 || 2 * L.c + i < X.tile_cols) worth = lds32f(blob + 272 * X.nc + 4 * col);
             acc[(NTILE == 2 ? 4 * p : 0) + i] += worth * (da * (float)is[p][i]);
             acc[(NTILE == 2 ? 4 * p : 0) + 2 + i] += worth * (db * (float)is[p][2 + i]);
         }
@@ -589,7 +607,7 @@ __global__ void __launch_bounds__((RT * KS + 1) * 32, 1) dwim_smallm_kernel(cons
     const int grow = (FMT == Q4K_I8 || FMT == Q8_I8) ? ((L.g & 3) * 2 + (L.g >> 2)) : L.g;
     // the digit planes' columns: one tile of 4n columns (one and two tokens), or a tile of n columns per plane
     constexpr bool ONE = NT == 0, PACKED = NT <= 1;
-    const I8Cols X = {a.ncols, PACKED ? 0 : NT == 2 ? 8 : a.n_tokens, PACKED ? a.ncols : NT == 2 ? 8 : a.n_tokens};
+    const I8Cols X = i8_cols<PACKED ? 1 : NT>(a.ncols, a.n_tokens);
 
     uint32_t it = 0;
     int tile_parity = 0;
@@ -671,8 +689,8 @@ __global__ void __launch_bounds__((RT * KS + 1) * 32, 1) dwim_smallm_kernel(cons
                 emit(a, t0 + t, r1, n_mats == 2 ? silu_mul(gate[2], vb) : vb);
             }
         } else if constexpr (NT == 2) {
-            // Lane c of a row's four finishes tokens c and c + 4: their planes' columns are p*n + t, column
-            // col in lane (col & 7) >> 1, tile col >> 3, the even or odd one of its pair.
+            // Lane c of a row's four finishes tokens c and c + 4: their planes' columns are p*n + t; a tile's
+            // column i is in lane i >> 1, the even or odd one of its pair.
             float v[4];
 #pragma unroll
             for (int s = 0; s < 2; s++) {
@@ -680,12 +698,13 @@ __global__ void __launch_bounds__((RT * KS + 1) * 32, 1) dwim_smallm_kernel(cons
                 v[s] = v[2 + s] = 0.0f;
 #pragma unroll
                 for (int p = 0; p < 3; p++) {
-                    const int col = t < a.n_tokens ? p * a.n_tokens + t : 0, from = (lane & ~3) | ((col & 7) >> 1);
+                    const int col = t < a.n_tokens ? p * a.n_tokens + t : 0, i2 = col < 8 ? col : col - X.tile_stride;
+                    const int from = (lane & ~3) | (i2 >> 1);
                     float x[8];
 #pragma unroll
                     for (int i = 0; i < 8; i++) x[i] = __shfl_sync(0xffffffffu, acc[i], from);
-                    const float ra = col < 8 ? ((col & 1) ? x[1] : x[0]) : ((col & 1) ? x[5] : x[4]);
-                    const float rb = col < 8 ? ((col & 1) ? x[3] : x[2]) : ((col & 1) ? x[7] : x[6]);
+                    const float ra = col < 8 ? ((i2 & 1) ? x[1] : x[0]) : ((i2 & 1) ? x[5] : x[4]);
+                    const float rb = col < 8 ? ((i2 & 1) ? x[3] : x[2]) : ((i2 & 1) ? x[7] : x[6]);
                     v[s] += ra;
                     v[2 + s] += rb;
                 }
@@ -914,8 +933,7 @@ int gemv_small_i8(dwim_b200_ctx *ctx, const WeightView &w, const uint8_t *panels
         a.up_scales = up->scales;
     }
     a.status = ctx->status;
-    // one column tile (4 planes x 1-2 tokens), two (3 planes x 3-5 tokens), or one per plane (3 planes)
-    const int tiles = n_tokens <= 2 ? 1 : n_tokens <= 5 ? 2 : 3;
+    const int tiles = i8_tiles(n_tokens);
     switch (w.fmt) {
     case Q4_K: return tiles == 1 ? launch_shape<Q4K_I8, 1>(ctx, a) : tiles == 2 ? launch_shape<Q4K_I8, 2>(ctx, a) : launch_shape<Q4K_I8, 3>(ctx, a);
     case Q8_0: return tiles == 1 ? launch_shape<Q8_I8, 1>(ctx, a) : tiles == 2 ? launch_shape<Q8_I8, 2>(ctx, a) : launch_shape<Q8_I8, 3>(ctx, a);
