@@ -23,6 +23,19 @@ namespace dwim {
 bool gemm_supports(const WeightView &w);
 int gemm_large(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, size_t n, int split, const OutSpec &out,
                const float *aux, int epilogue);
+
+int reserve_shadow(dwim_b200_ctx *ctx, dwim_b200_buffer *b, size_t need) {
+    if (need <= b->shadow_cap) return 0;
+    if (b->shadow) {
+        DWIM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        cudaFree(b->shadow);
+        b->shadow = nullptr;
+        b->shadow_cap = 0;
+    }
+    DWIM_CUDA(ctx, cudaMalloc(&b->shadow, need));
+    b->shadow_cap = need;
+    return 0;
+}
 }  // namespace dwim
 
 extern "C" {
@@ -299,6 +312,7 @@ int dwim_b200_buffer_free(dwim_b200_ctx *ctx, dwim_b200_buffer *buf) {
     if (buf->sh_world) shared_release(buf);
     if (buf->owned && buf->data) cudaFree(buf->data);
     if (buf->shadow) cudaFree(buf->shadow);
+    if (buf->groups) cudaFree(buf->groups);
     delete buf;
     return 0;
 }
@@ -446,24 +460,39 @@ static int ensure_shadow(dwim_b200_ctx *ctx, dwim_b200_buffer *x, int kind, size
     if (x->shadow_kind == kind && x->shadow_cols == cols && x->shadow_split == split) return 0;
     size_t n = x->len / cols;
     size_t need = kind == SHADOW_GEMM ? gemm_operand_bytes(cols, n, split) : panel_i8_bytes(cols, n);
-    if (need > x->shadow_cap) {
-        if (x->shadow) {
-            DWIM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            cudaFree(x->shadow);
-            x->shadow = nullptr;
-            x->shadow_cap = 0;
-        }
-        DWIM_CUDA(ctx, cudaMalloc(&x->shadow, need));
-        x->shadow_cap = need;
-    }
+    int rc = reserve_shadow(ctx, x, need);
+    if (rc) return rc;
     x->shadow_kind = SHADOW_NONE;
-    int rc = kind == SHADOW_GEMM ? build_gemm_operand(ctx, x->data, n, cols, split, (__half *)x->shadow)
-                                 : build_panels_i8(ctx, x->data, n, cols, (uint8_t *)x->shadow);
+    rc = kind == SHADOW_GEMM ? build_gemm_operand(ctx, x->data, n, cols, split, (__half *)x->shadow)
+                             : build_panels_i8(ctx, x->data, n, cols, (uint8_t *)x->shadow);
     if (rc) return rc;
     x->shadow_kind = kind;
     x->shadow_cols = cols;
     x->shadow_split = split;
     return 0;
+}
+
+constexpr size_t GROUPS_AT_ONCE = 64;
+
+// Room for the digit planes of all the groups of eight tokens that `x` can hold, up to GROUPS_AT_ONCE.  It spares
+// launches and no product needs it: it is never made anew at another length of the buffer (a graph captured at one
+// length may still read it), not allocated under a stream capture, and done without when memory is short.
+static void reserve_groups(dwim_b200_ctx *ctx, dwim_b200_buffer *x, size_t cols, size_t group) {
+    size_t most = x->cap / cols / I8_MAX_TOKENS;
+    if (most > GROUPS_AT_ONCE) most = GROUPS_AT_ONCE;
+    if (x->groups_tried || most < 2) return;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return;
+    }
+    x->groups_tried = true;
+    if (cudaMalloc(&x->groups, most * group) == cudaSuccess) {
+        x->groups_cap = most * group;
+    } else {
+        x->groups = nullptr;
+        cudaGetLastError();
+    }
 }
 
 static int product(dwim_b200_ctx *ctx, const OutSpec &out, size_t out_len, const dwim_b200_weight *w, dwim_b200_buffer *x,
@@ -500,28 +529,25 @@ static int product(dwim_b200_ctx *ctx, const OutSpec &out, size_t out_len, const
         if (rc) return rc;
         return gemv_small_i8(ctx, v, (const uint8_t *)x->shadow, (int)n, 0, out, aux, epilogue);
     }
-    // Groups of eight tokens, each with its own digit planes: full groups in one launch, up to
-    // GROUPS_AT_ONCE of them (a group's blocks start as the one before runs out of tiles, and its weights
-    // come from L2), then what is left.  [5120, 5120] Q8_0 by 48 tokens: six pairs of launches 101 us, like this 51.
-    constexpr size_t GROUPS_AT_ONCE = 64;
-    const size_t groups = n / I8_MAX_TOKENS < GROUPS_AT_ONCE ? n / I8_MAX_TOKENS : GROUPS_AT_ONCE;
-    const size_t need = groups * panel_i8_bytes(v.cols, I8_MAX_TOKENS);
-    if (need > x->shadow_cap) {
-        if (x->shadow) {
-            DWIM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            cudaFree(x->shadow);
-            x->shadow = nullptr;
-            x->shadow_cap = 0;
-        }
-        DWIM_CUDA(ctx, cudaMalloc(&x->shadow, need));
-        x->shadow_cap = need;
+    // Groups of eight tokens, each with its own digit planes: full groups in one launch, as many as there is
+    // room for (a group's blocks start as the one before runs out of tiles, and its weights come from L2), then
+    // what is left.  [5120, 5120] Q8_0 by 48 tokens: six pairs of launches 101 us, like this 51.
+    const size_t group = panel_i8_bytes(v.cols, I8_MAX_TOKENS);
+    int rc = reserve_shadow(ctx, x, group);
+    if (rc) return rc;
+    size_t groups = n / I8_MAX_TOKENS < GROUPS_AT_ONCE ? n / I8_MAX_TOKENS : GROUPS_AT_ONCE;
+    if (groups * group > x->shadow_cap) {
+        reserve_groups(ctx, x, v.cols, group);
+        const size_t room = (x->groups_cap > x->shadow_cap ? x->groups_cap : x->shadow_cap) / group;
+        if (groups > room) groups = room;
     }
-    x->shadow_kind = SHADOW_NONE;
+    uint8_t *const panels = (uint8_t *)(groups * group > x->shadow_cap ? x->groups : x->shadow);
+    if (panels == x->shadow) x->shadow_kind = SHADOW_NONE;
     for (size_t t0 = 0; t0 < n;) {
         const size_t left = n - t0, g = left < (size_t)I8_MAX_TOKENS ? 1 : left / I8_MAX_TOKENS < groups ? left / I8_MAX_TOKENS : groups;
         const size_t nt = left < (size_t)I8_MAX_TOKENS ? left : (size_t)I8_MAX_TOKENS;
-        int rc = build_panels_i8(ctx, x->data + t0 * v.cols, nt, v.cols, (uint8_t *)x->shadow, nullptr, 0.0f, nullptr, g);
-        if (rc == 0) rc = gemv_small_i8(ctx, v, (const uint8_t *)x->shadow, (int)nt, t0, out, aux, epilogue, nullptr, g);
+        rc = build_panels_i8(ctx, x->data + t0 * v.cols, nt, v.cols, panels, nullptr, 0.0f, nullptr, g);
+        if (rc == 0) rc = gemv_small_i8(ctx, v, panels, (int)nt, t0, out, aux, epilogue, nullptr, g);
         if (rc) return rc;
         t0 += g * nt;
     }

@@ -40,6 +40,11 @@ struct dwim_b200_buffer {
     int shadow_kind = SHADOW_NONE;
     size_t shadow_cols = 0;      // K the shadow was built for
     int shadow_split = 0;        // 1: hi/lo column pairs, 0: single f16
+    // The digit planes of several groups of eight tokens (products of Q6_K and Q8_0 by nine tokens and more),
+    // where the shadow holds fewer.  Allocated once and kept to the buffer's end.
+    void *groups = nullptr;
+    size_t groups_cap = 0;       // bytes
+    bool groups_tried = false;
 };
 
 struct dwim_b200_weight {
@@ -208,6 +213,9 @@ int gemv_small_i8(dwim_b200_ctx *ctx, const WeightView &w, const uint8_t *panels
                   const float *aux, int epilogue, const WeightView *up = nullptr, size_t groups = 1);
 void peer_release(dwim_b200_ctx *ctx);
 void shared_release(dwim_b200_buffer *buf);
+// abi.cu
+// The buffer's shadow made at least `need` bytes long (a longer one takes the place of the old).
+int reserve_shadow(dwim_b200_ctx *ctx, dwim_b200_buffer *b, size_t need);
 // neighbours.cu
 int matmul_bf16(dwim_b200_ctx *ctx, const WeightView &w, const float *x, size_t n, const OutSpec &out, const float *aux, int epi);
 // static_scratch.cu

@@ -261,19 +261,6 @@ __global__ void __launch_bounds__(256) argmax_kernel(const float *__restrict__ l
     }
 }
 
-int reserve_shadow(dwim_b200_ctx *ctx, dwim_b200_buffer *b, size_t need) {
-    if (need <= b->shadow_cap) return 0;
-    if (b->shadow) {
-        DWIM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        cudaFree(b->shadow);
-        b->shadow = nullptr;
-        b->shadow_cap = 0;
-    }
-    DWIM_CUDA(ctx, cudaMalloc(&b->shadow, need));
-    b->shadow_cap = need;
-    return 0;
-}
-
 }  // namespace
 
 namespace dwim {

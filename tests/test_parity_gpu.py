@@ -235,6 +235,57 @@ def test_groups_of_eight_tokens(dev, oracle, fmt, rows, cols, n):
     assert np.abs(dev.read(acc).reshape(n, rows) - (want + res)).max() <= bar + 1e-6
 
 
+def test_groups_under_capture(oracle):
+    """A product of more than eight tokens captured into a CUDA graph after a warm-up at another token count
+    (the buffer resized between): no allocation is needed there, and none made later takes away what a captured
+    graph reads.  Every token as the eager product gives it."""
+    import torch
+    from dwim_b200 import B200, Tensor
+    stream = torch.cuda.Stream()
+    d = B200(0, stream=stream.cuda_stream)
+    try:
+        rng = np.random.default_rng(71)
+        rows, cols, most = 96, 2048, 48
+        blocks = oracle.quantize("q8_0", (0.02 * rng.standard_normal((rows, cols))).astype(np.float32))
+        weight = d.upload(Tensor("q8_0", (rows, cols), blocks))
+        x = rng.standard_normal((most, cols)).astype(np.float32)
+        want = oracle.matmul("q8_0", blocks, rows, cols, x).reshape(most, rows)
+        xb, out = d.buffer(x), d.alloc(most * rows)
+
+        def at(n):
+            d.resize(xb, n * cols)
+            d.resize(out, n * rows)
+
+        def right(n):
+            got = d.read(out).reshape(n, rows)
+            d.write(out, np.zeros(n * rows, np.float32))
+            return max_rel_err(got, want[:n]) <= 2e-5
+
+        def captured(n):
+            at(n)
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                d.matmul(out, weight, xb)
+            return graph
+
+        at(8)
+        d.matmul(out, weight, xb)
+        assert right(8)
+        graphs = {n: captured(n) for n in (most, 16)}
+        at(most)
+        d.matmul(out, weight, xb)                       # eager: the planes of all its groups at once
+        assert right(most)
+        graphs[24] = captured(24)
+        for n, graph in list(graphs.items()) * 2:
+            at(n)
+            with torch.cuda.stream(stream):
+                graph.replay()
+            assert right(n), n
+        del graphs
+    finally:
+        d.close()
+
+
 @pytest.mark.parametrize("bf16", [False, True])
 def test_q4_k_gemm_scale_extremes(dev, oracle, bf16):
     """The tensor-core kernel folds a block's minimums into the same accumulator
