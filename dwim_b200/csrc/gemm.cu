@@ -48,6 +48,7 @@
 #include <cuda.h>
 #include <stdlib.h>
 
+#include <atomic>
 
 #include "common.cuh"
 #include "ptx.cuh"
@@ -1021,7 +1022,7 @@ typedef CUresult (*EncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, 
                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 EncodeTiled encode_fn() {
-    static EncodeTiled fn = [] {
+    static const EncodeTiled fn = [] {
         void *p = nullptr;
         cudaDriverEntryPointQueryResult q;
         if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
@@ -1057,14 +1058,15 @@ namespace {
 struct SplitCost {
     double tile, shared;      // what a tile costs besides its units: alone, shared
 };
+// known: clusters of so many blocks that a device holds at once (0: not asked yet); contexts of several threads share it.
 template <typename Kernel, typename Fits>
-int pick_split(dwim_b200_ctx *ctx, Kernel kern, int threads, size_t smem, Fits fits, SplitCost cost, int (&known)[64][MAX_SPLIT + 1], long tiles,
-               int units, double *time = nullptr) {
+int pick_split(dwim_b200_ctx *ctx, Kernel kern, int threads, size_t smem, Fits fits, SplitCost cost,
+               std::atomic<int> (&known)[64][MAX_SPLIT + 1], long tiles, int units, double *time = nullptr) {
     int best = 1;
     double t_best = 0;
     for (int s = 1; s <= MAX_SPLIT && s <= units; s++) {
         if (!fits(s)) continue;
-        int &k = known[ctx->device & 63][s];      // clusters of s blocks that the device holds at once
+        int k = known[ctx->device & 63][s];
         if (!k) {
             int n = ctx->sm_count;
             if (s > 1) {
@@ -1084,7 +1086,7 @@ int pick_split(dwim_b200_ctx *ctx, Kernel kern, int threads, size_t smem, Fits f
                     n = 1;
                 }
             }
-            k = n;
+            known[ctx->device & 63][s] = k = n;
         }
         const double t = (double)((tiles + k - 1) / k) * ((units + s - 1) / s + (s > 1 ? cost.shared : cost.tile));
         if (s == 1 || t < 0.97 * t_best) {
@@ -1100,7 +1102,7 @@ int pick_split(dwim_b200_ctx *ctx, Kernel kern, int threads, size_t smem, Fits f
 // (in units on the busiest block).
 template <int BN>
 int gemm_split(dwim_b200_ctx *ctx, const WeightView &w, size_t ncols, double *time = nullptr) {
-    static int known[64][MAX_SPLIT + 1] = {};
+    static std::atomic<int> known[64][MAX_SPLIT + 1] = {};
     const long tiles = (long)((w.rows + TILE_M - 1) / TILE_M) * (long)((ncols + BN - 1) / BN);
     return pick_split(ctx, gemm_q4k_kernel<BN, 0>, GEMM_THREADS, (size_t)Cfg<BN>::SMEM, Cfg<BN>::split_fits, SplitCost{3.0, 6.5}, known, tiles,
                       (int)(w.cols / 256), time);
@@ -1147,7 +1149,7 @@ int launch_gemm(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, 
                 return rc;
     }
     auto kern = shared == 2 ? gemm_q4k_kernel<BN, 2> : shared == 1 ? gemm_q4k_kernel<BN, 1> : gemm_q4k_kernel<BN, 0>;
-    static bool configured[64][3] = {};
+    static std::atomic<bool> configured[64][3] = {};
     if (!configured[ctx->device & 63][shared]) {
         DWIM_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
         configured[ctx->device & 63][shared] = true;
@@ -1183,14 +1185,14 @@ int launch_dense(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand,
     DenseArgs a{w.rows, n, units, split, epi, 1, out, w.scales, w.srow, tok_scale, aux, ctx->status};
     const bool shared = out.world > 1 && !out.scatter_per;
     auto kern = shared ? gemm_dense_kernel<FMT, BN, true> : gemm_dense_kernel<FMT, BN, false>;
-    static bool configured[64][2] = {};
+    static std::atomic<bool> configured[64][2] = {};
     if (!configured[ctx->device & 63][shared]) {
         DWIM_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
         configured[ctx->device & 63][shared] = true;
     }
     dim3 grid((unsigned)((w.rows + TILE_M - 1) / TILE_M), (unsigned)((ncols + BN - 1) / BN));
     if (!shared) {
-        static int known[64][MAX_SPLIT + 1] = {};
+        static std::atomic<int> known[64][MAX_SPLIT + 1] = {};
         a.split_k = pick_split(ctx, kern, GEMM_THREADS, (size_t)C::SMEM, C::split_fits, SplitCost{2.0, 4.5}, known, (long)grid.x * grid.y, (int)units);
         grid.x *= a.split_k;
     }

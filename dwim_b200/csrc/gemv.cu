@@ -33,6 +33,8 @@
 #include <cuda_fp16.h>
 #include <stdlib.h>
 
+#include <atomic>
+
 #include "common.cuh"
 #include "ptx.cuh"
 #include "tmap.cuh"
@@ -834,7 +836,7 @@ static int launch(dwim_b200_ctx *ctx, GemvArgs &a) {
     a.n_tiles = (int)((a.w.rows + R - 1) / R);
     const int smem = fixed + (ALIGN - 128) + pad(a.xres_bytes) + a.stages * a.stage_bytes;
     auto kern = dwim_smallm_kernel<FMT, NT, RT, KS>;
-    static bool configured[64] = {false};   // per instantiation, per device
+    static std::atomic<bool> configured[64] = {};   // per instantiation, per device; contexts of several threads share it
     if (!configured[ctx->device & 63]) {
         DWIM_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT));
         configured[ctx->device & 63] = true;

@@ -1,4 +1,4 @@
-"""Rules of the hardware that the kernels' sources must keep, read from the sources.
+"""Rules of the hardware and of the language that the library's sources must keep, read from the sources.
 
 A breach of these is undefined behaviour that timing can hide on every run, so that no result shows it:
 they are checked where the code is, without a GPU.
@@ -10,6 +10,7 @@ import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "dwim_b200", "csrc")
 SOURCES = sorted(f for f in os.listdir(CSRC) if f.endswith(".cu"))
+HEADERS = sorted(f for f in os.listdir(CSRC) if f.endswith(".cuh"))
 
 # what reaches another block's shared memory, and what proves that the block is there (ptx.cuh)
 REMOTE = re.compile(r"\b(?:st_cluster_f32|ld_cluster_f32|cluster_addr)\s*\(")
@@ -50,3 +51,11 @@ def test_a_cluster_meets_before_its_blocks_reach_each_other(name):
         if remote:
             met = MET.search(body)
             assert met and met.start() < remote.start(), f"{kernel}: a remote access ahead of the cluster's first meeting"
+
+
+@pytest.mark.parametrize("name", SOURCES + HEADERS)
+def test_process_wide_variables_may_be_shared_by_threads(name):
+    """Several threads may drive a context each, so what all contexts share is constant, atomic or a thread's own."""
+    for m in re.finditer(r"\bstatic\s+((?:[\w:]|<[^<>]*>|\s|\*)+?)\s*\b(\w+)\s*(?:\[[^\]]*\]\s*)*(?:=|;|\{)", source(name)):
+        kind = m.group(1)
+        assert re.search(r"\b(const|constexpr|thread_local|__device__)\b|\batomic<", kind), f"{name}: static {kind} {m.group(2)}"
