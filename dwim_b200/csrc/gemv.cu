@@ -746,15 +746,25 @@ __global__ void __launch_bounds__((RT * KS + 1) * 32, 1) dwim_smallm_kernel(cons
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
+// A CTA's shared memory (one CTA per SM): barriers, the K-split warps' sums, then resident planes and stages.
+template <int FMT, int NT, int RT, int KS> struct Smem {
+    static constexpr int LIMIT = 227 * 1024;
+    static constexpr int FIXED = 256 + (KS > 1 ? 2 * KS * RT * (NT == 2 ? 8 : 4) * 32 * 4 : 0);
+    static constexpr int ALIGN = base_of(FMT) == Q8_0 ? 1024 : 128;     // the stages' start is rounded up
+    static constexpr int BUDGET = LIMIT - FIXED - (ALIGN - 128);
+    static int pad(int b) { return (b + ALIGN - 1) & ~(ALIGN - 1); }
+    // bytes of a stage of whole rows without planes
+    static int whole(const GemvArgs &a) { return (int)(16 * RT * (a.w.qpitch + a.w.srow * 2)); }
+    // the planes and two stages of whole rows
+    static bool two_whole_fit(const GemvArgs &a) { return pad(a.units * a.xunit) + 2 * pad(whole(a)) <= BUDGET; }
+};
+
 template <int FMT, int NT, int RT, int KS>
 static int launch(dwim_b200_ctx *ctx, GemvArgs &a) {
     constexpr int R = RT * 16;
     constexpr int UNIT_Q = Traits<FMT>::UNIT_Q;
     constexpr int BASE = base_of(FMT);
-    constexpr int RED_BYTES = KS > 1 ? 2 * KS * RT * (NT == 2 ? 8 : 4) * 32 * 4 : 0;
-    constexpr int SMEM_LIMIT = 227 * 1024;
-    const int SMEM_MAX = SMEM_LIMIT;   // one CTA per SM
-    const int fixed = 256 + RED_BYTES;
+    using S = Smem<FMT, NT, RT, KS>;
     // K per stage.  Whole rows when two stages of them fit: the tile is then one contiguous run of
     // HBM and moves with a single bulk copy (issuing a bulk copy costs the producer on the order of a
     // hundred cycles, so a stage made of one copy per row starves the consumers).  Longer rows are cut
@@ -764,16 +774,14 @@ static int launch(dwim_b200_ctx *ctx, GemvArgs &a) {
     // eight tokens of a 5120-wide row are 132 KB, beside which two whole rows' stages do not fit and
     // three boxes of seven units do (planes that travel with the stages are twice the weights' bytes:
     // the [151936, 5120] head by eight tokens 350 us so, 287 in boxes).
-    auto pad = [](int b) { return (b + (BASE == Q8_0 ? 1023 : 127)) & ~(BASE == Q8_0 ? 1023 : 127); };
+    auto pad = [](int b) { return S::pad(b); };
     const int xall = a.units * a.xunit, srow_bytes = (int)a.w.srow * 2;
-    const int whole = (int)(R * (a.w.qpitch + srow_bytes));
+    const int whole = S::whole(a);
     // odd: a box of 256 elements of 8 bytes; Q8_0: a lane for each half unit and one for the scales
     constexpr int MAX_BOX = BASE == Q8_0 ? 15 : (2048 / UNIT_Q - 1) / 2 * 2 + 1;
-    constexpr int ALIGN = BASE == Q8_0 ? 1024 : 128;
     auto box_units = [&](int chunks) { return ((a.units + chunks - 1) / chunks) | 1; };
-    const int whole_budget = SMEM_MAX - fixed - (ALIGN - 128);   // the stages' start is rounded up
-    a.x_resident = xall <= 80 * 1024 || pad(xall) + 2 * pad(whole) <= whole_budget;
-    a.whole_rows = 2 * pad(whole + (a.x_resident ? 0 : xall)) <= whole_budget - (a.x_resident ? pad(xall) : 0);
+    a.x_resident = xall <= 80 * 1024 || S::two_whole_fit(a);
+    a.whole_rows = 2 * pad(whole + (a.x_resident ? 0 : xall)) <= S::BUDGET - (a.x_resident ? pad(xall) : 0);
     a.boxed = 0;
     // scale bytes of a row in a box's stage: Q8_0's own box, Q6_K's whole row
     auto box_scales = [&](int kc) { return BASE == Q8_0 ? kc * 16 : srow_bytes; };
@@ -781,12 +789,12 @@ static int launch(dwim_b200_ctx *ctx, GemvArgs &a) {
         // the fewest chunks that a box takes and of which three stages fit (two where planes travel with them)
         for (int pass = 0; pass < 2 && !a.boxed; pass++) {
             const int resident = pass == 0, want = resident ? 3 : 2;
-            if (resident && pad(xall) + 3 * pad(R * (UNIT_Q + box_scales(1))) > whole_budget) continue;
+            if (resident && pad(xall) + 3 * pad(R * (UNIT_Q + box_scales(1))) > S::BUDGET) continue;
             for (int chunks = (a.units + MAX_BOX - 1) / MAX_BOX; chunks <= a.units; chunks++) {
                 const int kc = box_units(chunks);
                 if (kc > MAX_BOX) continue;
                 const int bytes = pad(R * (kc * UNIT_Q + box_scales(kc)) + (resident ? 0 : kc * a.xunit));
-                if (want * bytes > whole_budget - (resident ? pad(xall) : 0)) {
+                if (want * bytes > S::BUDGET - (resident ? pad(xall) : 0)) {
                     if (kc == 1) break;
                     continue;
                 }
@@ -805,7 +813,7 @@ static int launch(dwim_b200_ctx *ctx, GemvArgs &a) {
         }
     }
     a.xres_bytes = a.x_resident ? xall : 0;
-    const int budget = whole_budget - pad(a.xres_bytes);
+    const int budget = S::BUDGET - pad(a.xres_bytes);
     if (a.boxed) {
         a.stages = budget / a.stage_bytes;
     } else if (a.whole_rows) {
@@ -834,11 +842,11 @@ static int launch(dwim_b200_ctx *ctx, GemvArgs &a) {
     if (a.stages > MAX_STAGES) a.stages = MAX_STAGES;
     if (a.stages < 2) return fail(ctx, DWIM_B200_EINVAL, "small-M kernel: a stage of %d bytes does not fit", a.stage_bytes);
     a.n_tiles = (int)((a.w.rows + R - 1) / R);
-    const int smem = fixed + (ALIGN - 128) + pad(a.xres_bytes) + a.stages * a.stage_bytes;
+    const int smem = S::LIMIT - S::BUDGET + pad(a.xres_bytes) + a.stages * a.stage_bytes;
     auto kern = dwim_smallm_kernel<FMT, NT, RT, KS>;
     static std::atomic<bool> configured[64] = {};   // per instantiation, per device; contexts of several threads share it
     if (!configured[ctx->device & 63]) {
-        DWIM_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT));
+        DWIM_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::LIMIT));
         configured[ctx->device & 63] = true;
     }
     int grid = a.n_tiles < ctx->sm_count ? a.n_tiles : ctx->sm_count;
@@ -876,12 +884,12 @@ static int launch_shape(dwim_b200_ctx *ctx, GemvArgs &a) {
     // 13.4 14.7, [5120, 6144] 9.7 10.4 9.2 10.0, [1024, 5120] 6.2 6.7 7.8 8.4; [5120, 17408] by five
     // tokens 30.6 35.5 25.8 31.1; Q6_K [5120, 17408] by eight 42.9 46.3 34.2 45.5; the [151936, 5120] head
     // by one 167 170 152 162, by eight 287 282 225 249.  Four is for Q4_K alone; Q8_0's
-    // whole rows by one or two tokens beat its boxes, two swizzled ones a unit, unless the boxes take a
+    // whole rows, where they fit, by one or two tokens beat its boxes, two swizzled ones a unit, unless the boxes take a
     // single round ([12288, 5120] 16.0 whole, 17.0 in boxes; [5120, 5120] 10.9 and 10.5; by eight 29.9 and
     // 22.5, 18.1 and 12.9).  Rows beyond 65536 columns keep one row tile: the stage with the fewest units is the narrowest then.
     int rt = 1;
     if (a.w.cols <= 65536) {
-        const bool whole = FMT == Q8_I8 && NT == 1 && 2 * 16 * (a.w.qpitch + a.w.srow * 2) + (size_t)a.units * a.xunit <= 222 * 1024;
+        const bool whole = FMT == Q8_I8 && NT == 1 && Smem<FMT, NT, 1, 8>::two_whole_fit(a);
         double best = 0;
         for (int t = 1; t <= (FMT == Q4K_I8 ? 4 : 3); t++) {
             const size_t tiles = (a.w.rows + 16 * t - 1) / (16 * t);
