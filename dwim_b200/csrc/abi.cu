@@ -510,9 +510,10 @@ static int product(dwim_b200_ctx *ctx, const OutSpec &out, size_t out_len, const
     // (value and rounding remainder), summed again in the epilogue.
     // Up to eight tokens: the small-M kernel's int8 routines.  Above: the tensor-core kernels -- Q4_K
     // from nine tokens on (measured on B200 at [17408, 5120]: 26 us at nine to sixteen tokens, against
-    // 57 us for sixteen through two small-M launches); Q6_K and Q8_0, whose dense kernel sums in the tensor
-    // cores (4e-7 to 7e-7 of the result, where the groups' integer products give 1e-7), from 65 on, and in
-    // groups of eight through the small-M kernel below that.
+    // 57 us for sixteen through two small-M launches); Q6_K and Q8_0 from 65 on, and in groups of eight through
+    // the small-M kernel below that.  (Their dense kernel would be faster from 33 tokens, but sums in the tensor
+    // cores: 2.8e-7 to 6.7e-7 of the result in 2-norm, where the groups' integer products give 3e-7 by f32
+    // activations and 1.2e-7 by bf16 ones.)
     const bool dense = gemm_supports(v) && n > (v.fmt == Q4_K ? (size_t)I8_MAX_TOKENS : (size_t)64);
     if (dense) {
         // bf16 activations are exact in one f16 column; f32 ones travel as two
@@ -619,7 +620,7 @@ int dwim_b200_swiglu(dwim_b200_ctx *ctx, dwim_b200_buffer *out, const dwim_b200_
     const size_t n = gate->v.cols ? x->len / gate->v.cols : 0;
     if (gate->v.fmt == up->v.fmt && gate->v.qpitch == up->v.qpitch && gemv_takes_i8(gate->v, n) &&
         x->len == n * gate->v.cols && out->len == n * gate->v.rows && out->data != x->data && gate->v.rows) {
-        // one and two tokens: both matrices in one launch, the activation applied where the two sums meet
+        // up to eight tokens: both matrices in one launch, the activation applied where the two sums meet
         rc = ensure_shadow(ctx, x, SHADOW_PANEL_I8, gate->v.cols, 0);
         if (rc == 0)
             rc = gemv_small_i8(ctx, gate->v, (const uint8_t *)x->shadow, (int)n, 0, out_local(out->data, gate->v.rows), nullptr, EPI_STORE, &up->v);

@@ -64,8 +64,6 @@ struct dwim_b200_ctx {
     uint64_t launches = 0;
     char name[256] = {0};
     char err[512] = {0};
-    // the GEMM path's lazily created state
-    void *gemm_state = nullptr;
     // A kernel on the stream has written weight memory since the last small-M launch
     // (an upload's repack): that launch must be an ordinary one, because a
     // programmatic dependent streams weights before it waits for the kernels ahead.
@@ -204,11 +202,10 @@ int build_gemm_operand(dwim_b200_ctx *ctx, const float *x, size_t n, size_t cols
 
 // gemv.cu
 enum Epilogue : int { EPI_STORE = 0, EPI_ADD = 1, EPI_SWIGLU = 2 };
-// One launch: tokens [t0, t0 + n_tokens) of a panel array holding ncols_total
-// columns, the launch's first at col0.  aux is the `up` product for EPI_SWIGLU.
 bool gemv_takes_i8(const WeightView &w, size_t n);
-// n_tokens tokens (at most eight) whose results are tokens [t0, t0 + n_tokens) of out and aux; or
-// `groups` such groups in a row, each with panels of its own.
+// One launch: n_tokens tokens (at most eight) whose results are tokens [t0, t0 + n_tokens) of out and aux (the
+// `up` product for EPI_SWIGLU); or `groups` such groups in a row, each with panels of its own.  `up`, when given,
+// makes it the SwiGLU of the pair (w = gate).
 int gemv_small_i8(dwim_b200_ctx *ctx, const WeightView &w, const uint8_t *panels, int n_tokens, size_t t0, const OutSpec &out,
                   const float *aux, int epilogue, const WeightView *up = nullptr, size_t groups = 1);
 void peer_release(dwim_b200_ctx *ctx);

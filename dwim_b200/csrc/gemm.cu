@@ -61,7 +61,7 @@ namespace {
 
 constexpr int TILE_M = 128;   // weight rows per CTA
 constexpr int BK = 64;        // K per stage: one 128-byte swizzled row of f16
-constexpr int KBLOCKS = 4;    // K blocks per unit = stages of the A ring: A stage index == K block within the unit
+constexpr int KBLOCKS = 4;    // K blocks per unit; each is a stage of the A ring and a hand-over of its own
 constexpr int SCALE_SLOTS = 4;
 constexpr int N_WORKERS = 16;                                      // warps 2..17: four per TMEM lane quadrant
 constexpr int RAW_WARP = 2 + N_WORKERS;                            // the packed weights' producer
@@ -88,18 +88,16 @@ struct GemmArgs {
 // ring.  Up to 128 these are one and a quarter to two units deep, so that the
 // workers decode a unit while the one before multiplies ([5120, 17408] by 16
 // tokens: 41 us one unit deep, 38 like this; [17408, 5120] by 48 tokens 39.1
-// with K blocks handed over in pairs, one unit deep, and 37.4).  At 256 columns a decoded weight is used twice
+// with K blocks handed over in pairs, one unit deep, and 37.4 one by one like this).
+// At 256 columns a decoded weight is used twice
 // as often, an MMA takes 128 cycles, and shared memory is the limit: three B
-// stages, two raw stages, one stage of the minimums' operands, and a hand-over
-// per K block (a B stage is reloaded as soon as its own K block is done).
+// stages, two raw stages, one stage of the minimums' operands (a B stage is
+// reloaded as soon as its own K block is done).
 template <int BN> struct Cfg {
     static constexpr int A_STAGES = BN <= 32 ? 8 : BN <= 64 ? 6 : BN <= 128 ? 5 : KBLOCKS;
     static constexpr int B_STAGES = BN > 192 ? 3 : A_STAGES;
     static constexpr int RAW_STAGES = BN <= 32 || BN >= 128 ? 2 : 3;
     static constexpr int MIN_STAGES = BN > 128 ? 1 : 2;
-    static constexpr int HAND = 1;                                 // K blocks per hand-over
-    static constexpr int NHAND = KBLOCKS / HAND;
-    static constexpr int SLOTS = A_STAGES / HAND;                  // hand-over barriers
     static constexpr int B_BYTES = BN * BK * 2;
     static constexpr int BMIN_BYTES = BN * 16 * 2;                 // [K group of 8][column][16 B]: the means' hi and lo parts
     static constexpr int MIN_BYTES = AMIN_BYTES + ((BMIN_BYTES + 1023) / 1024) * 1024;
@@ -235,6 +233,47 @@ __device__ __forceinline__ void gemm_emit(const EmitTo &e, size_t rows, size_t n
         }
 }
 
+// A split tile's exchange.  Eight columns at a time belong to the cluster's blocks in turn: the others' sums
+// of them go into their owner's rings (whose last unit is done when the blocks have met), by rank, draining
+// warp group, column and row ...
+template <int COLS>
+__device__ __forceinline__ void push_shares(const float (&acc)[COLS], uint32_t rings, int own, int g, int rl, int rank, int split_k) {
+    cluster_sync();
+#pragma unroll
+    for (int q = 0; q < COLS / 8; q++) {
+        if (q % split_k == rank) continue;
+        const uint32_t to = cluster_addr(rings + (((rank * 4 + g) * own + q / split_k * 8) * TILE_M + rl) * 4, q % split_k);
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to + j * TILE_M * 4), "f"(acc[8 * q + j]) : "memory");
+    }
+    cluster_sync();
+}
+// ... and the owner of columns 8q .. 8q + 7 adds its blocks' sums in rank order.
+template <int COLS>
+__device__ __forceinline__ void sum_shares(const float (&acc)[COLS], int q, uint32_t rings, int own, int g, int rl, int rank, int split_k,
+                                           float (&v)[8]) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = 0.0f;
+    for (int r = 0; r < split_k; r++) {
+        const uint32_t from = rings + (((r * 4 + g) * own + q / split_k * 8) * TILE_M + rl) * 4;
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] += r == rank ? acc[8 * q + j] : lds32f(from + j * TILE_M * 4);
+    }
+}
+// Eight finished columns from column c on: a token each, or (split) the two terms of four.
+template <bool SHARED>
+__device__ __forceinline__ void emit_columns(const EmitTo &to, size_t rows, size_t n, int split, size_t c, float (&v)[8]) {
+    if (split) {
+        float y[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) y[j] = v[2 * j] + v[2 * j + 1];
+        gemm_emit<SHARED>(to, rows, n, c >> 1, y);
+    } else {
+        gemm_emit<SHARED>(to, rows, n, c, v);
+    }
+}
+
 constexpr uint32_t H2_1024 = 0x64006400u, H2_M1024 = 0xE400E400u, H2_64 = 0x54005400u, H2_M64 = 0xD400D400u;
 
 // ---- dequantizer: the 64 weights of one row and K block as exact sc*q halves ----------
@@ -358,8 +397,8 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     const int ub = (int)a.units * rank / split_k, units = (int)a.units * (rank + 1) / split_k - ub;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < C::SLOTS; s++) {
-            mbar_init(full0 + 8 * s, 1 + 4 * C::HAND);   // the producer's expect_tx arrival + the hand-over's worker warps
+        for (int s = 0; s < C::A_STAGES; s++) {
+            mbar_init(full0 + 8 * s, 1 + 4);             // the producer's expect_tx arrival + the K block's worker warps
             mbar_init(empty0 + 8 * s, 1);                // the MMA warp's commit
         }
         for (int s = 0; s < 2; s++) {
@@ -393,16 +432,18 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
         if (elect_one()) {
             for (int u = 0; u < units; u++) {
                 const int ms = u % C::MIN_STAGES;
-                for (int h = 0; h < C::NHAND; h++) {
-                    // B stage kb % B_STAGES was last read by K block kb - B_STAGES
-                    for (int g = h * C::HAND; g < (h + 1) * C::HAND; g++) {
+                for (int h = 0; h < KBLOCKS; h++) {
+                    // B stage kb % B_STAGES was last read by K block kb - B_STAGES.  (The loops of one turn keep
+                    // the compiler's code for the whole loop as it is: written out, however unrolled, a layer of
+                    // 16 tokens takes 161.5 us instead of 160.5.)
+                    for (int g = h; g < h + 1; g++) {
                         const int prev = KBLOCKS * u + g - C::B_STAGES;
                         if (prev >= 0)
-                            mbar_wait_parked(empty0 + 8 * (prev / C::HAND % C::SLOTS), (prev / C::HAND / C::SLOTS) & 1, a.status, 0x20u);
+                            mbar_wait_parked(empty0 + 8 * (prev % C::A_STAGES), (prev / C::A_STAGES) & 1, a.status, 0x20u);
                     }
-                    const uint32_t full = full0 + 8 * ((u * C::NHAND + h) % C::SLOTS);
-                    mbar_expect_tx(full, C::HAND * C::B_BYTES);
-                    for (int g = h * C::HAND; g < (h + 1) * C::HAND; g++) {
+                    const uint32_t full = full0 + 8 * ((u * KBLOCKS + h) % C::A_STAGES);
+                    mbar_expect_tx(full, C::B_BYTES);
+                    for (int g = h; g < h + 1; g++) {
                         const int kb = KBLOCKS * u + g;
                         tma_load_2d(bstage0 + (kb % C::B_STAGES) * C::B_BYTES, &tmap_x, (KBLOCKS * ub + kb) * BK, col0, full);
                     }
@@ -440,7 +481,7 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
         const uint32_t a_lo = desc_lo_sw128(astage0), b_lo = desc_lo_sw128(bstage0);
         const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
         int bs = 0;                                                   // the B stage of the next K block
-        uint32_t slot = 0, turn = 0;                                  // the next hand-over's barriers, their phase
+        uint32_t slot = 0, turn = 0;                                  // its hand-over's barriers, their phase
         for (int u0 = 0; u0 < units; u0 += 2) {
 #pragma unroll
             for (int ab = 0; ab < 2; ab++) {
@@ -450,27 +491,23 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
                 const uint32_t upar = (u0 >> 1) & 1;
                 mbar_wait_parked(accempty0 + 8 * ab, upar ^ 1, a.status, 0x80u);   // the drain of unit u-2 is done
 #pragma unroll
-                for (int h = 0; h < C::NHAND; h++) {
-                    if (C::SLOTS == C::NHAND) slot = h, turn = ab;
+                for (int g = 0; g < KBLOCKS; g++) {
+                    if (C::A_STAGES == KBLOCKS) slot = g, turn = ab;
                     mbar_wait_parked(full0 + 8 * slot, turn, a.status, 0x100u);
                     tc_fence_after();
+                    const uint32_t ad = a_lo + (C::A_STAGES == KBLOCKS ? g : bs) * (A_BYTES >> 4);
+                    const uint32_t bd = b_lo + (C::B_STAGES == KBLOCKS ? g : bs) * (C::B_BYTES >> 4);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int gg = 0; gg < C::HAND; gg++) {
-                        const int g = h * C::HAND + gg;
-                        const uint32_t ad = a_lo + (C::A_STAGES == KBLOCKS ? g : bs) * (A_BYTES >> 4);
-                        const uint32_t bd = b_lo + (C::B_STAGES == KBLOCKS ? g : bs) * (C::B_BYTES >> 4);
-                        if (elect_one()) {
-#pragma unroll
-                            for (int k = 0; k < BK / 16; k++) {   // 32 bytes further along the swizzled row per K=16
-                                if (g == 0 && k == 0) umma_f16_lo<0>(s1, ad, bd, desc_hi, idesc);
-                                else umma_f16_lo<1>(s1, ad + 2 * k, bd + 2 * k, desc_hi, idesc);
-                            }
+                        for (int k = 0; k < BK / 16; k++) {   // 32 bytes further along the swizzled row per K=16
+                            if (g == 0 && k == 0) umma_f16_lo<0>(s1, ad, bd, desc_hi, idesc);
+                            else umma_f16_lo<1>(s1, ad + 2 * k, bd + 2 * k, desc_hi, idesc);
                         }
-                        bs = bs + 1 == C::B_STAGES ? 0 : bs + 1;
                     }
+                    bs = bs + 1 == C::B_STAGES ? 0 : bs + 1;
                     if (elect_one()) umma_commit(empty0 + 8 * slot);   // the stages may be refilled once these finish
                     __syncwarp();
-                    if (C::SLOTS != C::NHAND && ++slot == C::SLOTS) slot = 0, turn ^= 1;
+                    if (C::A_STAGES != KBLOCKS && ++slot == C::A_STAGES) slot = 0, turn ^= 1;
                 }
                 const int ms = u % C::MIN_STAGES;
                 mbar_wait_parked(minfull0 + 8 * ms, (u / C::MIN_STAGES) & 1, a.status, 0x200u);
@@ -530,12 +567,12 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             const uint4 hdr = lds128(raw_row);
             Q4kBlock blk;
             load_q4k_block(hdr, raw_row, g, blk);
-            const int kb = KBLOCKS * u + g, hand = kb / C::HAND;
-            mbar_wait_parked(empty0 + 8 * (hand % C::SLOTS), ((hand / C::SLOTS) & 1) ^ 1, a.status, 0x800u);   // the MMAs that read this stage are done
-            store_q4k_block(blk, a_row_sw + kb % C::A_STAGES * A_BYTES);
+            const int kb = KBLOCKS * u + g, stage = kb % C::A_STAGES;
+            mbar_wait_parked(empty0 + 8 * stage, ((kb / C::A_STAGES) & 1) ^ 1, a.status, 0x800u);   // the MMAs that read this stage are done
+            store_q4k_block(blk, a_row_sw + stage * A_BYTES);
             fence_async_smem();          // the tensor core reads shared memory through the async proxy
             __syncwarp();
-            if (lane == 0) mbar_arrive(full0 + 8 * (hand % C::SLOTS));
+            if (lane == 0) mbar_arrive(full0 + 8 * stage);
             if (g >= 2) {
                 // the minimums' A operand [K group][row][16 B]: groups (hi, hi, lo, lo) of the
                 // two f16 terms of -(32*dmin/s)*m_j; K block 2's warp writes m_0..m_3, K block 3's m_4..m_7
@@ -592,49 +629,21 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             for (int j = 0; j < C::DRAIN_COLS / 2; j++) unpack2(acc2[j], acc[2 * j], acc[2 * j + 1]);
             const size_t row = (size_t)row0 + rl;
             if (OUT == 0 && split_k > 1) {
-                // Eight columns at a time belong to the cluster's blocks in turn.  The others' sums go into
-                // their owner's rings (whose last unit is done when the blocks have met), the owner adds
-                // its blocks' sums in rank order.
                 const int own = C::owned(split_k);
-                cluster_sync();
-#pragma unroll
-                for (int q = 0; q < C::DRAIN_COLS / 8; q++) {
-                    if (q % split_k == rank) continue;
-                    const uint32_t to = cluster_addr(astage0 + (((rank * 4 + g) * own + q / split_k * 8) * TILE_M + rl) * 4, q % split_k);
-#pragma unroll
-                    for (int j = 0; j < 8; j++)
-                        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to + j * TILE_M * 4), "f"(acc[8 * q + j]) : "memory");
-                }
-                cluster_sync();
+                push_shares(acc, astage0, own, g, rl, rank, split_k);
                 const EmitTo to = emit_to(a.out, a.aux, a.epi, row);
 #pragma unroll
                 for (int q = 0; q < C::DRAIN_COLS / 8; q++) {
                     if (q % split_k != rank) continue;
                     float v[8];
-#pragma unroll
-                    for (int j = 0; j < 8; j++) v[j] = 0.0f;
-                    for (int r = 0; r < split_k; r++) {
-                        const uint32_t from = astage0 + (((r * 4 + g) * own + q / split_k * 8) * TILE_M + rl) * 4;
-#pragma unroll
-                        for (int j = 0; j < 8; j++) v[j] += r == rank ? acc[8 * q + j] : lds32f(from + j * TILE_M * 4);
-                    }
+                    sum_shares(acc, q, astage0, own, g, rl, rank, split_k, v);
                     if (scaled) {
 #pragma unroll
                         for (int j = 0; j < 8; j++) v[j] *= lds32f(tk + (8 * q + j) * 4);
                     }
-                    if (row >= a.rows) continue;
-                    const size_t c = (size_t)col0 + g * C::DRAIN_COLS + 8 * q;
-                    if (a.split) {
-                        float y[4];
-#pragma unroll
-                        for (int j = 0; j < 4; j++) y[j] = v[2 * j] + v[2 * j + 1];
-                        gemm_emit<false>(to, a.rows, a.n, c >> 1, y);
-                    } else {
-                        gemm_emit<false>(to, a.rows, a.n, c, v);
-                    }
+                    if (row < a.rows) emit_columns<false>(to, a.rows, a.n, a.split, (size_t)col0 + g * C::DRAIN_COLS + 8 * q, v);
                 }
-            } else
-            if (OUT == 2) {
+            } else if (OUT == 2) {
                 // The group's tile [token][row] into the rings' shared memory, which nothing reads any
                 // more (the last unit's MMAs are done, its accumulator drained), then one store per
                 // destination.  Rows and tokens past the end are cut off by the maps' bounds.
@@ -715,9 +724,14 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
 // The kernel is Q4_K's in outline (roles, hand-overs, drains; see there), but for: two A stages of a hi and
 // a lo tile, K block kb in stage kb % 2; a ring of its own for the activations; no minimums.
 // (The terms used to be written to memory by a pass of their own and loaded by every column of tiles: 64 KB
-// from L2 per K block of 1024 cycles, 9.1 TB/s, was what bound it.  [12288, 5120] Q6_K by 512 f32 tokens
-// 299 us then, 210 now; [5120, 5120] Q8_0 by 131 of them 97 and 69.  The error fell with the drains: 1e-6 to
-// 1e-5 of the result over K = 2304 to 12288 then, 4e-7 and 7e-7 now at any K.)
+// from L2 per K block of 1024 cycles, 9.1 TB/s, was what bound it.  Products with their operand, in short bursts:
+// [12288, 5120] Q6_K by 512 f32 tokens 299 us then, 209 now (198 the kernel alone; 253 in a long run, under the
+// power limit); [5120, 5120] Q8_0 by 131 of them 97 and 69.  The error fell with the drains: 1e-6 to 1e-5 of
+// the result in 2-norm over K = 2304 to 12288 then; now, at any K from 512 to 17408, 4.6e-7 (Q6_K) and 6.7e-7
+// (Q8_0) by f32 activations, 2.8e-7 and 6.4e-7 by bf16 ones, the largest difference 2.5e-6 and 4.2e-6 of the
+// result's root mean square.)
+// Bound by the tensor pipe (68 % active by 512 columns), beside which 96 registers a thread are short: the
+// 256-column form spills 60 (Q6_K) and 28 bytes (Q8_0).
 struct DenseArgs {
     size_t rows, n, units;
     int split, epi, split_k;
@@ -960,32 +974,14 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 #pragma unroll
         for (int j = 0; j < C::DRAIN_COLS / 2; j++) unpack2(acc2[j], acc[2 * j], acc[2 * j + 1]);
         const int own = C::owned(split_k);
-        if (split_k > 1) {
-            // eight columns at a time belong to the cluster's blocks in turn, as in the Q4_K kernel
-            cluster_sync();
-#pragma unroll
-            for (int q = 0; q < C::DRAIN_COLS / 8; q++) {
-                if (q % split_k == rank) continue;
-                const uint32_t to = cluster_addr(astage0 + (((rank * 4 + g) * own + q / split_k * 8) * TILE_M + rl) * 4, q % split_k);
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to + j * TILE_M * 4), "f"(acc[8 * q + j]) : "memory");
-            }
-            cluster_sync();
-        }
+        if (split_k > 1) push_shares(acc, astage0, own, g, rl, rank, split_k);
         const EmitTo to = emit_to(a.out, a.aux, a.epi, row);
 #pragma unroll
         for (int q = 0; q < C::DRAIN_COLS / 8; q++) {
             if (q % split_k != rank) continue;
             float v[8];
             if (split_k > 1) {
-#pragma unroll
-                for (int j = 0; j < 8; j++) v[j] = 0.0f;
-                for (int r = 0; r < split_k; r++) {
-                    const uint32_t from = astage0 + (((r * 4 + g) * own + q / split_k * 8) * TILE_M + rl) * 4;
-#pragma unroll
-                    for (int j = 0; j < 8; j++) v[j] += r == rank ? acc[8 * q + j] : lds32f(from + j * TILE_M * 4);
-                }
+                sum_shares(acc, q, astage0, own, g, rl, rank, split_k, v);
             } else {
 #pragma unroll
                 for (int j = 0; j < 8; j++) v[j] = acc[8 * q + j];
@@ -993,15 +989,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             if (row >= a.rows) continue;
 #pragma unroll
             for (int j = 0; j < 8; j++) v[j] *= lds32f(tk + (8 * q + j) * 4);
-            const size_t c = (size_t)col0 + g * C::DRAIN_COLS + 8 * q;
-            if (a.split) {
-                float y[4];
-#pragma unroll
-                for (int j = 0; j < 4; j++) y[j] = v[2 * j] + v[2 * j + 1];
-                gemm_emit<SHARED>(to, a.rows, a.n, c >> 1, y);
-            } else {
-                gemm_emit<SHARED>(to, a.rows, a.n, c, v);
-            }
+            emit_columns<SHARED>(to, a.rows, a.n, a.split, (size_t)col0 + g * C::DRAIN_COLS + 8 * q, v);
         }
     }
     if (warp < 2 || warp == RAW_WARP) {
@@ -1055,6 +1043,9 @@ namespace {
 // six shapes by 16 to 2048 tokens; the choice is within 3 % of the best of them but for [1024, 5120] by
 // 2048).  Without it 40 tiles left 108 of 148 SMs idle: [5120, 17408] by 16 tokens 85 us, 39 with three
 // blocks a tile; by 131 bf16 tokens 134 and 67; by 512 f32 tokens (160 tiles) 299 and 236.
+// The dense kernel's units are twice as long, so a tile's other costs are fewer of them: two, and four and
+// a half with the exchange.  Over every split of twelve products (rows 1024 to 17408, K 5120 and 12288, 80 to 2048
+// tokens) the choice is within 3 % of the best, but for [5120, 5120] by 131 f32 tokens (63.6 us alone, 60.4 by three).
 struct SplitCost {
     double tile, shared;      // what a tile costs besides its units: alone, shared
 };
@@ -1148,7 +1139,13 @@ int launch_gemm(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, 
                                 CU_TENSOR_MAP_SWIZZLE_NONE, "output")))
                 return rc;
     }
-    auto kern = shared == 2 ? gemm_q4k_kernel<BN, 2> : shared == 1 ? gemm_q4k_kernel<BN, 1> : gemm_q4k_kernel<BN, 0>;
+    auto kern = gemm_q4k_kernel<BN, 0>;
+    if constexpr (BN != 192) {      // which gemm_large takes for one destination alone
+        if (shared == 2) kern = gemm_q4k_kernel<BN, 2>;
+        if (shared == 1) kern = gemm_q4k_kernel<BN, 1>;
+    } else if (shared) {
+        return fail(ctx, DWIM_B200_EINVAL, "tiles of 192 columns have one destination");
+    }
     static std::atomic<bool> configured[64][3] = {};
     if (!configured[ctx->device & 63][shared]) {
         DWIM_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
@@ -1205,8 +1202,13 @@ int launch_dense(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand,
 
 }  // namespace
 
-// Formats the tensor-core kernels take: Q4_K, and the others up to 12288 columns (longer rows go
-// through the small-M kernel in groups of eight tokens).
+// Formats the tensor-core kernels take: Q4_K, and the others up to 12288 columns.  Longer rows go through the
+// small-M kernel in groups of eight tokens at any token count.  The dense kernel could take them (its error and
+// shared memory do not depend on K; the operand's prologue ends at 51200 columns) and would be faster: [5120,
+// 17408] Q6_K by 65 bf16 tokens 212 us in groups, 70 dense, by 512 f32 ones 1445 and 336; Q8_0 193 and 72,
+// 1293 and 337.  But it sums in the tensor cores: 4.6e-7 (Q6_K) and 6.7e-7 (Q8_0) of the result in 2-norm by f32
+// activations where the groups give 3.1e-7, 2.8e-7 and 6.4e-7 by bf16 ones where they give 1.2e-7.  So the line
+// stays where the two paths' precision has been since the dense path was limited by its decoder to such rows.
 bool gemm_supports(const WeightView &w) {
     if (w.cols % 256) return false;
     return w.fmt == Q4_K || ((w.fmt == Q6_K || w.fmt == Q8_0) && w.cols <= 12288);
@@ -1220,9 +1222,10 @@ int gemm_large(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, s
         if (ncols <= 32) return launch_gemm<32>(ctx, w, operand, n, split, out, aux, epilogue);
         if (ncols <= 64) return launch_gemm<64>(ctx, w, operand, n, split, out, aux, epilogue);
         if (ncols <= 128) return launch_gemm<128>(ctx, w, operand, n, split, out, aux, epilogue);
-        // Above that, tiles of 192 or 256 columns: a wave of the narrower ones lasts 0.82 of one of the wider
-        // (three quarters of the columns, an activations' ring of four stages instead of three), so the
-        // waves decide: [17408, 5120] by 131 bf16 tokens 51.9 us in tiles of 256 and 41.5 of 192, by 384 94.0 and
+        // Above that, tiles of 192 or 256 columns: a wave of the narrower ones lasts 0.77 of one of the wider
+        // when it is the only one ([18944, 5120], 148 tiles: 36.5 us and 47.4; K = 17408: 116 and 150), 0.82 in a
+        // row of them (three quarters of the columns, an activations' ring of four stages instead of three), so
+        // the waves decide: [17408, 5120] by 131 bf16 tokens 51.9 us in tiles of 256 and 41.5 of 192, by 384 94.0 and
         // 76.9; [5120, 17408] by 131 64.4 and 54.6; by 2048 tokens 256 takes eight waves, 192 eleven.
         if (out.world == 1 && 0.82 * gemm_time<192>(ctx, w, ncols) < gemm_time<256>(ctx, w, ncols))
             return launch_gemm<192>(ctx, w, operand, n, split, out, aux, epilogue);

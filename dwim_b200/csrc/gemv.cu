@@ -77,10 +77,9 @@ struct GemvArgs {
 };
 
 
-// Q4_K through the int8 tensor-core path (one or two tokens): the same blocks,
-// another activation operand and unit routine.
+// The formats as the int8 tensor-core routines read them.
 constexpr int Q4K_I8 = 1012;
-constexpr int Q8_I8 = 1008;     // Q8_0 and Q6_K through the same int8 path (up to eight tokens)
+constexpr int Q8_I8 = 1008;
 constexpr int Q6K_I8 = 1014;
 constexpr bool is_i8(int fmt) { return fmt == Q4K_I8 || fmt == Q8_I8 || fmt == Q6K_I8; }
 constexpr int base_of(int fmt) { return fmt == Q4K_I8 ? (int)Q4_K : fmt == Q8_I8 ? (int)Q8_0 : fmt == Q6K_I8 ? (int)Q6_K : fmt; }
@@ -102,17 +101,17 @@ struct Lane {
 };
 
 // ---------------------------------------------------------------------------
-// Q4_K, one or two tokens, int8 tensor-core path
+// the unit routines
 // ---------------------------------------------------------------------------
-// The nibbles stay integers: four of them per AND, multiplied on the tensor
+// Q4_K's nibbles stay integers: four of them per AND, multiplied on the tensor
 // cores (mma.sync m16n8k32 u8 x s8 -> s32) with the activations' signed
-// base-256 digit planes as columns (prologue.cu: column = 4*token + plane).
+// base-256 digit planes as columns (prologue.cu).
 // One MMA covers one 32-weight sub-block of 16 rows; its sums are weighted by
 // the sub-block's 6-bit scale with integer multiply-adds, so a whole unit is an
 // exact integer per (row, column), which d and the plane's worth then scale.
 // High nibbles are masked in place (16*q: no shift), the low ones' scales are
-// 16 times larger instead, and the unit's sum is divided by 16 in d.  The minimums use the digits' per-sub-block sums (dp4a).
-// About half the instructions of the f16 routine above for the same weights.
+// 16 times larger instead, and the unit's sum is divided by 16 in d.  The minimums
+// use the digits' per-sub-block sums (dp4a).
 // c = a * b (the accumulator operand is zero, not a register that has to be cleared first)
 __device__ __forceinline__ void imma_u8s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
@@ -607,7 +606,6 @@ __global__ void __launch_bounds__((RT * KS + 1) * 32, 1) dwim_smallm_kernel(cons
     // apart to cover all banks, so lanes g = 0..3 take rows 0, 2, 4, 6 of the
     // eight and g = 4..7 rows 1, 3, 5, 7.
     const int grow = (FMT == Q4K_I8 || FMT == Q8_I8) ? ((L.g & 3) * 2 + (L.g >> 2)) : L.g;
-    // the digit planes' columns: one tile of 4n columns (one and two tokens), or a tile of n columns per plane
     constexpr bool ONE = NT == 0, PACKED = NT <= 1;
     const I8Cols X = i8_cols<PACKED ? 1 : NT>(a.ncols, a.n_tokens);
 

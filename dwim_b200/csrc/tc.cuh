@@ -1,4 +1,4 @@
-// tcgen05 wrappers and descriptors shared by the tensor-core kernels (gemm.cu, skinny.cu).
+// tcgen05 wrappers and descriptors of the tensor-core kernels (gemm.cu).
 #pragma once
 #include "ptx.cuh"
 

@@ -19,6 +19,11 @@
  *   - Weights are GGUF blocks, row-major: rows * dwim_b200_row_bytes(fmt,
  *     cols) bytes.  Activations are f32, one row of `cols` per token;
  *     results are token-major, out[t * rows + r] (gpu/cpu.rs:144-148).
+ *   - A call gives the same bits every time it is made with the same inputs
+ *     and sizes.  The same tokens in another batch, or the same rows in another
+ *     matrix (a shard's), may be summed in another order: kernels, and how many
+ *     blocks and warps share a sum, are chosen by the sizes.  Such results
+ *     agree within 1e-5 of their root mean square.
  *   - There is no CPU fallback: without a CUDA device dwim_b200_open fails.
  */
 #ifndef DWIM_B200_H
@@ -208,7 +213,7 @@ DWIM_B200_API int dwim_b200_swiglu(dwim_b200_ctx *ctx, dwim_b200_buffer *out, co
  * tile kernels read; here the same launch writes the f32 result and, where rows
  * are whole 256-weight units, the 16-bit operand form the next product of `out`
  * will read (int8 digit planes for up to eight rows, the tensor-core kernel's
- * f16 rows, means and scales above sixteen), so that no activation prologue
+ * f16 rows, means and scales above eight), so that no activation prologue
  * runs before that product. */
 DWIM_B200_API int dwim_b200_normalize(dwim_b200_ctx *ctx, dwim_b200_buffer *out, const dwim_b200_buffer *x,
                                       const dwim_b200_buffer *weight, size_t len, float eps);

@@ -23,11 +23,11 @@ def source(name):
     return re.sub(r"//[^\n]*|/\*.*?\*/", "", text, flags=re.S)
 
 
-def kernels(text):
-    """(name, body) of every __global__ function."""
-    for m in re.finditer(r"__global__", text):
+def functions(text):
+    """(name, body) of every kernel and device function."""
+    for m in re.finditer(r"__global__|__device__ __forceinline__", text):
         at = text.index("{", m.start())
-        name = re.findall(r"(\w+)\s*\(", text[m.start():at])[-1]
+        name = next(n for n in re.findall(r"(\w+)\s*\(", text[m.start():at]) if not n.startswith("__"))
         depth, end = 0, at
         while True:
             depth += {"{": 1, "}": -1}.get(text[end], 0)
@@ -37,20 +37,21 @@ def kernels(text):
         yield name, text[at:end]
 
 
-def test_every_kernel_is_found():
-    names = [name for f in SOURCES for name, _ in kernels(source(f))]
-    assert {"normalize_i8_kernel", "matmul_bf16_tile_kernel", "gemm_q4k_kernel", "gemm_dense_kernel", "dwim_smallm_kernel"} <= set(names)
+def test_every_function_is_found():
+    names = [name for f in SOURCES for name, _ in functions(source(f))]
+    assert {"normalize_i8_kernel", "matmul_bf16_tile_kernel", "gemm_q4k_kernel", "gemm_dense_kernel", "dwim_smallm_kernel",
+            "push_shares"} <= set(names)
 
 
 @pytest.mark.parametrize("name", SOURCES)
 def test_a_cluster_meets_before_its_blocks_reach_each_other(name):
     """A block may touch another's shared memory once that block is known to run: after a barrier of the cluster
     (being scheduled together is not having started)."""
-    for kernel, body in kernels(source(name)):
+    for function, body in functions(source(name)):
         remote = REMOTE.search(body)
         if remote:
             met = MET.search(body)
-            assert met and met.start() < remote.start(), f"{kernel}: a remote access ahead of the cluster's first meeting"
+            assert met and met.start() < remote.start(), f"{function}: a remote access ahead of the cluster's first meeting"
 
 
 @pytest.mark.parametrize("name", SOURCES + HEADERS)
