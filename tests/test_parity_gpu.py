@@ -40,6 +40,20 @@ def upload(dev, fmt, rows, cols, blocks):
     return dev.upload(Tensor(fmt, (rows, cols), blocks))
 
 
+def random_pair(dev, oracle, fmt, rows, cols, rng):
+    """A matrix of N(0, 0.02) weights and the same rows in another order, uploaded, and what the oracle decodes
+    from their blocks, in double precision: (matrix, its weights, reordered matrix, its weights)."""
+    blocks = dev.quantize(fmt, (0.02 * rng.standard_normal((rows, cols))).astype(np.float32)).data.reshape(rows, -1)
+    other = np.roll(blocks, 1, axis=0)
+    w = oracle.dequantize(fmt, blocks.reshape(-1), rows, cols).reshape(rows, cols).astype(np.float64)
+    return (upload(dev, fmt, rows, cols, blocks.reshape(-1)), w, upload(dev, fmt, rows, cols, np.ascontiguousarray(other).reshape(-1)),
+            np.roll(w, 1, axis=0))
+
+
+def silu_times(gate, up):
+    return gate / (1 + np.exp(-gate)) * up
+
+
 # ---- device plumbing (gpu/tests.rs:166-186, 962-975) --------------------------------
 def test_write_and_read_round_trip(dev, oracle):
     data = oracle.Lcg(1).floats(100_003)
@@ -200,8 +214,7 @@ def test_small_m_row_tiles_and_boxes(dev, oracle, fmt, rows, cols):
     more than one row tile; the three epilogues.  Eight tokens round an activation at 2^-23 of its unit's
     largest: 1e-5 of the result's root mean square is sixty times that."""
     rng = np.random.default_rng(rows + cols)
-    weight = dev.upload(dev.quantize(fmt, (0.02 * rng.standard_normal((rows, cols))).astype(np.float32)))
-    w = dev.dequantize(weight).astype(np.float64)
+    weight, w, other, w2 = random_pair(dev, oracle, fmt, rows, cols, rng)
     for n in (1, 2, 3, 5, 8):
         x = rng.standard_normal((n, cols)).astype(np.float32)
         res = rng.standard_normal((n, rows)).astype(np.float32)
@@ -212,8 +225,8 @@ def test_small_m_row_tiles_and_boxes(dev, oracle, fmt, rows, cols):
         assert np.abs(dev.read(out).reshape(n, rows) - want).max() <= bar, n
         dev.matmul_add(acc, weight, xb)
         assert np.abs(dev.read(acc).reshape(n, rows) - (want + res)).max() <= bar + 1e-6, n
-        dev.swiglu(out, weight, weight, xb, dev.alloc(n * rows))
-        silu = want / (1 + np.exp(-want)) * want
+        dev.swiglu(out, weight, other, xb, dev.alloc(n * rows))
+        silu = silu_times(want, x.astype(np.float64) @ w2.T)
         assert np.abs(dev.read(out).reshape(n, rows) - silu).max() <= 4 * bar * max(1.0, np.abs(want).max()), n
 
 
@@ -223,9 +236,9 @@ def test_groups_of_eight_tokens(dev, oracle, fmt, rows, cols, n):
     """Full groups in one launch (up to 64 of them), the rest in another; every token against the oracle's
     weights in double precision, 1e-5 of the result's root mean square as for eight tokens."""
     rng = np.random.default_rng(rows + n)
-    weight = dev.upload(dev.quantize(fmt, (0.02 * rng.standard_normal((rows, cols))).astype(np.float32)))
+    weight, w, _, _ = random_pair(dev, oracle, fmt, rows, cols, rng)
     x = rng.standard_normal((n, cols)).astype(np.float32)
-    want = x.astype(np.float64) @ dev.dequantize(weight).astype(np.float64).T
+    want = x.astype(np.float64) @ w.T
     res = rng.standard_normal((n, rows)).astype(np.float32)
     xb, out, acc = dev.buffer(x), dev.alloc(n * rows), dev.buffer(res)
     bar = 1e-5 * np.sqrt((want ** 2).mean())
@@ -784,8 +797,8 @@ def test_config2_gemm_full_size(dev, oracle, rows, cols, n):
 
 @pytest.mark.parametrize("n", [17, 33, 130, 300])
 def test_gemm_bf16_token_counts(dev, oracle, n):
-    """bf16 activations (one f16 column per token) at every tile width of the
-    tensor-core kernel: 32, 64, 256 columns, ragged against each."""
+    """bf16 activations (one f16 column per token) in tiles of 32, 64 and 192 or
+    256 columns of the tensor-core kernel, ragged against each."""
     rng = np.random.default_rng(3000 + n)
     rows, cols = 1000, 5120
     blocks = oracle.quantize("q4_k", (0.02 * rng.standard_normal((rows, cols))).astype(np.float32))
@@ -804,7 +817,7 @@ def test_gemm_shares_k_between_blocks(dev, oracle, rows, cols, n, bf16):
     tokens), with the three epilogues.  fp32 sums: the oracle in double precision from the decoded
     weights, 2e-5 of the result's root mean square (measured 2e-6)."""
     rng = np.random.default_rng(rows + n)
-    weight = dev.upload(dev.quantize("q4_k", (0.02 * rng.standard_normal((rows, cols))).astype(np.float32)))
+    weight, w, other, w2 = random_pair(dev, oracle, "q4_k", rows, cols, rng)
     x = rng.standard_normal((n, cols)).astype(np.float32)
     xb = dev.alloc(n * cols)
     if bf16:
@@ -813,7 +826,7 @@ def test_gemm_shares_k_between_blocks(dev, oracle, rows, cols, n, bf16):
         x = oracle.bf16(bits).reshape(n, cols)
     else:
         dev.write(xb, x)
-    want = x.astype(np.float64) @ dev.dequantize(weight).astype(np.float64).T
+    want = x.astype(np.float64) @ w.T
     bar = 2e-5 * np.sqrt((want ** 2).mean())
     out, again = dev.alloc(n * rows), dev.alloc(n * rows)
     dev.matmul(out, weight, xb)
@@ -825,9 +838,39 @@ def test_gemm_shares_k_between_blocks(dev, oracle, rows, cols, n, bf16):
     acc = dev.buffer(res)
     dev.matmul_add(acc, weight, xb)
     assert np.abs(dev.read(acc).reshape(n, rows) - (want + res)).max() <= bar + 1e-6
-    dev.swiglu(out, weight, weight, xb, again)
-    silu = want / (1 + np.exp(-want)) * want
+    dev.swiglu(out, weight, other, xb, again)
+    silu = silu_times(want, x.astype(np.float64) @ w2.T)
     assert np.abs(dev.read(out).reshape(n, rows) - silu).max() <= 4 * bar * max(1.0, np.abs(want).max())
+
+
+@pytest.mark.parametrize("fmt", FORMATS)
+@pytest.mark.parametrize("n,cut", [(300, 128), (40, 17), (8, 3)])
+def test_chunks_and_shards_agree_with_the_whole(dev, oracle, fmt, n, cut):
+    """What the header says of a result's bits: a call gives the same ones every time; the same tokens in
+    another batch, or the same rows in another matrix, may be summed in another order and agree within
+    1e-5 of the result's root mean square (either is within 5e-6 of it from the exact sum)."""
+    rng = np.random.default_rng(n)
+    rows, cols, row_cut = 1030, 2304, 517
+    blocks = dev.quantize(fmt, (0.02 * rng.standard_normal((rows, cols))).astype(np.float32)).data.reshape(rows, -1)
+    x = rng.standard_normal((n, cols)).astype(np.float32)
+
+    def product(r, t):
+        part = np.ascontiguousarray(blocks[r]).reshape(-1)
+        xs = np.ascontiguousarray(x[t])
+        out = dev.alloc(xs.shape[0] * blocks[r].shape[0])
+        weight, xb = upload(dev, fmt, blocks[r].shape[0], cols, part), dev.buffer(xs)
+        results = []
+        for _ in range(2):
+            dev.matmul(out, weight, xb)
+            results.append(dev.read(out).reshape(xs.shape[0], -1))
+        assert np.array_equal(results[0], results[1])
+        return results[0]
+
+    whole = product(slice(0, rows), slice(0, n))
+    bar = 1e-5 * np.sqrt((whole.astype(np.float64) ** 2).mean())
+    chunks = np.concatenate([product(slice(0, rows), slice(0, cut)), product(slice(0, rows), slice(cut, n))], axis=0)
+    shards = np.concatenate([product(slice(0, row_cut), slice(0, n)), product(slice(row_cut, rows), slice(0, n))], axis=1)
+    assert np.abs(chunks - whole).max() <= bar and np.abs(shards - whole).max() <= bar
 
 
 @pytest.mark.parametrize("fmt", ["q6_k", "q8_0"])
@@ -848,7 +891,7 @@ def test_dense_kernel_scale_extremes(dev, oracle, fmt):
     blocks[:, :, at] = d & 0xff
     blocks[:, :, at + 1] = d >> 8
     weight = dev.upload(Tensor(fmt, (rows, cols), blocks.reshape(-1)))
-    w = dev.dequantize(weight).astype(np.float64)
+    w = oracle.dequantize(fmt, blocks.reshape(-1), rows, cols).reshape(rows, cols).astype(np.float64)
     x = rng.standard_normal((n, cols)).astype(np.float32)
     out = dev.alloc(n * rows)
     dev.matmul(out, weight, dev.buffer(x))
@@ -862,12 +905,12 @@ def test_dense_kernel_scale_extremes(dev, oracle, fmt):
 def test_dense_kernel_shares_k_between_blocks(dev, oracle, fmt, rows, cols, n):
     """The dense kernel with one to eight blocks on a tile (uneven shares of K, ragged rows and tokens), with
     the three epilogues.  The tensor cores' additions within a unit are not rounded to nearest: 2e-5 of the
-    result's root mean square (measured 5e-6)."""
+    result's root mean square (the largest difference measured at any K is 4.2e-6 of it)."""
     rng = np.random.default_rng(rows + n)
-    weight = dev.upload(dev.quantize(fmt, (0.02 * rng.standard_normal((rows, cols))).astype(np.float32)))
+    weight, w, other, w2 = random_pair(dev, oracle, fmt, rows, cols, rng)
     x = rng.standard_normal((n, cols)).astype(np.float32)
     xb, out, again = dev.buffer(x), dev.alloc(n * rows), dev.alloc(n * rows)
-    want = x.astype(np.float64) @ dev.dequantize(weight).astype(np.float64).T
+    want = x.astype(np.float64) @ w.T
     bar = 2e-5 * np.sqrt((want ** 2).mean())
     dev.matmul(out, weight, xb)
     got = dev.read(out)
@@ -878,8 +921,8 @@ def test_dense_kernel_shares_k_between_blocks(dev, oracle, fmt, rows, cols, n):
     acc = dev.buffer(res)
     dev.matmul_add(acc, weight, xb)
     assert np.abs(dev.read(acc).reshape(n, rows) - (want + res)).max() <= bar + 1e-6
-    dev.swiglu(out, weight, weight, xb, again)
-    silu = want / (1 + np.exp(-want)) * want
+    dev.swiglu(out, weight, other, xb, again)
+    silu = silu_times(want, x.astype(np.float64) @ w2.T)
     assert np.abs(dev.read(out).reshape(n, rows) - silu).max() <= 4 * bar * max(1.0, np.abs(want).max())
 
 
@@ -913,10 +956,10 @@ def test_gemm_fused_epilogues_at_256_columns(dev, oracle, bf16):
 @pytest.mark.parametrize("n,bf16", [(12, False), (33, False), (65, True), (130, False), (300, True)])
 def test_dense_pair_gemm_for_q6_k_and_q8_0(dev, oracle, fmt, n, bf16):
     """Above the small-M kernel's eight tokens Q6_K and Q8_0 go in groups of eight
-    (up to 64 tokens) and then through the dense kernel on dequantized f16 pairs:
-    every tile width, ragged rows, both activation forms, fused epilogues.  The
-    dense kernel sums the whole of K in the tensor cores' accumulator, whose
-    additions are not rounded to nearest: its error grows with K (6e-5 at 5120)."""
+    (up to 64 tokens) and then through the dense kernel, whose weights are pairs of
+    f16 terms: both tile widths, ragged rows, both activation forms, fused epilogues.
+    Against the oracle's fp32 sums: 2e-5 for either path (4.2e-6 of the result's root
+    mean square is the most the dense kernel was measured to be off, at any K)."""
     rng = np.random.default_rng(4000 + n)
     rows, cols = 1030, 2304
     gate = oracle.quantize(fmt, (0.02 * rng.standard_normal((rows, cols))).astype(np.float32))
@@ -931,19 +974,20 @@ def test_dense_pair_gemm_for_q6_k_and_q8_0(dev, oracle, fmt, n, bf16):
     wg, wu = upload(dev, fmt, rows, cols, gate), upload(dev, fmt, rows, cols, up)
     out, scratch = dev.alloc(n * rows), dev.alloc(n * rows)
     dev.matmul(out, wg, xb)
-    assert max_rel_err(dev.read(out), oracle.matmul(fmt, gate, rows, cols, x)) <= (2e-5 if n <= 64 else 1e-4)
+    assert max_rel_err(dev.read(out), oracle.matmul(fmt, gate, rows, cols, x)) <= 2e-5
     dev.swiglu(out, wg, wu, xb, scratch)
-    assert max_rel_err(dev.read(out), oracle.swiglu(fmt, gate, up, rows, cols, x)) <= 1e-4
+    # either product's error times the other factor, at most 4.5 of its rms: 4.2e-6 * 4.5 * 2 over silu(g) u's smaller rms
+    assert max_rel_err(dev.read(out), oracle.swiglu(fmt, gate, up, rows, cols, x)) <= 8e-5
     res = rng.standard_normal((n, rows)).astype(np.float32)
     acc = dev.buffer(res)
     dev.matmul_add(acc, wu, xb)
     got, want = dev.read(acc).reshape(n, rows), oracle.matmul_add(fmt, up, rows, cols, x, res)
-    assert max_rel_err(got - res, want - res) <= 1e-4
+    assert max_rel_err(got - res, want - res) <= 2e-5
 
 
 @pytest.mark.parametrize("fmt,rows,cols,n", [("q6_k", 151936, 5120, 128), ("q8_0", 5120, 5120, 2048), ("q6_k", 20000, 5120, 512)])
 def test_dense_pair_gemm_full_size(dev, oracle, fmt, rows, cols, n):
-    """Config 3's matrices at GEMM sizes: several row panels (the vocabulary head),
+    """The head's and the projections' matrices at GEMM sizes through the dense kernel,
     against the oracle on sampled rows and every token."""
     rng = np.random.default_rng(4100 + n)
     srows = 2048                                      # distinct rows; the matrix repeats them (generation time)
@@ -960,7 +1004,7 @@ def test_dense_pair_gemm_full_size(dev, oracle, fmt, rows, cols, n):
     sample = sampled_rows(rows, rng)
     rb = row_bytes(fmt, cols)
     want = oracle.matmul(fmt, blocks.reshape(rows, rb)[sample].reshape(-1), sample.size, cols, x)
-    assert max_rel_err(got[:, sample], want) <= 2e-4
+    assert max_rel_err(got[:, sample], want) <= 2e-5
 
 
 # ---- the boundary: a caller's stream, a caller's writes -----------------------------------------
