@@ -6,6 +6,8 @@
 // sub-block means and a scale per token for the tensor-core kernels; either
 // can be written by the same launch that applies the RMS norm in front of the
 // product (rmsnorm.cu:11-58).
+#include <type_traits>
+
 #include "common.cuh"
 #include "ptx.cuh"
 
@@ -183,35 +185,90 @@ size_t gemm_operand_bytes(size_t cols, size_t n, int split) {
     return ncols * cols * sizeof(__half) + ncols * (cols / 256) * 16 * sizeof(__half) + ((n * sizeof(float) + 15) & ~size_t(15));
 }
 
-// Reductions over a block of THREADS, every thread the result.
+// Reductions over a block of THREADS and its cluster (`cluster` blocks share a row), every thread the
+// result: the warps' values through shared memory, the blocks' through each other's, both in a fixed order.
+constexpr size_t OPERAND_MAX_COLS = 51200;
+struct RowScratch {
+    float warps[16];
+    float blocks[8];
+};
 template <int THREADS>
-__device__ __forceinline__ float block_max(float v, float *scratch) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    __syncthreads();                                   // scratch may still be read from the reduction before
-    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
+__device__ __forceinline__ float row_sum(float v, RowScratch &s, int rank, int cluster) {
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) s.warps[threadIdx.x >> 5] = v;
     __syncthreads();
-    v = scratch[0];
+    v = s.warps[0];
 #pragma unroll
-    for (int i = 1; i < THREADS / 32; i++) v = fmaxf(v, scratch[i]);
+    for (int i = 1; i < THREADS / 32; i++) v += s.warps[i];
+    if (cluster > 1) {
+        cluster_wait();                     // opened at the kernel's start: all the row's blocks run
+        if ((int)threadIdx.x < cluster) st_cluster_f32(smem_u32(s.blocks + rank), threadIdx.x, v);
+        cluster_sync();
+        v = s.blocks[0];
+        for (int i = 1; i < cluster; i++) v += s.blocks[i];
+    }
     return v;
 }
+// The largest of non-negative floats' bits (a NaN's are above infinity's).
 template <int THREADS>
-__device__ __forceinline__ float block_sum(float v, float *scratch) {
-    v = warp_sum(v);
+__device__ __forceinline__ uint32_t row_max(uint32_t v, RowScratch &s, int rank, int cluster, bool met) {
+    v = __reduce_max_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0) s.warps[threadIdx.x >> 5] = __uint_as_float(v);
     __syncthreads();
-    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float s = scratch[0];
+    v = __float_as_uint(s.warps[0]);
 #pragma unroll
-    for (int i = 1; i < THREADS / 32; i++) s += scratch[i];      // warp order: the same sum on every thread
-    return s;
+    for (int i = 1; i < THREADS / 32; i++) v = max(v, __float_as_uint(s.warps[i]));
+    if (cluster > 1) {
+        if (!met) cluster_wait();
+        if ((int)threadIdx.x < cluster) st_cluster_f32(smem_u32(s.blocks + rank), threadIdx.x, __uint_as_float(v));
+        cluster_sync();
+        v = __float_as_uint(s.blocks[0]);
+        for (int i = 1; i < cluster; i++) v = max(v, __float_as_uint(s.blocks[i]));
+    }
+    return v;
 }
 
-// One block of OPERAND_THREADS per token row; the row passes through shared memory
-// (cols floats of dynamic shared memory).  Bound by the row's chain of loads, two
-// reductions and stores, not by its bytes: for 16 tokens of 17408 11.2 us with 256 threads, 9.0 with
-// 512; a feed-forward block of 16 tokens 95.3 and 93.0.
+// Four values as f16 (hi) and what the rounding left, as f16 (lo), in the order (0, 2, 1, 3): the order the
+// weights' bytes decode in; sh and sl: the terms' sums.
+struct Terms {
+    uint2 hi, lo;
+    float sh, sl;
+};
+__device__ __forceinline__ uint32_t pack_f16(float a, float b) {
+    uint32_t r;
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+    return r;
+}
+template <bool SPLIT> __device__ __forceinline__ Terms terms_finite(const float (&f)[4]) {
+    Terms t;
+    t.hi = make_uint2(pack_f16(f[0], f[2]), pack_f16(f[1], f[3]));
+    const float h0 = h2f_lo(t.hi.x), h2 = h2f_hi(t.hi.x), h1 = h2f_lo(t.hi.y), h3 = h2f_hi(t.hi.y);
+    t.sh = (h0 + h1) + (h2 + h3);
+    if (!SPLIT) return t;
+    t.lo = make_uint2(pack_f16(f[0] - h0, f[2] - h2), pack_f16(f[1] - h1, f[3] - h3));
+    t.sl = (h2f_lo(t.lo.x) + h2f_lo(t.lo.y)) + (h2f_hi(t.lo.x) + h2f_hi(t.lo.y));
+    return t;
+}
+// The same where a value may be an infinity or a NaN: clamped to f16's largest.
+__device__ __noinline__ Terms terms_clamped(float f0, float f1, float f2, float f3) {
+    const float f[4] = {f0, f1, f2, f3};
+    uint32_t hi[4], lo[4];
+    Terms t;
+    t.sh = t.sl = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        hi[i] = to_f16_bits(f[i]);
+        lo[i] = to_f16_bits(f[i] - from_f16_bits(hi[i]));
+        t.sh += from_f16_bits(hi[i]);
+        t.sl += from_f16_bits(lo[i]);
+    }
+    t.hi = make_uint2(hi[0] | hi[2] << 16, hi[1] | hi[3] << 16);
+    t.lo = make_uint2(lo[0] | lo[2] << 16, lo[1] | lo[3] << 16);
+    return t;
+}
+
+// A block per token row, or a cluster of up to eight; the row in chunks of THREADS * 4 activations (four a
+// thread), dealt to the blocks in turn, R of them a block, and held in registers until its largest magnitude is known.
 //   NORM: the row is first normalized by its root mean square and multiplied
 //   by `weight` (Cpu::rmsnorm, gpu/cpu.rs:157-166: v * (scale * w) with
 //   scale = 1 / sqrt(sum(v^2) / dim + eps)); the f32 result goes to `xout`.
@@ -223,96 +280,93 @@ __device__ __forceinline__ float block_sum(float v, float *scratch) {
 // again.  (Rows of typical normalized activations, largest magnitude 4 to 8,
 // are not scaled at all.  Scaling them up instead, to just below f16's
 // maximum, was measured to slow the tensor-core kernel by half: the same
-// kernel on larger operand magnitudes runs into the power limit earlier.)  A thread takes
-// four consecutive activations per round, eight threads a 32-wide sub-block,
-// 64 a unit, the block eight units.
-constexpr int OPERAND_THREADS = 512;
-template <bool NORM, bool ALIGNED>   // ALIGNED: x (and xout, weight) are 16-byte aligned (a wrapped caller's pointer need not be)
-__global__ void __launch_bounds__(OPERAND_THREADS) gemm_operand_kernel(const float *x, const float *__restrict__ weight, float eps,
-                                                           float *xout, size_t cols, size_t units, int split,
-                                                           __half *__restrict__ x16, __half *__restrict__ means,
-                                                           float *__restrict__ tok_scale) {
+// kernel on larger operand magnitudes runs into the power limit earlier.)
+template <bool NORM, bool SPLIT, int THREADS, int R>
+__global__ void __launch_bounds__(THREADS, THREADS == 512 ? (R > 9 ? 1 : 2) : R > 3 ? 5 : 6) gemm_operand_kernel(const float *x, const float *__restrict__ weight, float eps, float *xout,
+                                                               size_t cols, size_t units, int cluster, __half *__restrict__ x16,
+                                                               __half *__restrict__ means, float *__restrict__ tok_scale) {
+    if (cluster > 1) cluster_arrive();
     // as the small-M prologues: let the product's kernel begin (it streams weights first),
     // wait for the kernel ahead, which may still read the operand or write x
     griddep_launch();
     griddep_wait();
-    extern __shared__ __align__(16) float row[];
-    __shared__ float scratch[OPERAND_THREADS / 32];
-    constexpr size_t STEP = OPERAND_THREADS * 4;
-    const int t = blockIdx.x, k = threadIdx.x;
-    const float *src = x + (size_t)t * cols;
-    float amax = 0.0f, ssq = 0.0f;
-#pragma unroll 3
-    for (size_t at = (size_t)k * 4; at < cols; at += STEP) {
-        float4 v;
-        if (ALIGNED) v = *reinterpret_cast<const float4 *>(src + at);
-        else v = make_float4(src[at], src[at + 1], src[at + 2], src[at + 3]);
-        *reinterpret_cast<float4 *>(row + at) = v;
-        if (NORM) ssq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-        else amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fmaxf(fabsf(v.z), fabsf(v.w)), amax));
-    }
-    if (NORM) {
-        const float total = block_sum<OPERAND_THREADS>(ssq, scratch);
-        const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, (float)cols), eps)));
-        float *dst = xout + (size_t)t * cols;
-        for (size_t at = (size_t)k * 4; at < cols; at += STEP) {
-            float4 v = *reinterpret_cast<float4 *>(row + at), w;
-            if (ALIGNED) w = *reinterpret_cast<const float4 *>(weight + at);
-            else w = make_float4(weight[at], weight[at + 1], weight[at + 2], weight[at + 3]);
-            v.x = __fmul_rn(v.x, __fmul_rn(scale, w.x));
-            v.y = __fmul_rn(v.y, __fmul_rn(scale, w.y));
-            v.z = __fmul_rn(v.z, __fmul_rn(scale, w.z));
-            v.w = __fmul_rn(v.w, __fmul_rn(scale, w.w));
-            *reinterpret_cast<float4 *>(row + at) = v;
-            if (ALIGNED) *reinterpret_cast<float4 *>(dst + at) = v;
-            else { dst[at] = v.x; dst[at + 1] = v.y; dst[at + 2] = v.z; dst[at + 3] = v.w; }
-            amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fmaxf(fabsf(v.z), fabsf(v.w)), amax));
-        }
-    }
-    amax = block_max<OPERAND_THREADS>(amax, scratch);
-    // amax in [2^(b-127), 2^(b-126)) for its biased exponent b; e = b - 127 - 2, kept where 2^e and
-    // 2^-e are normal floats (a row of zeros, subnormals or infinities takes the nearest end)
-    int e = (int)((__float_as_uint(amax) >> 23) & 0xffu) - 129;
-    e = amax > 0.0f ? max(-100, min(100, e)) : 0;
-    const float down = __uint_as_float((uint32_t)(127 - e) << 23);
-    if (k == 0) tok_scale[t] = __uint_as_float((uint32_t)(127 + e) << 23);
-    const size_t col = split ? 2 * (size_t)t : (size_t)t;
-    for (size_t at = (size_t)k * 4; at < cols; at += STEP) {
-        const float4 v = *reinterpret_cast<float4 *>(row + at);
-        const float f[4] = {v.x * down, v.y * down, v.z * down, v.w * down};
-        __half hi[4], lo[4];
-        float sh = 0.0f, sl = 0.0f;
+    __shared__ RowScratch s[3];
+    const int rank = (int)(blockIdx.x % cluster), k = threadIdx.x;
+    const size_t t = blockIdx.x / cluster;
+    const float *src = x + t * cols;
+    // this thread's place in its block's chunk r; whole warps are in or out (cols is whole units)
+    auto place = [&](int r) { return ((size_t)(rank + cluster * r) * THREADS + k) * 4; };
+    float4 v[R];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            hi[i] = to_f16_clamped(f[i]);
-            lo[i] = to_f16_clamped(f[i] - __half2float(hi[i]));
-            sh += __half2float(hi[i]);
-            sl += __half2float(lo[i]);
+    for (int r = 0; r < R; r++) v[r] = place(r) < cols ? *reinterpret_cast<const float4 *>(src + place(r)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (NORM) {
+        float4 w[R];      // (fetched ahead of the sum where the registers last)
+        constexpr bool AHEAD = R <= 3;
+#pragma unroll
+        for (int r = 0; r < R && AHEAD; r++) w[r] = place(r) < cols ? *reinterpret_cast<const float4 *>(weight + place(r)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float ssq = 0.0f;
+#pragma unroll
+        for (int r = 0; r < R; r++) ssq += (v[r].x * v[r].x + v[r].y * v[r].y) + (v[r].z * v[r].z + v[r].w * v[r].w);
+        const float total = row_sum<THREADS>(ssq, s[0], rank, cluster);
+        const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, (float)cols), eps)));
+        float *dst = xout + t * cols;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            if (!AHEAD) w[r] = place(r) < cols ? *reinterpret_cast<const float4 *>(weight + place(r)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            v[r].x = __fmul_rn(v[r].x, __fmul_rn(scale, w[r].x));
+            v[r].y = __fmul_rn(v[r].y, __fmul_rn(scale, w[r].y));
+            v[r].z = __fmul_rn(v[r].z, __fmul_rn(scale, w[r].z));
+            v[r].w = __fmul_rn(v[r].w, __fmul_rn(scale, w[r].w));
+            if (place(r) < cols) *reinterpret_cast<float4 *>(dst + place(r)) = v[r];
         }
-        // a group of four goes out in the order (0, 2, 1, 3): the order the weights' bytes decode in
-        auto pack = [](const __half (&h)[4]) {
-            uint2 r;
-            r.x = (uint32_t)__half_as_ushort(h[0]) | ((uint32_t)__half_as_ushort(h[2]) << 16);
-            r.y = (uint32_t)__half_as_ushort(h[1]) | ((uint32_t)__half_as_ushort(h[3]) << 16);
-            return r;
-        };
-        *reinterpret_cast<uint2 *>(x16 + col * cols + at) = pack(hi);
-        if (split) *reinterpret_cast<uint2 *>(x16 + (col + 1) * cols + at) = pack(lo);
-        // sub-block sums over the eight threads that share it (cols is whole units: whole warps take part)
+    }
+    auto largest = [&](uint32_t limit) {     // of the magnitudes whose bits are below the limit
+        uint32_t m = 0;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const float f[4] = {v[r].x, v[r].y, v[r].z, v[r].w};
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const uint32_t b = __float_as_uint(f[i]) & 0x7fffffffu;
+                if (b < limit) m = max(m, b);
+            }
+        }
+        return m;
+    };
+    uint32_t top = row_max<THREADS>(largest(0x80000000u), s[1], rank, cluster, NORM);
+    const bool finite = top < 0x7f800000u;
+    if (!finite) top = row_max<THREADS>(largest(0x7f800001u), s[2], rank, cluster, true);     // a NaN is passed over
+    // the largest in [2^(b-127), 2^(b-126)) for its biased exponent b; e = b - 127 - 2, kept where 2^e and
+    // 2^-e are normal floats (a row of zeros, subnormals or infinities takes the nearest end)
+    const int e = top ? max(-100, min(100, (int)(top >> 23) - 129)) : 0;
+    const float down = __uint_as_float((uint32_t)(127 - e) << 23);
+    if (rank == 0 && k == 0) tok_scale[t] = __uint_as_float((uint32_t)(127 + e) << 23);
+    const size_t col = SPLIT ? 2 * t : t;
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const size_t at = place(r);
+        if (at >= cols) break;
+        const float f[4] = {v[r].x * down, v[r].y * down, v[r].z * down, v[r].w * down};
+        Terms y;
+        if (finite) y = terms_finite<SPLIT>(f);
+        else y = terms_clamped(f[0], f[1], f[2], f[3]);
+        *reinterpret_cast<uint2 *>(x16 + col * cols + at) = y.hi;
+        if (SPLIT) *reinterpret_cast<uint2 *>(x16 + (col + 1) * cols + at) = y.lo;
+        // sub-block sums over the eight threads that share it
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) {
-            sh += __shfl_xor_sync(0xffffffffu, sh, o);
-            sl += __shfl_xor_sync(0xffffffffu, sl, o);
+            y.sh += __shfl_xor_sync(0xffffffffu, y.sh, o);
+            if (SPLIT) y.sl += __shfl_xor_sync(0xffffffffu, y.sl, o);
         }
         if ((k & 7) == 0) {
             const size_t u = at >> 8;
             const int j = (int)(at & 255) >> 5;
-            const float mh = sh * (1.0f / 32.0f), ml = sl * (1.0f / 32.0f);
+            const float mh = y.sh * (1.0f / 32.0f), ml = y.sl * (1.0f / 32.0f);
             __half *m = means + (col * units + u) * 16;
             const __half a = to_f16_clamped(mh);
             m[j] = a;
             m[8 + j] = to_f16_clamped(mh - __half2float(a));
-            if (split) {
+            if (SPLIT) {
                 __half *m2 = m + units * 16;
                 const __half b = to_f16_clamped(ml);
                 m2[j] = b;
@@ -331,16 +385,40 @@ int build_gemm_operand(dwim_b200_ctx *ctx, const float *x, size_t n, size_t cols
     const size_t units = cols / 256, ncols = n * (split ? 2 : 1);
     __half *means = out + ncols * cols;
     float *tok_scale = reinterpret_cast<float *>(means + ncols * units * 16);
-    const size_t smem = cols * sizeof(float);
-    if (smem > 200 * 1024) return fail(ctx, DWIM_B200_EINVAL, "GEMM operand: rows of %zu activations are too long", cols);
-    const bool norm = weight != nullptr;
-    const bool aligned = reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(weight) % 16 == 0 &&
-                         reinterpret_cast<uintptr_t>(xout) % 16 == 0;
-    auto kern = norm ? (aligned ? gemm_operand_kernel<true, true> : gemm_operand_kernel<true, false>)
-                     : (aligned ? gemm_operand_kernel<false, true> : gemm_operand_kernel<false, false>);
-    if (smem > 47 * 1024) DWIM_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    DWIM_CUDA(ctx, launch_dependent(!ctx->weights_written, kern, dim3((unsigned)n), dim3(OPERAND_THREADS), smem, ctx->stream, x,
-                                    weight, eps, xout, cols, units, split, out, means, tok_scale));
+    if (cols > OPERAND_MAX_COLS) return fail(ctx, DWIM_B200_EINVAL, "GEMM operand: rows of %zu activations are too long", cols);
+    // A block a row once there are rows for every SM; below that as many blocks a row as there are SMs for.
+    // Bound by a row's chain of load, reduction and store at few rows, by the bytes and the conversion's
+    // instructions at many (the bytes of 2048 rows of 17408 f32 are 33 to 44 us).  The kernel alone, us, by cluster:
+    // 16 rows of 17408 4.2 with eight blocks (9.0 with the row in one block's shared memory, as it was), 131 rows 5.9
+    // with one; 16 rows of 5120 3.4 with five, 3.8 with one; 512 rows 6.6 with one, 9.0 with two; 2048 rows
+    // 13.1 with one, 24 with two (a cluster's blocks start and end together); 2048 rows of 17408 51 as one
+    // block of 512 threads (64 with both terms), 69 as four of 256.
+    const size_t chunks = (cols + 1023) / 1024;
+    size_t cluster = (size_t)ctx->sm_count / n;
+    if (cluster < 1) cluster = 1;
+    if (cluster > 8) cluster = 8;
+    if (cluster > chunks) cluster = chunks;
+    size_t each = (chunks + cluster - 1) / cluster;     // in chunks of 1024
+    const bool wide = each > 5;                         // 512 threads, chunks of 2048
+    if (wide) {
+        each = (chunks + 2 * cluster - 1) / (2 * cluster);
+        each = each <= 5 ? 5 : each <= 9 ? 9 : 13;
+        cluster = ((chunks + 1) / 2 + each - 1) / each;
+    } else {
+        each = each <= 3 ? each : 5;
+        cluster = (chunks + each - 1) / each;
+    }
+    auto pick = [&](auto norm, auto terms) {
+        constexpr bool N = decltype(norm)::value, S = decltype(terms)::value;
+        if (wide) return each == 5 ? gemm_operand_kernel<N, S, 512, 5> : each == 9 ? gemm_operand_kernel<N, S, 512, 9> : gemm_operand_kernel<N, S, 512, 13>;
+        return each == 1 ? gemm_operand_kernel<N, S, 256, 1> : each == 2 ? gemm_operand_kernel<N, S, 256, 2>
+               : each == 3 ? gemm_operand_kernel<N, S, 256, 3> : gemm_operand_kernel<N, S, 256, 5>;
+    };
+    using T = std::true_type;
+    using F = std::false_type;
+    auto kern = weight ? (split ? pick(T(), T()) : pick(T(), F())) : (split ? pick(F(), T()) : pick(F(), F()));
+    DWIM_CUDA(ctx, launch_clustered(!ctx->weights_written, (unsigned)cluster, kern, dim3((unsigned)(n * cluster)), dim3(wide ? 512 : 256), 0,
+                                    ctx->stream, x, weight, eps, xout, cols, units, (int)cluster, out, means, tok_scale));
     DWIM_LAUNCHED(ctx);
     return 0;
 }

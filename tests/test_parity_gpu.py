@@ -582,6 +582,39 @@ def test_gemm_activation_range(dev, oracle, scale, bf16):
         assert max_rel_err(got[t], want[t]) <= 2e-5, (t, max_rel_err(got[t], want[t]))
 
 
+@pytest.mark.parametrize("cols", [256, 1024, 3328, 5120, 5376, 6144, 10496, 18432, 18688, 26880])
+@pytest.mark.parametrize("n,norm", [(9, False), (9, True), (40, False), (150, True), (300, False)])
+def test_gemm_operand_rows_of_every_length(dev, oracle, cols, n, norm):
+    """The tensor-core kernels' operand, rows held by one block or a cluster's, in whole chunks of 1024 and 2048 and
+    a rest: a norm's row and its product, an infinite and a NaN activation that stay their token's own."""
+    rng = np.random.default_rng(cols + n)
+    rows = 16
+    blocks = oracle.quantize("q4_k", (0.02 * rng.standard_normal((rows, cols))).astype(np.float32))
+    w = oracle.dequantize("q4_k", blocks, rows, cols).reshape(rows, cols).astype(np.float64)
+    x = rng.standard_normal((n, cols)).astype(np.float32)
+    x[2, cols - 1] = 50.0
+    out, xb = dev.alloc(n * rows), dev.buffer(x)
+    x = x.astype(np.float64)
+    if norm:
+        gain = (1 + 0.1 * rng.standard_normal(cols)).astype(np.float32)
+        xn = dev.alloc(n * cols)
+        dev.normalize(xn, xb, dev.buffer(gain), n * cols, 1e-6)
+        x = x / np.sqrt((x * x).mean(1, keepdims=True) + 1e-6) * gain
+        # scale and product rounded to fp32 each, a sum of cols terms: a few 2^-24
+        assert max_rel_err(dev.read(xn), x) <= 2e-6
+        xb = xn
+    elif n == 9:
+        bad = x.astype(np.float32)
+        bad[4, cols // 2], bad[5, 3] = np.inf, np.nan
+        dev.write(xb, bad)
+    dev.matmul(out, upload(dev, "q4_k", rows, cols, blocks), xb)
+    got, want = dev.read(out).reshape(n, rows), x @ w.T
+    assert np.isfinite(got).all()
+    good = [t for t in range(n) if norm or n != 9 or t not in (4, 5)]
+    # fp32 sums of up to 26880 products, f16 pairs for the activations (2^-22): 1e-5 of the result's magnitude
+    assert max_rel_err(got[good], want[good]) <= 1e-5
+
+
 # ---- the operators either side of the product (the norm before it, the arg-max after it, bf16 matrices) ----
 def test_normalize_matches_cpu(dev, oracle):
     """normalize_matches_cpu (gpu/tests.rs:788-812): the reference's shapes and
