@@ -21,7 +21,7 @@ static constexpr size_t WEIGHT_SLACK = 1024;
 namespace dwim {
 // gemm.cu
 bool gemm_supports(const WeightView &w);
-int gemm_large(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, size_t n, int split, const OutSpec &out,
+int gemm_large(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, size_t n, int terms, const OutSpec &out,
                const float *aux, int epilogue);
 
 int reserve_shadow(dwim_b200_ctx *ctx, dwim_b200_buffer *b, size_t need) {
@@ -506,8 +506,6 @@ static int product(dwim_b200_ctx *ctx, const OutSpec &out, size_t out_len, const
     REQUIRE(ctx, out.dst[0] != x->data, DWIM_B200_EINVAL, "%s: output aliases input", what);
     // bf16 weights (the small gate matrices): f32 activations as they are, fp32 throughout
     if (v.fmt == BF16) return matmul_bf16(ctx, v, x->data, n, out, aux, epilogue);
-    // bf16 activations are exact in one f16 column; f32 ones travel as two
-    // (value and rounding remainder), summed again in the epilogue.
     // Up to eight tokens: the small-M kernel's int8 routines.  Above: the tensor-core kernels -- Q4_K
     // from nine tokens on (measured on B200 at [17408, 5120]: 26 us at nine to sixteen tokens, against
     // 57 us for sixteen through two small-M launches); Q6_K and Q8_0 from 65 on, and in groups of eight through
@@ -516,12 +514,11 @@ static int product(dwim_b200_ctx *ctx, const OutSpec &out, size_t out_len, const
     // activations and 1.2e-7 by bf16 ones.)
     const bool dense = gemm_supports(v) && n > (v.fmt == Q4_K ? (size_t)I8_MAX_TOKENS : (size_t)64);
     if (dense) {
-        // bf16 activations are exact in one f16 column; f32 ones travel as two
-        // (value and rounding remainder), summed again in the epilogue.
+        // bf16 activations are exact in one f16 term; f32 ones travel as two (value and rounding remainder)
         int split = x->bf16_exact || ctx->act_f16 ? 0 : 1;
         int rc = ensure_shadow(ctx, x, SHADOW_GEMM, v.cols, split);
         if (rc) return rc;
-        return gemm_large(ctx, v, (const __half *)x->shadow, n, split, out, aux, epilogue);
+        return gemm_large(ctx, v, (const __half *)x->shadow, n, split ? 2 : 1, out, aux, epilogue);
     }
     if (!gemv_takes_i8(v, n < (size_t)I8_MAX_TOKENS ? n : (size_t)I8_MAX_TOKENS))
         return fail(ctx, DWIM_B200_EFORMAT, "%s: no kernel takes format %d with %zu columns", what, v.fmt, v.cols);

@@ -15,21 +15,24 @@
 // bits each), and a power of two moves between d and the operands when dmin/d
 // is large (q4k_fold below).  The reference's tile kernel rounds every
 // dequantized weight to f16 instead (matmul_tile.cu:66-74): 2e-4 of rms error
-// against 5e-7 here.  An f32 activation travels as two f16 columns, value and
-// rounding remainder, which the epilogue adds up again; a bf16 one is exact in
-// one column.
+// against 5e-7 here.  An f32 activation travels as two f16 terms, value and
+// rounding remainder; a bf16 one is exact in one.  The terms share a token's
+// decoded weights and its minimums (whose means are of the activations
+// themselves), and from 129 tokens on its accumulator.  (As two columns with
+// sums, minimums and an epilogue of their own, a tile was half as many tokens:
+// [17408, 5120] by 2048 f32 tokens 827 us then, 690 now.)
 //
 // A CTA owns 128 weight rows (one TMEM lane each) by BN columns (32..256):
-//   warp 0        activations' producer (one thread): per K block of 64 the f16
+//   warp 16       activations' producer (one thread): per K block of 64 the f16
 //                 tile [BN][64] (TMA, 128-byte swizzle) into the B ring; per
 //                 unit the sub-block means' hi and lo parts.
-//   warp 1        MMA issuer: tcgen05.mma M=128 N=BN K=16 into the unit's
+//   warp 17       MMA issuer: tcgen05.mma M=128 N=BN K=16 into the unit's
 //                 accumulator buffer (two buffers, so unit u+1 multiplies
 //                 while unit u drains).  The whole warp runs the loop and one
 //                 lane issues: that thread has about one instruction slot per
 //                 five cycles, and an N=128 MMA leaves it 64 cycles.
-//   warps 2-17    workers.  Warp w owns TMEM lane quadrant w % 4 (weight rows
-//                 32*(w % 4) + lane) and K block (w - 2) / 4 of every unit:
+//   warps 0-15    workers.  Warp w owns TMEM lane quadrant w % 4 (weight rows
+//                 32*(w % 4) + lane) and K block w / 4 of every unit:
 //                 thread = row turns the block's 64 nibbles into sc*q halves
 //                 (lop3 magic number + one HFMA2 per two weights) and stores
 //                 them into the stage's A tile in the K-major 128-byte-
@@ -43,12 +46,16 @@
 //                 blocks [128 rows][144 B] from HBM into the raw ring.
 // Where the tiles do not fill the chip, a cluster's blocks share a tile's K and add up
 // through each other's shared memory (pick_split).
+// Warp 19 makes whole warpgroups of them, which trade registers: 96 a thread at launch,
+// 104 for a worker then.  (At 96 the 256-column form spilled in its main loop: [17408,
+// 5120] by 2048 bf16 tokens 391 us, 375 like this; with 100 bytes of spills 442.)
 // Every mbarrier wait is bounded (ptx.cuh); a kernel that gave up says so in
 // the context's status word.
 #include <cuda.h>
 #include <stdlib.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 #include "ptx.cuh"
@@ -63,9 +70,15 @@ constexpr int TILE_M = 128;   // weight rows per CTA
 constexpr int BK = 64;        // K per stage: one 128-byte swizzled row of f16
 constexpr int KBLOCKS = 4;    // K blocks per unit; each is a stage of the A ring and a hand-over of its own
 constexpr int SCALE_SLOTS = 4;
-constexpr int N_WORKERS = 16;                                      // warps 2..17: four per TMEM lane quadrant
-constexpr int RAW_WARP = 2 + N_WORKERS;                            // the packed weights' producer
-constexpr int GEMM_THREADS = (3 + N_WORKERS) * 32;
+constexpr int N_WORKERS = 16;                                      // warps 0..15: four per TMEM lane quadrant
+constexpr int X_WARP = 16, MMA_WARP = 17, RAW_WARP = 18;           // the activations' producer, the issuer, the weights' producer
+constexpr int GEMM_THREADS = 640;                                  // whole warpgroups (one warp has no role)
+// A thread's registers are 96 at launch (65536 / 640, whole eights); the four warps without sums give some of theirs to
+// the workers.  The dense kernel's workers take all there are ([12288, 5120] Q6_K by 512 f32 tokens 213 us with the
+// Q4_K kernel's shares, 208 with these); the Q4_K kernel's issuer wants more than 32 (375 and 387 us).
+constexpr int WORKER_REGS = 104, OTHER_REGS = 56, DENSE_WORKER_REGS = 112, DENSE_OTHER_REGS = 32;
+static_assert(512 * WORKER_REGS + 128 * OTHER_REGS <= 640 * 96 && 512 * DENSE_WORKER_REGS + 128 * DENSE_OTHER_REGS <= 640 * 96,
+              "a warpgroup would wait for registers that nobody gives up");
 constexpr int RAW_BYTES = ((TILE_M * 144 + 1023) / 1024) * 1024;   // 18 KB
 constexpr int A_BYTES = TILE_M * BK * 2;                           // 16 KB
 constexpr int AMIN_BYTES = TILE_M * 16 * 4;                        // 8 KB: [K group of 8][row][16 B], four groups
@@ -74,8 +87,8 @@ constexpr int BAR_BYTES = 1024;
 constexpr int MAX_SPLIT = 8;                                       // blocks of a portable cluster
 
 struct GemmArgs {
-    size_t rows, n, ncols, units;   // weight rows, tokens, operand columns, 256-weight units of K
-    int split;                      // 1: columns 2t, 2t+1 are token t's hi and lo halves
+    size_t rows, n, units;          // weight rows, tokens, 256-weight units of K
+    int terms;                      // f16 terms of an activation: 1, or 2 (value and rounding remainder)
     OutSpec out;
     const float *tok_scale;         // per token: the power of two its activations were divided by (prologue.cu)
     const float *aux;               // EPI_SWIGLU: the `up` product, token-major [n][rows]
@@ -84,7 +97,11 @@ struct GemmArgs {
     uint32_t *status;
 };
 
-// Per tile width.  Up to 192 columns the B ring has as many stages as the A
+// The terms of an activation: one alone; up to two, the second's columns beside the first's, one MMA for both
+// (while that is at most 256 columns); or two that take turns on one accumulator.
+enum Mode : int { ONE_TERM, SIDE_BY_SIDE, TWO_PASSES };
+
+// Per tile width.  Up to 192 columns of one MMA the B ring has as many stages as the A
 // ring.  Up to 128 these are one and a quarter to two units deep, so that the
 // workers decode a unit while the one before multiplies ([5120, 17408] by 16
 // tokens: 41 us one unit deep, 38 like this; [17408, 5120] by 48 tokens 39.1
@@ -93,12 +110,13 @@ struct GemmArgs {
 // as often, an MMA takes 128 cycles, and shared memory is the limit: three B
 // stages, two raw stages, one stage of the minimums' operands (a B stage is
 // reloaded as soon as its own K block is done).
-template <int BN> struct Cfg {
-    static constexpr int A_STAGES = BN <= 32 ? 8 : BN <= 64 ? 6 : BN <= 128 ? 5 : KBLOCKS;
-    static constexpr int B_STAGES = BN > 192 ? 3 : A_STAGES;
-    static constexpr int RAW_STAGES = BN <= 32 || BN >= 128 ? 2 : 3;
+template <int BN, int MODE> struct Cfg {
+    static constexpr int A_STAGES = BN <= 16 ? 8 : BN <= 32 ? 6 : BN <= (MODE == SIDE_BY_SIDE ? 64 : 128) ? 5 : KBLOCKS;
+    static constexpr int B_STAGES = BN > 192 || (BN == 128 && MODE == SIDE_BY_SIDE) ? 3 : A_STAGES;
+    static constexpr int RAW_STAGES = BN == 32 ? 3 : 2;
     static constexpr int MIN_STAGES = BN > 128 ? 1 : 2;
-    static constexpr int B_BYTES = BN * BK * 2;
+    static constexpr bool WIDE = MODE == SIDE_BY_SIDE;
+    static constexpr int TERM_BYTES = BN * BK * 2, B_BYTES = TERM_BYTES * (WIDE ? 2 : 1), ACC_COLS = BN * (WIDE ? 2 : 1);
     static constexpr int BMIN_BYTES = BN * 16 * 2;                 // [K group of 8][column][16 B]: the means' hi and lo parts
     static constexpr int MIN_BYTES = AMIN_BYTES + ((BMIN_BYTES + 1023) / 1024) * 1024;
     static constexpr int SCALE_BYTES = SCALE_SLOTS * TILE_M * 4;   // the unit's scale per row
@@ -106,7 +124,7 @@ template <int BN> struct Cfg {
     static constexpr int SMEM = BAR_BYTES + A_STAGES * A_BYTES + B_STAGES * B_BYTES + MIN_STAGES * MIN_BYTES +
                                 RAW_STAGES * RAW_BYTES + SCALE_BYTES + TOK_BYTES + 1024;   // + alignment slack
     static_assert(SMEM <= MAX_SMEM, "the tile does not fit shared memory");
-    static constexpr int TMEM_COLS = BN > 128 ? 512 : 2 * BN < 32 ? 32 : 2 * BN;   // two accumulator buffers, a power of two
+    static constexpr int TMEM_COLS = BN > 128 ? 512 : 2 * ACC_COLS;   // two accumulator buffers, a power of two
     static constexpr int DRAIN_COLS = BN / 4 < 16 ? 16 : BN / 4;   // accumulator columns per draining warp
     static constexpr int DRAINERS = BN / DRAIN_COLS;               // draining warps per lane quadrant (4, or 2 at BN=32)
     static constexpr int RINGS = A_STAGES * A_BYTES + B_STAGES * B_BYTES + MIN_STAGES * MIN_BYTES + RAW_STAGES * RAW_BYTES;
@@ -143,6 +161,19 @@ __device__ __forceinline__ void umma_f16_lo(uint32_t d_tmem, uint32_t a_lo, uint
         "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t"
         "}\n" ::"r"(d_tmem),
         "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "n"(ACC)
+        : "memory");
+}
+__device__ __forceinline__ void umma_f16_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, bool acc) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .b64 da, db;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "mov.b64 da, {%1, %3};\n\t"
+        "mov.b64 db, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t"
+        "}\n" ::"r"(d_tmem),
+        "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"((uint32_t)acc)
         : "memory");
 }
 __device__ __forceinline__ void sts128(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
@@ -261,18 +292,6 @@ __device__ __forceinline__ void sum_shares(const float (&acc)[COLS], int q, uint
         for (int j = 0; j < 8; j++) v[j] += r == rank ? acc[8 * q + j] : lds32f(from + j * TILE_M * 4);
     }
 }
-// Eight finished columns from column c on: a token each, or (split) the two terms of four.
-template <bool SHARED>
-__device__ __forceinline__ void emit_columns(const EmitTo &to, size_t rows, size_t n, int split, size_t c, float (&v)[8]) {
-    if (split) {
-        float y[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) y[j] = v[2 * j] + v[2 * j + 1];
-        gemm_emit<SHARED>(to, rows, n, c >> 1, y);
-    } else {
-        gemm_emit<SHARED>(to, rows, n, c, v);
-    }
-}
 
 constexpr uint32_t H2_1024 = 0x64006400u, H2_M1024 = 0xE400E400u, H2_64 = 0x54005400u, H2_M64 = 0xD400D400u;
 
@@ -370,19 +389,22 @@ struct OutMaps {
 // OUT: 0 = one destination (or a scattered one); 1 = a result shared by several ranks, every value
 // stored to each copy from registers; 2 = the same through shared memory and one TMA store per
 // destination and group of columns (whole 512-byte runs over NVLink instead of 4-byte stores).
-template <int BN, int OUT>
+template <int BN, int OUT, int MODE>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                 const __grid_constant__ CUtensorMap tmap_m, const __grid_constant__ GemmArgs a,
                 const __grid_constant__ OutMaps maps) {
     constexpr bool SHARED = OUT == 1;
-    using C = Cfg<BN>;
+    using C = Cfg<BN, MODE>;
+    // One pass over a unit's K blocks: a K block's A and B stages are handed over and released together.
+    constexpr int PASSES = MODE == TWO_PASSES ? 2 : 1;
+    constexpr bool JOINT = PASSES == 1;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;   // the swizzled tiles want 1024-byte alignment
     // barriers, 8 bytes each
-    const uint32_t full0 = base, empty0 = base + 64, minfull0 = base + 128;
-    const uint32_t rawfull0 = base + 160, rawempty0 = base + 192, accfull0 = base + 224, accempty0 = base + 240;
-    const uint32_t tmem_slot = base + 256;
+    const uint32_t afull0 = base, aempty0 = base + 64, bfull0 = base + 128, bempty0 = base + 192, minfull0 = base + 256;
+    const uint32_t rawfull0 = base + 288, rawempty0 = base + 320, accfull0 = base + 352, accempty0 = base + 368;
+    const uint32_t tmem_slot = base + 384;
     const uint32_t astage0 = base + BAR_BYTES;
     const uint32_t bstage0 = astage0 + C::A_STAGES * A_BYTES;
     const uint32_t min0 = bstage0 + C::B_STAGES * C::B_BYTES;
@@ -398,8 +420,12 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::A_STAGES; s++) {
-            mbar_init(full0 + 8 * s, 1 + 4);             // the producer's expect_tx arrival + the K block's worker warps
-            mbar_init(empty0 + 8 * s, 1);                // the MMA warp's commit
+            mbar_init(afull0 + 8 * s, JOINT ? 1 + 4 : 4);   // (the producer's expect_tx arrival +) the K block's worker warps
+            mbar_init(aempty0 + 8 * s, 1);               // the MMA warp's commit
+        }
+        for (int s = 0; s < C::B_STAGES; s++) {
+            mbar_init(bfull0 + 8 * s, 1);                // the producer's expect_tx arrival
+            mbar_init(bempty0 + 8 * s, 1);
         }
         for (int s = 0; s < 2; s++) {
             mbar_init(minfull0 + 8 * s, 1 + 8);          // the producer + the eight warps that write the minimums
@@ -412,7 +438,7 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) {
+    if (warp == MMA_WARP) {
         tmem_alloc(tmem_slot, C::TMEM_COLS);
         tmem_relinquish();
     }
@@ -426,28 +452,33 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     // before their first store.
     griddep_launch();
 
-    if (warp == 0) {
+    if (warp == X_WARP) {
+        regs_dec<OTHER_REGS>();
         // ------------------------------ TMA producer ------------------------------
         griddep_wait();   // the operand comes from the prologue kernel just ahead
         if (elect_one()) {
+            int bs = 0, bturn = 1;
             for (int u = 0; u < units; u++) {
                 const int ms = u % C::MIN_STAGES;
-                for (int h = 0; h < KBLOCKS; h++) {
-                    // B stage kb % B_STAGES was last read by K block kb - B_STAGES.  (The loops of one turn keep
-                    // the compiler's code for the whole loop as it is: written out, however unrolled, a layer of
-                    // 16 tokens takes 161.5 us instead of 160.5.)
-                    for (int g = h; g < h + 1; g++) {
-                        const int prev = KBLOCKS * u + g - C::B_STAGES;
-                        if (prev >= 0)
-                            mbar_wait_parked(empty0 + 8 * (prev % C::A_STAGES), (prev / C::A_STAGES) & 1, a.status, 0x20u);
+                for (int p = PASSES - 1; p >= 0; p--)      // the remainders first
+                    for (int h = 0; h < KBLOCKS; h++) {
+                        uint32_t full = bfull0 + 8 * bs;
+                        if (JOINT) {
+                            // B stage kb % B_STAGES was last read by K block kb - B_STAGES
+                            const int kb = KBLOCKS * u + h, prev = kb - C::B_STAGES;
+                            if (prev >= 0)
+                                mbar_wait_parked(aempty0 + 8 * (prev % C::A_STAGES), (prev / C::A_STAGES) & 1, a.status, 0x20u);
+                            full = afull0 + 8 * (kb % C::A_STAGES);
+                        } else {
+                            mbar_wait_parked(bempty0 + 8 * bs, bturn, a.status, 0x20u);
+                        }
+                        mbar_expect_tx(full, C::TERM_BYTES * (C::WIDE ? a.terms : 1));
+                        const uint32_t to = bstage0 + bs * C::B_BYTES;
+                        const int k = (KBLOCKS * (ub + u) + h) * BK;
+                        tma_load_2d(to, &tmap_x, k, p * (int)a.n + col0, full);
+                        if (C::WIDE && a.terms == 2) tma_load_2d(to + C::TERM_BYTES, &tmap_x, k, (int)a.n + col0, full);
+                        if (++bs == C::B_STAGES) bs = 0, bturn ^= 1;
                     }
-                    const uint32_t full = full0 + 8 * ((u * KBLOCKS + h) % C::A_STAGES);
-                    mbar_expect_tx(full, C::B_BYTES);
-                    for (int g = h; g < h + 1; g++) {
-                        const int kb = KBLOCKS * u + g;
-                        tma_load_2d(bstage0 + (kb % C::B_STAGES) * C::B_BYTES, &tmap_x, (KBLOCKS * ub + kb) * BK, col0, full);
-                    }
-                }
                 // the minimums' stage was last read by unit u - MIN_STAGES
                 if (u >= C::MIN_STAGES) {
                     const int uu = u - C::MIN_STAGES;
@@ -460,6 +491,7 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             }
         }
     } else if (warp == RAW_WARP) {
+        regs_dec<OTHER_REGS>();
         // ------------------------------ packed weights' producer ------------------------------
         // Its own warp: the blocks come from HBM and must run as far ahead as the
         // ring allows, whatever the activations' producer is waiting for.
@@ -471,43 +503,54 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
                 tma_load_2d(raw0 + rs * RAW_BYTES, &tmap_w, (ub + u) * 144, row0, rawfull0 + 8 * rs);
             }
         }
-    } else if (warp == 1) {
+    } else if (warp == MMA_WARP) {
+        regs_dec<OTHER_REGS>();
         // ------------------------------ MMA issuer ------------------------------
         // The whole warp runs the loop (uniform control flow keeps addresses
         // and descriptors on the uniform data path) and one lane issues.  Units
         // are taken two at a time so that the accumulator buffer is static.
-        constexpr uint32_t idesc = idesc_f16(TILE_M, BN);
+        constexpr uint32_t idesc_min = idesc_f16(TILE_M, BN);
+        const uint32_t idesc = C::WIDE && a.terms == 2 ? idesc_f16(TILE_M, C::ACC_COLS) : idesc_min;
         constexpr uint32_t desc_hi = DESC_HI_SW128;
         const uint32_t a_lo = desc_lo_sw128(astage0), b_lo = desc_lo_sw128(bstage0);
         const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
-        int bs = 0;                                                   // the B stage of the next K block
-        uint32_t slot = 0, turn = 0;                                  // its hand-over's barriers, their phase
+        int bs = 0;                                                   // the next B stage
+        uint32_t bturn = 0, slot = 0, turn = 0;                       // its phase; the next A stage and its phase
         for (int u0 = 0; u0 < units; u0 += 2) {
-#pragma unroll
-            for (int ab = 0; ab < 2; ab++) {
+#pragma unroll 1
+            for (int ab = 0; ab < 2; ab++) {      // (unrolled, the 256-column form spilled more and took 475 us instead of 403)
                 const int u = u0 + ab;
                 if (u >= units) break;
-                const uint32_t s1 = tm + ab * BN;
+                const uint32_t s1 = tm + ab * C::ACC_COLS;
                 const uint32_t upar = (u0 >> 1) & 1;
                 mbar_wait_parked(accempty0 + 8 * ab, upar ^ 1, a.status, 0x80u);   // the drain of unit u-2 is done
+                const uint32_t slot0 = slot, turn0 = turn;
+                // All of the unit's remainders, then its values: the sum grows to its size in the second pass only,
+                // whose additions alone the accumulator rounds at that size.
+                for (int p = PASSES - 1; p >= 0; p--) {
+                    const bool first = p == PASSES - 1;
+                    slot = slot0, turn = turn0;
 #pragma unroll
-                for (int g = 0; g < KBLOCKS; g++) {
-                    if (C::A_STAGES == KBLOCKS) slot = g, turn = ab;
-                    mbar_wait_parked(full0 + 8 * slot, turn, a.status, 0x100u);
-                    tc_fence_after();
-                    const uint32_t ad = a_lo + (C::A_STAGES == KBLOCKS ? g : bs) * (A_BYTES >> 4);
-                    const uint32_t bd = b_lo + (C::B_STAGES == KBLOCKS ? g : bs) * (C::B_BYTES >> 4);
-                    if (elect_one()) {
+                    for (int g = 0; g < KBLOCKS; g++) {
+                        if (C::A_STAGES == KBLOCKS) slot = g, turn = ab;
+                        if (first) mbar_wait_parked(afull0 + 8 * slot, turn, a.status, 0x100u);
+                        if (!JOINT) mbar_wait_parked(bfull0 + 8 * bs, bturn, a.status, 0x8000u);
+                        tc_fence_after();
+                        const uint32_t ad = a_lo + slot * (A_BYTES >> 4), bd = b_lo + bs * (C::B_BYTES >> 4);
+                        if (elect_one()) {
 #pragma unroll
-                        for (int k = 0; k < BK / 16; k++) {   // 32 bytes further along the swizzled row per K=16
-                            if (g == 0 && k == 0) umma_f16_lo<0>(s1, ad, bd, desc_hi, idesc);
-                            else umma_f16_lo<1>(s1, ad + 2 * k, bd + 2 * k, desc_hi, idesc);
+                            for (int k = 0; k < BK / 16; k++) {   // 32 bytes further along the swizzled row per K=16
+                                if (g == 0 && k == 0) umma_f16_lo(s1, ad, bd, desc_hi, idesc, !first);
+                                else umma_f16_lo<1>(s1, ad + 2 * k, bd + 2 * k, desc_hi, idesc);
+                            }
+                            // the stages may be refilled once these finish
+                            if (!JOINT) umma_commit(bempty0 + 8 * bs);
+                            if (p == 0) umma_commit(aempty0 + 8 * slot);
                         }
+                        __syncwarp();
+                        if (++bs == C::B_STAGES) bs = 0, bturn ^= 1;
+                        if (C::A_STAGES != KBLOCKS && ++slot == C::A_STAGES) slot = 0, turn ^= 1;
                     }
-                    bs = bs + 1 == C::B_STAGES ? 0 : bs + 1;
-                    if (elect_one()) umma_commit(empty0 + 8 * slot);   // the stages may be refilled once these finish
-                    __syncwarp();
-                    if (C::A_STAGES != KBLOCKS && ++slot == C::A_STAGES) slot = 0, turn ^= 1;
                 }
                 const int ms = u % C::MIN_STAGES;
                 mbar_wait_parked(minfull0 + 8 * ms, (u / C::MIN_STAGES) & 1, a.status, 0x200u);
@@ -516,21 +559,22 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
                     // the minimums: terms (hi, hi | lo, lo) against the means' (hi, lo) twice
                     const uint32_t am = min0 + ms * C::MIN_BYTES;
                     const uint64_t bdm = smem_desc_plain(am + AMIN_BYTES, BN * 16);
-                    umma_f16(s1, smem_desc_plain(am, TILE_M * 16), bdm, idesc, 1);
-                    umma_f16(s1, smem_desc_plain(am + 2 * TILE_M * 16, TILE_M * 16), bdm, idesc, 1);
+                    umma_f16(s1, smem_desc_plain(am, TILE_M * 16), bdm, idesc_min, 1);
+                    umma_f16(s1, smem_desc_plain(am + 2 * TILE_M * 16, TILE_M * 16), bdm, idesc_min, 1);
                     umma_commit(accfull0 + 8 * ab);     // the unit's sum is complete
                 }
                 __syncwarp();
             }
         }
-    } else {
-        // ------------------------------ workers (warps 2-17) ------------------------------
+    } else if (warp < N_WORKERS) {
+        regs_inc<WORKER_REGS>();
+        // ------------------------------ workers ------------------------------
         // Warp w owns TMEM lane quadrant w % 4 (weight rows 32*(w % 4) + lane)
-        // and K block g = (w - 2) / 4 of every unit: it decodes that block of
+        // and K block g = w / 4 of every unit: it decodes that block of
         // its rows into the stage's A tile, then drains column quarter g of the
         // previous unit's sums while the tensor cores work on this one.
         const int quad = warp & 3;
-        const int g = (warp - 2) >> 2;
+        const int g = warp >> 2;
         const int rl = quad * 32 + lane;                // row within the tile = TMEM lane
         const bool drains = g < C::DRAINERS;
         const uint32_t drain_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + g * C::DRAIN_COLS;
@@ -550,10 +594,16 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
 #pragma unroll
             for (int c = 0; c < C::DRAIN_COLS / 16; c++) {
                 uint32_t v[16];
-                tmem_ld16(drain_addr + ab * BN + c * 16, v);
+                tmem_ld16(drain_addr + ab * C::ACC_COLS + c * 16, v);
                 tmem_ld_wait();
 #pragma unroll
                 for (int j = 0; j < 8; j++) ffma2(acc2[c * 8 + j], sc2, pack2(v[2 * j], v[2 * j + 1]));
+                if (C::WIDE && a.terms == 2) {      // the remainders' sums
+                    tmem_ld16(drain_addr + ab * C::ACC_COLS + BN + c * 16, v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 8; j++) ffma2(acc2[c * 8 + j], sc2, pack2(v[2 * j], v[2 * j + 1]));
+                }
             }
             tc_fence_before();
             __syncwarp();
@@ -568,11 +618,11 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             Q4kBlock blk;
             load_q4k_block(hdr, raw_row, g, blk);
             const int kb = KBLOCKS * u + g, stage = kb % C::A_STAGES;
-            mbar_wait_parked(empty0 + 8 * stage, ((kb / C::A_STAGES) & 1) ^ 1, a.status, 0x800u);   // the MMAs that read this stage are done
+            mbar_wait_parked(aempty0 + 8 * stage, ((kb / C::A_STAGES) & 1) ^ 1, a.status, 0x800u);   // the MMAs that read this stage are done
             store_q4k_block(blk, a_row_sw + stage * A_BYTES);
             fence_async_smem();          // the tensor core reads shared memory through the async proxy
             __syncwarp();
-            if (lane == 0) mbar_arrive(full0 + 8 * stage);
+            if (lane == 0) mbar_arrive(afull0 + 8 * stage);
             if (g >= 2) {
                 // the minimums' A operand [K group][row][16 B]: groups (hi, hi, lo, lo) of the
                 // two f16 terms of -(32*dmin/s)*m_j; K block 2's warp writes m_0..m_3, K block 3's m_4..m_7
@@ -600,27 +650,26 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             if (drains && u > 0) drain(u - 1);
         }
         if (drains) {
+            const uint32_t tk = tok0 + g * C::DRAIN_COLS * 4;
             griddep_wait();   // the kernel ahead may still read or write `out` and `aux`
             // this warp's columns' token scales through shared memory (the four quadrants' warps of a
             // column group write the same values): a load from global memory ahead of every store
             // would wait for the store before it
             for (int j = lane; j < C::DRAIN_COLS; j += 32) {
-                const size_t t = ((size_t)col0 + g * C::DRAIN_COLS + j) >> (a.split ? 1 : 0);
+                const size_t t = (size_t)col0 + g * C::DRAIN_COLS + j;
                 sts32f(tok0 + (g * C::DRAIN_COLS + j) * 4, t < a.n ? a.tok_scale[t] : 1.0f);
             }
             __syncwarp();
             // nothing to multiply by for activations of the usual range: every scale is one
-            const uint32_t tk = tok0 + g * C::DRAIN_COLS * 4;
             bool ones = true;
             for (int j = lane; j < C::DRAIN_COLS; j += 32) ones = ones && lds32f(tk + j * 4) == 1.0f;
             const bool scaled = !__all_sync(0xffffffffu, ones);
             if (OUT == 0 && a.epi != EPI_STORE && (size_t)row0 + quad * 32 < a.rows) {
                 // what the epilogue will read, on its way to L2 while the last unit multiplies
-                const int vals = C::DRAIN_COLS >> (a.split ? 1 : 0);
-                const size_t tb = ((size_t)col0 + g * C::DRAIN_COLS) >> (a.split ? 1 : 0);
+                const size_t tb = (size_t)col0 + g * C::DRAIN_COLS;
                 const float *src = a.epi == EPI_ADD ? a.out.dst[0] + a.out.row0 : a.aux;
                 const size_t step = a.epi == EPI_ADD ? a.out.pitch : a.rows;
-                for (int j = lane; j < vals; j += 32)
+                for (int j = lane; j < C::DRAIN_COLS; j += 32)
                     if (tb + j < a.n) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + (tb + j) * step + row0 + quad * 32));
             }
             drain(units - 1);
@@ -641,7 +690,7 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
 #pragma unroll
                         for (int j = 0; j < 8; j++) v[j] *= lds32f(tk + (8 * q + j) * 4);
                     }
-                    if (row < a.rows) emit_columns<false>(to, a.rows, a.n, a.split, (size_t)col0 + g * C::DRAIN_COLS + 8 * q, v);
+                    if (row < a.rows) gemm_emit<false>(to, a.rows, a.n, (size_t)col0 + g * C::DRAIN_COLS + 8 * q, v);
                 }
             } else if (OUT == 2) {
                 // The group's tile [token][row] into the rings' shared memory, which nothing reads any
@@ -652,18 +701,11 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
 #pragma unroll
                     for (int j = 0; j < C::DRAIN_COLS; j++) acc[j] *= lds32f(tk + j * 4);
                 }
-                int nvals = C::DRAIN_COLS;
-                if (a.split) {
 #pragma unroll
-                    for (int j = 0; j < C::DRAIN_COLS / 2; j++) acc[j] = acc[2 * j] + acc[2 * j + 1];
-                    nvals = C::DRAIN_COLS / 2;
-                }
-#pragma unroll
-                for (int j = 0; j < C::DRAIN_COLS; j++)
-                    if (j < nvals) sts32f(stage + (j * TILE_M + rl) * 4, acc[j]);
+                for (int j = 0; j < C::DRAIN_COLS; j++) sts32f(stage + (j * TILE_M + rl) * 4, acc[j]);
                 fence_async_smem();
                 asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");   // the group's four warps: all 128 rows are in
-                const size_t t0 = ((size_t)col0 + g * C::DRAIN_COLS) >> (a.split ? 1 : 0);
+                const size_t t0 = (size_t)col0 + g * C::DRAIN_COLS;
                 if (quad == 0 && lane == 0 && t0 < a.n) {
 #pragma unroll
                     for (int p = 0; p < DWIM_MAX_WORLD; p++)
@@ -678,22 +720,12 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
 #pragma unroll
                     for (int j = 0; j < C::DRAIN_COLS; j++) acc[j] *= lds32f(tk + j * 4);
                 }
-                if (a.split) {
 #pragma unroll
-                    for (int j = 0; j < C::DRAIN_COLS; j += 16) {
-                        float v[8];
+                for (int j = 0; j < C::DRAIN_COLS; j += 8) {
+                    float v[8];
 #pragma unroll
-                        for (int i = 0; i < 8; i++) v[i] = acc[j + 2 * i] + acc[j + 2 * i + 1];
-                        gemm_emit<SHARED>(to, rows, n, (cbase + j) >> 1, v);
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < C::DRAIN_COLS; j += 8) {
-                        float v[8];
-#pragma unroll
-                        for (int i = 0; i < 8; i++) v[i] = acc[j + i];
-                        gemm_emit<SHARED>(to, rows, n, cbase + j, v);
-                    }
+                    for (int i = 0; i < 8; i++) v[i] = acc[j + i];
+                    gemm_emit<SHARED>(to, rows, n, cbase + j, v);
                 }
             }
         }
@@ -702,7 +734,8 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             cluster_sync();
         }
     }
-    if (warp < 2 || warp == RAW_WARP) {
+    if (warp > RAW_WARP) regs_dec<OTHER_REGS>();      // (the warpgroup takes part as a whole)
+    if (warp >= N_WORKERS) {
         __syncwarp();
         if (split_k > 1) {      // the workers' two meetings are the whole cluster's
             cluster_sync();
@@ -711,7 +744,7 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem_base, C::TMEM_COLS);
+    if (warp == MMA_WARP) tmem_dealloc(tmem_base, C::TMEM_COLS);
 }
 
 // ---- the dense kernel: Q8_0 and Q6_K above the small-M kernel's range --------------------------
@@ -725,25 +758,34 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
 // a lo tile, K block kb in stage kb % 2; a ring of its own for the activations; no minimums.
 // (The terms used to be written to memory by a pass of their own and loaded by every column of tiles: 64 KB
 // from L2 per K block of 1024 cycles, 9.1 TB/s, was what bound it.  Products with their operand, in short bursts:
-// [12288, 5120] Q6_K by 512 f32 tokens 299 us then, 209 now (198 the kernel alone; 253 in a long run, under the
-// power limit); [5120, 5120] Q8_0 by 131 of them 97 and 69.  The error fell with the drains: 1e-6 to 1e-5 of
-// the result in 2-norm over K = 2304 to 12288 then; now, at any K from 512 to 17408, 4.6e-7 (Q6_K) and 6.7e-7
-// (Q8_0) by f32 activations, 2.8e-7 and 6.4e-7 by bf16 ones, the largest difference 2.5e-6 and 4.2e-6 of the
-// result's root mean square.)
-// Bound by the tensor pipe (68 % active by 512 columns), beside which 96 registers a thread are short: the
-// 256-column form spills 60 (Q6_K) and 28 bytes (Q8_0).
+// [12288, 5120] Q6_K by 512 f32 tokens 299 us then, 209 as two columns a token, 207 now (236 with their operand);
+// [5120, 5120] Q8_0 by 512 of them 127 as columns, 128 with spills in the main loop, 106 now.  Errors, 2-norm over the
+// result's: 1e-6 to 1e-5 over K = 2304 to 12288 then; now, at any K from 512 to 17408, by f32 activations 4.2e-7 (Q6_K)
+// and 5.9e-7 (Q8_0) up to 128 tokens and 3.2e-7 and 3.9e-7 above, by bf16 ones 2.7e-7 and 5.6e-7, the largest difference
+// 2.0e-6 and 3.0e-6 of the result's root mean square.)
+// Bound by the tensor pipe (68 % active by 256 tokens).  The scales are fetched where they are used: fetched a unit
+// ahead they cost the 256-column forms 130 to 400 bytes of spills.
 struct DenseArgs {
     size_t rows, n, units;
-    int split, epi, split_k;
+    int terms, epi, split_k;
     OutSpec out;
     const __half *scales;           // Q8_0: eight per unit and row; Q6_K: one
     size_t srow;
     const float *tok_scale, *aux;
     uint32_t *status;
 };
-template <int FMT, int BN> struct DenseCfg {
+// Two terms that take turns double the additions to an accumulator, so it is drained twice a unit.
+template <int FMT, int BN, int MODE> struct DenseCfg {
+    static constexpr bool WIDE = MODE == SIDE_BY_SIDE;
+    static constexpr int DRAIN_KB = MODE == TWO_PASSES ? 2 : KBLOCKS;      // K blocks between drains
+    static constexpr int TERM_BYTES = BN * BK * 2, ACC_COLS = BN * (WIDE ? 2 : 1);
     static constexpr int A_STAGES = 2, A_STAGE = 2 * A_BYTES;
-    static constexpr int B_STAGES = BN > 128 ? 3 : 4, B_BYTES = BN * BK * 2;
+    static constexpr int STEPS = KBLOCKS / DRAIN_KB;                // drains of a unit
+    // Accumulator buffers: two units' where tensor memory holds them, else two steps'.
+    static constexpr int ACC_BUFS = 2 * STEPS * ACC_COLS <= 512 ? 2 * STEPS : 2;
+    static_assert(ACC_BUFS == 2 * STEPS || STEPS == 2, "a unit of more steps than buffers would wait for itself");
+    static constexpr int TMEM_COLS = ACC_BUFS * ACC_COLS > 256 ? 512 : 256;
+    static constexpr int B_STAGES = ACC_COLS > 128 ? 3 : 4, B_BYTES = TERM_BYTES * (WIDE ? 2 : 1);
     // raw weights: a unit of Q6_K, half a unit of Q8_0 (128 bytes a row, swizzled)
     static constexpr int RAW_STEPS = FMT == Q8_0 ? 2 : 1;           // ring stages per unit
     static constexpr int RAW_STAGES = FMT == Q8_0 ? 3 : 2, RAW_STAGE = FMT == Q8_0 ? TILE_M * 128 : TILE_M * Q6_K_DEV;
@@ -773,15 +815,16 @@ __device__ __forceinline__ void store_terms(uint32_t w0, uint32_t w1, uint32_t o
     sts128((a_row_sw + A_BYTES) ^ (c << 4), l[0], l[1], l[2], l[3]);
 }
 
-template <int FMT, int BN, bool SHARED>
+template <int FMT, int BN, int MODE, bool SHARED>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ DenseArgs a) {
-    using C = DenseCfg<FMT, BN>;
+    using C = DenseCfg<FMT, BN, MODE>;
+    constexpr int DRAIN_KB = C::DRAIN_KB, PASSES = MODE == TWO_PASSES ? 2 : 1;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     // afull, adone: one per K block of the unit, completed once a unit
-    const uint32_t afull0 = base, adone0 = base + 32, bfull0 = base + 64, bempty0 = base + 96, accfull0 = base + 128, accempty0 = base + 144;
-    const uint32_t rawfull0 = base + 160, rawempty0 = base + 192, tmem_slot = base + 224;
+    const uint32_t afull0 = base, adone0 = base + 32, bfull0 = base + 64, bempty0 = base + 96, accfull0 = base + 128, accempty0 = base + 192;
+    const uint32_t rawfull0 = base + 256, rawempty0 = base + 288, tmem_slot = base + 320;
     const uint32_t astage0 = base + BAR_BYTES, bstage0 = astage0 + C::A_STAGES * C::A_STAGE, raw0 = bstage0 + C::B_STAGES * C::B_BYTES;
     const uint32_t scale0 = raw0 + C::RAW_STAGES * C::RAW_STAGE, tok0 = scale0 + SCALE_SLOTS * TILE_M * 4;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -793,7 +836,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             mbar_init(afull0 + 8 * g, 4);                // the K block's four worker warps
             mbar_init(adone0 + 8 * g, 1);
         }
-        for (int s = 0; s < 2; s++) {
+        for (int s = 0; s < C::ACC_BUFS; s++) {
             mbar_init(accfull0 + 8 * s, 1);
             mbar_init(accempty0 + 8 * s, N_WORKERS);
         }
@@ -807,8 +850,8 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) {
-        tmem_alloc(tmem_slot, 2 * BN);
+    if (warp == MMA_WARP) {
+        tmem_alloc(tmem_slot, C::TMEM_COLS);
         tmem_relinquish();
     }
     tc_fence_before();
@@ -817,17 +860,23 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     const uint32_t tmem_base = lds32(tmem_slot);
     griddep_launch();
 
-    if (warp == 0) {
+    if (warp == X_WARP) {
+        regs_dec<DENSE_OTHER_REGS>();
         griddep_wait();   // the operand comes from the prologue kernel just ahead
         if (elect_one()) {
-            for (int kb = 0; kb < KBLOCKS * units; kb++) {
-                const int s = kb % C::B_STAGES;
-                mbar_wait_parked(bempty0 + 8 * s, ((kb / C::B_STAGES) & 1) ^ 1, a.status, 0x100000u);
-                mbar_expect_tx(bfull0 + 8 * s, C::B_BYTES);
-                tma_load_2d(bstage0 + s * C::B_BYTES, &tmap_x, (KBLOCKS * ub + kb) * BK, col0, bfull0 + 8 * s);
-            }
+            int s = 0, turn = 1;
+            for (int kb = 0; kb < KBLOCKS * units; kb++)
+                for (int p = PASSES - 1; p >= 0; p--) {      // the remainders first
+                    mbar_wait_parked(bempty0 + 8 * s, turn, a.status, 0x100000u);
+                    mbar_expect_tx(bfull0 + 8 * s, C::TERM_BYTES * (C::WIDE ? a.terms : 1));
+                    const uint32_t to = bstage0 + s * C::B_BYTES;
+                    tma_load_2d(to, &tmap_x, (KBLOCKS * ub + kb) * BK, p * (int)a.n + col0, bfull0 + 8 * s);
+                    if (C::WIDE && a.terms == 2) tma_load_2d(to + C::TERM_BYTES, &tmap_x, (KBLOCKS * ub + kb) * BK, (int)a.n + col0, bfull0 + 8 * s);
+                    if (++s == C::B_STAGES) s = 0, turn ^= 1;
+                }
         }
     } else if (warp == RAW_WARP) {
+        regs_dec<DENSE_OTHER_REGS>();
         if (elect_one()) {
             for (int r = 0; r < C::RAW_STEPS * units; r++) {
                 const int s = r % C::RAW_STAGES;
@@ -836,45 +885,55 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 tma_load_2d(raw0 + s * C::RAW_STAGE, &tmap_w, FMT == Q8_0 ? (2 * ub + r) * 128 : (ub + r) * Q6_K_DEV, row0, rawfull0 + 8 * s);
             }
         }
-    } else if (warp == 1) {
-        constexpr uint32_t idesc = idesc_f16(TILE_M, BN);
+    } else if (warp == MMA_WARP) {
+        regs_dec<DENSE_OTHER_REGS>();
+        const uint32_t idesc = idesc_f16(TILE_M, C::WIDE && a.terms == 2 ? C::ACC_COLS : BN);
         const uint32_t a_lo = desc_lo_sw128(astage0), b_lo = desc_lo_sw128(bstage0);
         const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
-        int bs = 0, bturn = 0;
+        int bs = 0, bturn = 0, buf = 0, bufturn = 1;
         for (int u = 0; u < units; u++) {
-            const uint32_t acc = tm + (u & 1) * BN;
-            mbar_wait_parked(accempty0 + 8 * (u & 1), ((u >> 1) & 1) ^ 1, a.status, 0x400000u);
 #pragma unroll
             for (int g = 0; g < KBLOCKS; g++) {
-                mbar_wait_parked(bfull0 + 8 * bs, bturn, a.status, 0x800000u);
+                const uint32_t acc = tm + buf * C::ACC_COLS;
+                if (g % DRAIN_KB == 0) mbar_wait_parked(accempty0 + 8 * buf, bufturn, a.status, 0x400000u);
                 mbar_wait_parked(afull0 + 8 * g, u & 1, a.status, 0x1000000u);
-                tc_fence_after();
-                if (elect_one()) {
-                    const uint32_t hi = a_lo + (g & 1) * (C::A_STAGE >> 4), lo = hi + (A_BYTES >> 4), bd = b_lo + bs * (C::B_BYTES >> 4);
+                for (int p = PASSES - 1; p >= 0; p--) {
+                    mbar_wait_parked(bfull0 + 8 * bs, bturn, a.status, 0x800000u);
+                    tc_fence_after();
+                    if (elect_one()) {
+                        // the weights' remainders first: they are too small for the accumulator's rounding to matter
+                        const uint32_t hi = a_lo + (g & 1) * (C::A_STAGE >> 4), lo = hi + (A_BYTES >> 4), bd = b_lo + bs * (C::B_BYTES >> 4);
 #pragma unroll
-                    for (int k = 0; k < BK / 16; k++) {
-                        if (g == 0 && k == 0) umma_f16_lo<0>(acc, hi, bd, DESC_HI_SW128, idesc);
-                        else umma_f16_lo<1>(acc, hi + 2 * k, bd + 2 * k, DESC_HI_SW128, idesc);
-                        umma_f16_lo<1>(acc, lo + 2 * k, bd + 2 * k, DESC_HI_SW128, idesc);
+                        for (int k = 0; k < BK / 16; k++) {
+                            if (g % DRAIN_KB == 0 && k == 0) umma_f16_lo(acc, lo, bd, DESC_HI_SW128, idesc, p != PASSES - 1);
+                            else umma_f16_lo<1>(acc, lo + 2 * k, bd + 2 * k, DESC_HI_SW128, idesc);
+                        }
+#pragma unroll
+                        for (int k = 0; k < BK / 16; k++) umma_f16_lo<1>(acc, hi + 2 * k, bd + 2 * k, DESC_HI_SW128, idesc);
+                        umma_commit(bempty0 + 8 * bs);
+                        if (p == 0) {
+                            umma_commit(adone0 + 8 * g);
+                            if (g % DRAIN_KB == DRAIN_KB - 1) umma_commit(accfull0 + 8 * buf);
+                        }
                     }
-                    umma_commit(adone0 + 8 * g);
-                    umma_commit(bempty0 + 8 * bs);
-                    if (g == KBLOCKS - 1) umma_commit(accfull0 + 8 * (u & 1));
+                    __syncwarp();
+                    if (++bs == C::B_STAGES) bs = 0, bturn ^= 1;
                 }
-                __syncwarp();
-                if (++bs == C::B_STAGES) bs = 0, bturn ^= 1;
+                if (g % DRAIN_KB == DRAIN_KB - 1 && ++buf == C::ACC_BUFS) buf = 0, bufturn ^= 1;
             }
         }
-    } else {
-        const int quad = warp & 3, g = (warp - 2) >> 2, rl = quad * 32 + lane;
+    } else if (warp < N_WORKERS) {
+        regs_inc<DENSE_WORKER_REGS>();
+        const int quad = warp & 3, g = warp >> 2, rl = quad * 32 + lane;
         const uint32_t drain_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + g * C::DRAIN_COLS;
         const uint32_t a_row_sw = (astage0 + (g & 1) * C::A_STAGE + rl * 128) | ((rl & 7) << 4);
         const size_t row = (size_t)row0 + rl;
         uint64_t acc2[C::DRAIN_COLS / 2];
 #pragma unroll
         for (int j = 0; j < C::DRAIN_COLS / 2; j++) acc2[j] = 0ull;
-        auto drain = [&](int u) {
-            mbar_wait_parked(accfull0 + 8 * (u & 1), (u >> 1) & 1, a.status, 0x2000000u);
+        int buf = 0, bufturn = 0;
+        auto drain = [&](int u) {      // the next step, one of unit u's
+            mbar_wait_parked(accfull0 + 8 * buf, bufturn, a.status, 0x2000000u);
             tc_fence_after();
             // written before the unit's first K block was handed over
             const uint32_t sc = __float_as_uint(lds32f(scale0 + ((u % SCALE_SLOTS) * TILE_M + rl) * 4));
@@ -882,16 +941,26 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 #pragma unroll
             for (int c = 0; c < C::DRAIN_COLS / 16; c++) {
                 uint32_t v[16];
-                tmem_ld16(drain_addr + (u & 1) * BN + c * 16, v);
+                tmem_ld16(drain_addr + buf * C::ACC_COLS + c * 16, v);
                 tmem_ld_wait();
 #pragma unroll
                 for (int j = 0; j < 8; j++) ffma2(acc2[c * 8 + j], sc2, pack2(v[2 * j], v[2 * j + 1]));
+                if (C::WIDE && a.terms == 2) {
+                    tmem_ld16(drain_addr + buf * C::ACC_COLS + BN + c * 16, v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 8; j++) ffma2(acc2[c * 8 + j], sc2, pack2(v[2 * j], v[2 * j + 1]));
+                }
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(accempty0 + 8 * (u & 1));
+            if (lane == 0) mbar_arrive(accempty0 + 8 * buf);
+            if (++buf == C::ACC_BUFS) buf = 0, bufturn ^= 1;
         };
-        // the row's scales, a unit ahead (rows past the end: the last row's, their weights are zeros)
+        // With two buffers for a unit's two steps the first of the unit before is drained ahead of the decode: its
+        // buffer is the one that this unit's first step takes, which K blocks 2 and 3 wait for (their stages').
+        constexpr int EARLY = C::ACC_BUFS == 2 * C::STEPS ? 0 : 1;
+        // the row's scales (rows past the end: the last row's, their weights are zeros)
         const __half *srow = a.scales + (row < a.rows ? row : a.rows - 1) * a.srow;
         auto fetch = [&](int u) {
             uint4 v = make_uint4(0, 0, 0, 0);
@@ -901,75 +970,80 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             }
             return v;
         };
-        uint4 next = fetch(0);
-        for (int u = 0; u < units; u++) {
-            const uint4 sc = next;
-            next = fetch(u + 1);
-            const int r = C::RAW_STEPS == 2 ? 2 * u + (g >> 1) : u, rs = r % C::RAW_STAGES;
-            mbar_wait_parked(rawfull0 + 8 * rs, (r / C::RAW_STAGES) & 1, a.status, 0x4000000u);
-            // the stage's last user, two K blocks back, is done (this warp has waited for the use before that one)
-            mbar_wait_parked(adone0 + 8 * (g ^ 2), (u & 1) ^ (g < 2 ? 1 : 0), a.status, 0x8000000u);
-            const uint32_t raw = raw0 + rs * C::RAW_STAGE;
-            float unit_scale;
-            if constexpr (FMT == Q6_K) {
-                const uint32_t rrow = raw + rl * Q6_K_DEV, ql = rrow + (g >> 1) * 64, qh = rrow + 128 + (g >> 1) * 32;
-                const int nib = (g & 1) * 4;
-                const uint32_t s4 = lds32(rrow + 192 + 4 * g) ^ 0x80808080u;      // the four groups' sub-scales + 128
-                unit_scale = h2f_lo(sc.x);
+        // (One turn more than there are units, so that the drain is in the code once or twice.)
+        const uint32_t tk = tok0 + g * C::DRAIN_COLS * 4;
+        for (int u = 0; u <= units; u++) {
+            if (EARLY && u > 0) drain(u - 1);
+            if (u < units) {
+                const uint4 sc = fetch(u);
+                const int r = C::RAW_STEPS == 2 ? 2 * u + (g >> 1) : u, rs = r % C::RAW_STAGES;
+                mbar_wait_parked(rawfull0 + 8 * rs, (r / C::RAW_STAGES) & 1, a.status, 0x4000000u);
+                // the stage's last user, two K blocks back, is done (this warp has waited for the use before that one)
+                mbar_wait_parked(adone0 + 8 * (g ^ 2), (u & 1) ^ (g < 2 ? 1 : 0), a.status, 0x8000000u);
+                const uint32_t raw = raw0 + rs * C::RAW_STAGE;
+                float unit_scale;
+                if constexpr (FMT == Q6_K) {
+                    const uint32_t rrow = raw + rl * Q6_K_DEV, ql = rrow + (g >> 1) * 64, qh = rrow + 128 + (g >> 1) * 32;
+                    const int nib = (g & 1) * 4;
+                    const uint32_t s4 = lds32(rrow + 192 + 4 * g) ^ 0x80808080u;      // the four groups' sub-scales + 128
+                    unit_scale = h2f_lo(sc.x);
 #pragma unroll
-                for (int c = 0; c < 2; c++) {
-                    const uint4 h = lds128(qh + 16 * c), l0 = lds128(ql + 16 * c), l1 = lds128(ql + 32 + 16 * c);
-                    const uint32_t hw[4] = {h.x, h.y, h.z, h.w}, w0[4] = {l0.x, l0.y, l0.z, l0.w}, w1[4] = {l1.x, l1.y, l1.z, l1.w};
-                    // 0x6480 = 1152 = 1024 + 128
-                    const uint32_t f0 = hsub2(prmt(s4, 0x64006400u, 0x5050u + c * 0x0101u), 0x64806480u);
-                    const uint32_t f1 = hsub2(prmt(s4, 0x64006400u, 0x5252u + c * 0x0101u), 0x64806480u);
-                    uint32_t v0[4], v1[4];
+                    for (int c = 0; c < 2; c++) {
+                        const uint4 h = lds128(qh + 16 * c), l0 = lds128(ql + 16 * c), l1 = lds128(ql + 32 + 16 * c);
+                        const uint32_t hw[4] = {h.x, h.y, h.z, h.w}, w0[4] = {l0.x, l0.y, l0.z, l0.w}, w1[4] = {l1.x, l1.y, l1.z, l1.w};
+                        // 0x6480 = 1152 = 1024 + 128
+                        const uint32_t f0 = hsub2(prmt(s4, 0x64006400u, 0x5050u + c * 0x0101u), 0x64806480u);
+                        const uint32_t f1 = hsub2(prmt(s4, 0x64006400u, 0x5252u + c * 0x0101u), 0x64806480u);
+                        uint32_t v0[4], v1[4];
 #pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const uint32_t hh = hw[i] >> nib;      // bits 0-1 of a byte: the first 32 weights, bits 2-3: the second
-                        v0[i] = ((w0[i] >> nib) & 0x0f0f0f0fu) | ((hh << 4) & 0x30303030u);
-                        v1[i] = ((w1[i] >> nib) & 0x0f0f0f0fu) | ((hh << 2) & 0x30303030u);
+                        for (int i = 0; i < 4; i++) {
+                            const uint32_t hh = hw[i] >> nib;      // bits 0-1 of a byte: the first 32 weights, bits 2-3: the second
+                            v0[i] = ((w0[i] >> nib) & 0x0f0f0f0fu) | ((hh << 4) & 0x30303030u);
+                            v1[i] = ((w1[i] >> nib) & 0x0f0f0f0fu) | ((hh << 2) & 0x30303030u);
+                        }
+#pragma unroll
+                        for (int i = 0; i < 2; i++) {      // 0x6420 = 1056 = 1024 + 32
+                            store_terms(v0[2 * i], v0[2 * i + 1], 0x64206420u, f0, a_row_sw, 2 * c + i);
+                            store_terms(v1[2 * i], v1[2 * i + 1], 0x64206420u, f1, a_row_sw, 4 + 2 * c + i);
+                        }
                     }
+                } else {
+                    // the unit's power of two: its largest |d| to [64, 128)
+                    const uint32_t m2 = __vmaxu2(__vmaxu2(sc.x & 0x7fff7fffu, sc.y & 0x7fff7fffu), __vmaxu2(sc.z & 0x7fff7fffu, sc.w & 0x7fff7fffu));
+                    const int e = (int)(max(m2 & 0xffffu, m2 >> 16) >> 10);
+                    const int up = 6 - (max(e, 1) - 15);
+                    const float by = __uint_as_float((uint32_t)(127 + up) << 23);
+                    unit_scale = __uint_as_float((uint32_t)(127 - up) << 23);
+                    const uint32_t d2 = g == 0 ? sc.x : g == 1 ? sc.y : g == 2 ? sc.z : sc.w;
+                    const float d0 = h2f_lo(d2) * by, d1 = h2f_hi(d2) * by;
+                    const uint32_t f[2] = {f16x2_rn(d0, d0), f16x2_rn(d1, d1)};
 #pragma unroll
-                    for (int i = 0; i < 2; i++) {      // 0x6420 = 1056 = 1024 + 32
-                        store_terms(v0[2 * i], v0[2 * i + 1], 0x64206420u, f0, a_row_sw, 2 * c + i);
-                        store_terms(v1[2 * i], v1[2 * i + 1], 0x64206420u, f1, a_row_sw, 4 + 2 * c + i);
+                    for (int c = 0; c < 4; c++) {
+                        const uint4 q = lds128(raw + rl * 128 + ((((g & 1) * 4 + c) ^ (rl & 7)) << 4));
+                        store_terms(q.x ^ 0x80808080u, q.y ^ 0x80808080u, 0x64806480u, f[c >> 1], a_row_sw, 2 * c);
+                        store_terms(q.z ^ 0x80808080u, q.w ^ 0x80808080u, 0x64806480u, f[c >> 1], a_row_sw, 2 * c + 1);
                     }
+                }
+                if (g == 0) sts32f(scale0 + ((u % SCALE_SLOTS) * TILE_M + rl) * 4, unit_scale);
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(afull0 + 8 * g);
+                    mbar_arrive(rawempty0 + 8 * rs);
                 }
             } else {
-                // the unit's power of two: its largest |d| to [64, 128)
-                const uint32_t m2 = __vmaxu2(__vmaxu2(sc.x & 0x7fff7fffu, sc.y & 0x7fff7fffu), __vmaxu2(sc.z & 0x7fff7fffu, sc.w & 0x7fff7fffu));
-                const int e = (int)(max(m2 & 0xffffu, m2 >> 16) >> 10);
-                const int up = 6 - (max(e, 1) - 15);
-                const float by = __uint_as_float((uint32_t)(127 + up) << 23);
-                unit_scale = __uint_as_float((uint32_t)(127 - up) << 23);
-                const uint32_t d2 = g == 0 ? sc.x : g == 1 ? sc.y : g == 2 ? sc.z : sc.w;
-                const float d0 = h2f_lo(d2) * by, d1 = h2f_hi(d2) * by;
-                const uint32_t f[2] = {f16x2_rn(d0, d0), f16x2_rn(d1, d1)};
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const uint4 q = lds128(raw + rl * 128 + ((((g & 1) * 4 + c) ^ (rl & 7)) << 4));
-                    store_terms(q.x ^ 0x80808080u, q.y ^ 0x80808080u, 0x64806480u, f[c >> 1], a_row_sw, 2 * c);
-                    store_terms(q.z ^ 0x80808080u, q.w ^ 0x80808080u, 0x64806480u, f[c >> 1], a_row_sw, 2 * c + 1);
+                griddep_wait();   // the kernel ahead may still read or write `out` and `aux`
+                for (int j = lane; j < C::DRAIN_COLS; j += 32) {
+                    const size_t t = (size_t)col0 + g * C::DRAIN_COLS + j;
+                    sts32f(tok0 + (g * C::DRAIN_COLS + j) * 4, t < a.n ? a.tok_scale[t] : 1.0f);
                 }
+                __syncwarp();
             }
-            if (g == 0) sts32f(scale0 + ((u % SCALE_SLOTS) * TILE_M + rl) * 4, unit_scale);
-            fence_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(afull0 + 8 * g);
-                mbar_arrive(rawempty0 + 8 * rs);
+            if (u > 0) {
+#pragma unroll 1
+                for (int i = EARLY; i < C::STEPS; i++) drain(u - 1);
             }
-            if (u > 0) drain(u - 1);
         }
-        griddep_wait();   // the kernel ahead may still read or write `out` and `aux`
-        for (int j = lane; j < C::DRAIN_COLS; j += 32) {
-            const size_t t = ((size_t)col0 + g * C::DRAIN_COLS + j) >> (a.split ? 1 : 0);
-            sts32f(tok0 + (g * C::DRAIN_COLS + j) * 4, t < a.n ? a.tok_scale[t] : 1.0f);
-        }
-        __syncwarp();
-        const uint32_t tk = tok0 + g * C::DRAIN_COLS * 4;
-        drain(units - 1);
         float acc[C::DRAIN_COLS];
 #pragma unroll
         for (int j = 0; j < C::DRAIN_COLS / 2; j++) unpack2(acc2[j], acc[2 * j], acc[2 * j + 1]);
@@ -989,10 +1063,11 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             if (row >= a.rows) continue;
 #pragma unroll
             for (int j = 0; j < 8; j++) v[j] *= lds32f(tk + (8 * q + j) * 4);
-            emit_columns<SHARED>(to, a.rows, a.n, a.split, (size_t)col0 + g * C::DRAIN_COLS + 8 * q, v);
+            gemm_emit<SHARED>(to, a.rows, a.n, (size_t)col0 + g * C::DRAIN_COLS + 8 * q, v);
         }
     }
-    if (warp < 2 || warp == RAW_WARP) {
+    if (warp > RAW_WARP) regs_dec<DENSE_OTHER_REGS>();      // (the warpgroup takes part as a whole)
+    if (warp >= N_WORKERS) {
         __syncwarp();
         if (split_k > 1) {      // the workers' two meetings are the whole cluster's
             cluster_sync();
@@ -1001,7 +1076,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem_base, 2 * BN);
+    if (warp == MMA_WARP) tmem_dealloc(tmem_base, C::TMEM_COLS);
 }
 
 // ---- host side ---------------------------------------------------------------------
@@ -1052,7 +1127,7 @@ struct SplitCost {
 // known: clusters of so many blocks that a device holds at once (0: not asked yet); contexts of several threads share it.
 template <typename Kernel, typename Fits>
 int pick_split(dwim_b200_ctx *ctx, Kernel kern, int threads, size_t smem, Fits fits, SplitCost cost,
-               std::atomic<int> (&known)[64][MAX_SPLIT + 1], long tiles, int units, double *time = nullptr) {
+               std::atomic<int> (&known)[64][MAX_SPLIT + 1], long tiles, int units, double unit, double *time = nullptr) {
     int best = 1;
     double t_best = 0;
     for (int s = 1; s <= MAX_SPLIT && s <= units; s++) {
@@ -1079,7 +1154,7 @@ int pick_split(dwim_b200_ctx *ctx, Kernel kern, int threads, size_t smem, Fits f
             }
             known[ctx->device & 63][s] = k = n;
         }
-        const double t = (double)((tiles + k - 1) / k) * ((units + s - 1) / s + (s > 1 ? cost.shared : cost.tile));
+        const double t = (double)((tiles + k - 1) / k) * ((units + s - 1) / s * unit + (s > 1 ? cost.shared : cost.tile));
         if (s == 1 || t < 0.97 * t_best) {
             t_best = t;
             best = s;
@@ -1089,42 +1164,46 @@ int pick_split(dwim_b200_ctx *ctx, Kernel kern, int threads, size_t smem, Fits f
     return best;
 }
 
+// What a unit costs by two terms an activation, in units by one: the tensor work doubles, the decode does not.
+double q4k_unit(int bn, int terms) { return terms == 1 ? 1.0 : bn >= 128 ? 1.8 : 1.1; }
+
 // How many blocks share a tile of the Q4_K kernel at this width, and how long the product then takes
-// (in units on the busiest block).
-template <int BN>
-int gemm_split(dwim_b200_ctx *ctx, const WeightView &w, size_t ncols, double *time = nullptr) {
+// (in units of one term on the busiest block).
+template <int BN, int MODE>
+int gemm_split(dwim_b200_ctx *ctx, const WeightView &w, size_t n, int terms, double *time = nullptr) {
     static std::atomic<int> known[64][MAX_SPLIT + 1] = {};
-    const long tiles = (long)((w.rows + TILE_M - 1) / TILE_M) * (long)((ncols + BN - 1) / BN);
-    return pick_split(ctx, gemm_q4k_kernel<BN, 0>, GEMM_THREADS, (size_t)Cfg<BN>::SMEM, Cfg<BN>::split_fits, SplitCost{3.0, 6.5}, known, tiles,
-                      (int)(w.cols / 256), time);
+    const long tiles = (long)((w.rows + TILE_M - 1) / TILE_M) * (long)((n + BN - 1) / BN);
+    return pick_split(ctx, gemm_q4k_kernel<BN, 0, MODE>, GEMM_THREADS, (size_t)Cfg<BN, MODE>::SMEM, Cfg<BN, MODE>::split_fits, SplitCost{3.0, 6.5}, known, tiles,
+                      (int)(w.cols / 256), q4k_unit(BN, terms), time);
 }
-template <int BN> double gemm_time(dwim_b200_ctx *ctx, const WeightView &w, size_t ncols) {
+template <int BN, int MODE> double gemm_time(dwim_b200_ctx *ctx, const WeightView &w, size_t n, int terms) {
     double t = 0;
-    gemm_split<BN>(ctx, w, ncols, &t);
+    gemm_split<BN, MODE>(ctx, w, n, terms, &t);
     return t;
 }
 
-template <int BN>
-int launch_gemm(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, size_t n, int split, const OutSpec &out,
+template <int BN, int MODE>
+int launch_gemm(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, size_t n, int terms, const OutSpec &out,
                 const float *aux, int epi) {
-    using C = Cfg<BN>;
-    const size_t ncols = n * (split ? 2 : 1), units = w.cols / 256;
+    using C = Cfg<BN, MODE>;
+    const size_t units = w.cols / 256;
     CUtensorMap tw, tx, tm;
     int rc;
     // packed weights as bytes: [rows][qpitch], box [128 rows][144 bytes]; rows past the end read as zero blocks
     if ((rc = encode_2d(ctx, &tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, w.quants, w.qpitch, w.rows, w.qpitch, 144, TILE_M,
                         CU_TENSOR_MAP_SWIZZLE_NONE, "weight")))
         return rc;
-    // activations: [ncols][K] f16, box [BN][64], 128-byte swizzle; columns past the end read as zero
-    if ((rc = encode_2d(ctx, &tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, operand, w.cols, ncols, w.cols * 2, BK, BN,
+    // activations: [terms][n][K] f16, box [BN][64], 128-byte swizzle; columns past the last token read as another
+    // term's tokens or as zeros
+    if ((rc = encode_2d(ctx, &tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, operand, w.cols, terms * n, w.cols * 2, BK, BN,
                         CU_TENSOR_MAP_SWIZZLE_128B, "activation")))
         return rc;
-    // sub-block means: [ncols][units*16] f16, box [BN][8]
-    if ((rc = encode_2d(ctx, &tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, operand + ncols * w.cols, units * 16, ncols, units * 32, 8,
+    // sub-block means: [n][units*16] f16, box [BN][8]
+    if ((rc = encode_2d(ctx, &tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, operand + terms * n * w.cols, units * 16, n, units * 32, 8,
                         BN, CU_TENSOR_MAP_SWIZZLE_NONE, "means")))
         return rc;
-    const float *tok_scale = reinterpret_cast<const float *>(operand + ncols * w.cols + ncols * units * 16);
-    GemmArgs a{w.rows, n, ncols, units, split, out, tok_scale, aux, epi, 1, ctx->status};
+    const float *tok_scale = reinterpret_cast<const float *>(operand + (terms * w.cols + units * 16) * n);
+    GemmArgs a{w.rows, n, units, terms, out, tok_scale, aux, epi, 1, ctx->status};
     // A result shared by several ranks' copies takes an instantiation that stores to all of them: with
     // TMA from shared memory when every copy's slice starts on a 16-byte boundary, else from registers.
     int shared = out.world > 1 && !out.scatter_per ? 1 : 0;
@@ -1135,14 +1214,14 @@ int launch_gemm(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, 
             if (reinterpret_cast<uintptr_t>(out.dst[p] + out.row0) % 16) shared = 1;
         for (int p = 0; p < out.world && shared == 2; p++)
             if ((rc = encode_2d(ctx, &maps.m[p], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, out.dst[p] + out.row0, w.rows, n,
-                                out.pitch * sizeof(float), TILE_M, (uint32_t)(C::DRAIN_COLS >> (split ? 1 : 0)),
+                                out.pitch * sizeof(float), TILE_M, (uint32_t)C::DRAIN_COLS,
                                 CU_TENSOR_MAP_SWIZZLE_NONE, "output")))
                 return rc;
     }
-    auto kern = gemm_q4k_kernel<BN, 0>;
+    auto kern = gemm_q4k_kernel<BN, 0, MODE>;
     if constexpr (BN != 192) {      // which gemm_large takes for one destination alone
-        if (shared == 2) kern = gemm_q4k_kernel<BN, 2>;
-        if (shared == 1) kern = gemm_q4k_kernel<BN, 1>;
+        if (shared == 2) kern = gemm_q4k_kernel<BN, 2, MODE>;
+        if (shared == 1) kern = gemm_q4k_kernel<BN, 1, MODE>;
     } else if (shared) {
         return fail(ctx, DWIM_B200_EINVAL, "tiles of 192 columns have one destination");
     }
@@ -1151,9 +1230,9 @@ int launch_gemm(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, 
         DWIM_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
         configured[ctx->device & 63][shared] = true;
     }
-    dim3 grid((unsigned)((w.rows + TILE_M - 1) / TILE_M), (unsigned)((ncols + BN - 1) / BN));
+    dim3 grid((unsigned)((w.rows + TILE_M - 1) / TILE_M), (unsigned)((n + BN - 1) / BN));
     if (!shared) {
-        a.split_k = gemm_split<BN>(ctx, w, ncols);
+        a.split_k = gemm_split<BN, MODE>(ctx, w, n, terms);
         grid.x *= a.split_k;
     }
     const bool dependent = !ctx->weights_written;   // see dwim_b200_ctx::weights_written
@@ -1164,33 +1243,34 @@ int launch_gemm(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, 
     return 0;
 }
 
-template <int FMT, int BN>
-int launch_dense(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, size_t n, int split, const OutSpec &out, const float *aux,
+template <int FMT, int BN, int MODE>
+int launch_dense(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, size_t n, int terms, const OutSpec &out, const float *aux,
                  int epi) {
-    using C = DenseCfg<FMT, BN>;
-    const size_t ncols = n * (split ? 2 : 1), units = w.cols / 256;
+    using C = DenseCfg<FMT, BN, MODE>;
+    const size_t units = w.cols / 256;
     CUtensorMap tw, tx;
     int rc;
     // packed weights as bytes; rows past the end read as zeros (Q6_K's zero bytes are weights of -32 times a sub-scale of zero)
     if ((rc = encode_2d(ctx, &tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, w.quants, w.qpitch, w.rows, w.qpitch, FMT == Q8_0 ? 128 : Q6_K_DEV, TILE_M,
                         FMT == Q8_0 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, "weight")))
         return rc;
-    if ((rc = encode_2d(ctx, &tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, operand, w.cols, ncols, w.cols * 2, BK, BN, CU_TENSOR_MAP_SWIZZLE_128B,
+    if ((rc = encode_2d(ctx, &tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, operand, w.cols, terms * n, w.cols * 2, BK, BN, CU_TENSOR_MAP_SWIZZLE_128B,
                         "activation")))
         return rc;
-    const float *tok_scale = reinterpret_cast<const float *>(operand + ncols * w.cols + ncols * units * 16);
-    DenseArgs a{w.rows, n, units, split, epi, 1, out, w.scales, w.srow, tok_scale, aux, ctx->status};
+    const float *tok_scale = reinterpret_cast<const float *>(operand + (terms * w.cols + units * 16) * n);
+    DenseArgs a{w.rows, n, units, terms, epi, 1, out, w.scales, w.srow, tok_scale, aux, ctx->status};
     const bool shared = out.world > 1 && !out.scatter_per;
-    auto kern = shared ? gemm_dense_kernel<FMT, BN, true> : gemm_dense_kernel<FMT, BN, false>;
+    auto kern = shared ? gemm_dense_kernel<FMT, BN, MODE, true> : gemm_dense_kernel<FMT, BN, MODE, false>;
     static std::atomic<bool> configured[64][2] = {};
     if (!configured[ctx->device & 63][shared]) {
         DWIM_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
         configured[ctx->device & 63][shared] = true;
     }
-    dim3 grid((unsigned)((w.rows + TILE_M - 1) / TILE_M), (unsigned)((ncols + BN - 1) / BN));
+    dim3 grid((unsigned)((w.rows + TILE_M - 1) / TILE_M), (unsigned)((n + BN - 1) / BN));
     if (!shared) {
         static std::atomic<int> known[64][MAX_SPLIT + 1] = {};
-        a.split_k = pick_split(ctx, kern, GEMM_THREADS, (size_t)C::SMEM, C::split_fits, SplitCost{2.0, 4.5}, known, (long)grid.x * grid.y, (int)units);
+        a.split_k = pick_split(ctx, kern, GEMM_THREADS, (size_t)C::SMEM, C::split_fits, SplitCost{2.0, 4.5}, known, (long)grid.x * grid.y, (int)units,
+                               terms == 1 ? 1.0 : 1.9);
         grid.x *= a.split_k;
     }
     const bool dependent = !ctx->weights_written;   // see dwim_b200_ctx::weights_written
@@ -1214,29 +1294,33 @@ bool gemm_supports(const WeightView &w) {
     return w.fmt == Q4_K || ((w.fmt == Q6_K || w.fmt == Q8_0) && w.cols <= 12288);
 }
 
-int gemm_large(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, size_t n, int split, const OutSpec &out,
+int gemm_large(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, size_t n, int terms, const OutSpec &out,
                const float *aux, int epilogue) {
     if (!gemm_supports(w)) return fail(ctx, DWIM_B200_EFORMAT, "the tensor-core GEMM does not take format %d", w.fmt);
-    const size_t ncols = n * (split ? 2 : 1);
     if (w.fmt == Q4_K) {
-        if (ncols <= 32) return launch_gemm<32>(ctx, w, operand, n, split, out, aux, epilogue);
-        if (ncols <= 64) return launch_gemm<64>(ctx, w, operand, n, split, out, aux, epilogue);
-        if (ncols <= 128) return launch_gemm<128>(ctx, w, operand, n, split, out, aux, epilogue);
+        if (n <= 16) return launch_gemm<16, SIDE_BY_SIDE>(ctx, w, operand, n, terms, out, aux, epilogue);
+        if (n <= 32) return launch_gemm<32, SIDE_BY_SIDE>(ctx, w, operand, n, terms, out, aux, epilogue);
+        if (n <= 64) return launch_gemm<64, SIDE_BY_SIDE>(ctx, w, operand, n, terms, out, aux, epilogue);
+        if (n <= 128) return (terms == 1 ? launch_gemm<128, ONE_TERM> : launch_gemm<128, SIDE_BY_SIDE>)(ctx, w, operand, n, terms, out, aux, epilogue);
         // Above that, tiles of 192 or 256 columns: a wave of the narrower ones lasts 0.77 of one of the wider
         // when it is the only one ([18944, 5120], 148 tiles: 36.5 us and 47.4; K = 17408: 116 and 150), 0.82 in a
         // row of them (three quarters of the columns, an activations' ring of four stages instead of three), so
         // the waves decide: [17408, 5120] by 131 bf16 tokens 51.9 us in tiles of 256 and 41.5 of 192, by 384 94.0 and
         // 76.9; [5120, 17408] by 131 64.4 and 54.6; by 2048 tokens 256 takes eight waves, 192 eleven.
-        if (out.world == 1 && 0.82 * gemm_time<192>(ctx, w, ncols) < gemm_time<256>(ctx, w, ncols))
-            return launch_gemm<192>(ctx, w, operand, n, split, out, aux, epilogue);
-        return launch_gemm<256>(ctx, w, operand, n, split, out, aux, epilogue);
+        auto wide = [&](auto mode) {
+            constexpr int M = decltype(mode)::value;
+            if (out.world == 1 && 0.82 * gemm_time<192, M>(ctx, w, n, terms) < gemm_time<256, M>(ctx, w, n, terms))
+                return launch_gemm<192, M>(ctx, w, operand, n, terms, out, aux, epilogue);
+            return launch_gemm<256, M>(ctx, w, operand, n, terms, out, aux, epilogue);
+        };
+        return terms == 1 ? wide(std::integral_constant<int, ONE_TERM>()) : wide(std::integral_constant<int, TWO_PASSES>());
     }
-    if (w.fmt == Q6_K) {
-        if (ncols <= 128) return launch_dense<Q6_K, 128>(ctx, w, operand, n, split, out, aux, epilogue);
-        return launch_dense<Q6_K, 256>(ctx, w, operand, n, split, out, aux, epilogue);
-    }
-    if (ncols <= 128) return launch_dense<Q8_0, 128>(ctx, w, operand, n, split, out, aux, epilogue);
-    return launch_dense<Q8_0, 256>(ctx, w, operand, n, split, out, aux, epilogue);
+    auto dense = [&](auto fmt) {
+        constexpr int F = decltype(fmt)::value;
+        if (n <= 128) return launch_dense<F, 128, SIDE_BY_SIDE>(ctx, w, operand, n, terms, out, aux, epilogue);
+        return (terms == 1 ? launch_dense<F, 256, ONE_TERM> : launch_dense<F, 256, TWO_PASSES>)(ctx, w, operand, n, terms, out, aux, epilogue);
+    };
+    return w.fmt == Q6_K ? dense(std::integral_constant<int, Q6_K>()) : dense(std::integral_constant<int, Q8_0>());
 }
 
 }  // namespace dwim

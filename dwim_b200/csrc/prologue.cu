@@ -181,8 +181,8 @@ int build_panels_i8(dwim_b200_ctx *ctx, const float *x, size_t n, size_t cols, u
 // Bytes of the GEMM's operand for n tokens (ncols = n, or 2n when an f32 activation travels as two
 // columns): the f16 rows, the sub-block means, and one f32 scale per token.
 size_t gemm_operand_bytes(size_t cols, size_t n, int split) {
-    const size_t ncols = n * (split ? 2 : 1);
-    return ncols * cols * sizeof(__half) + ncols * (cols / 256) * 16 * sizeof(__half) + ((n * sizeof(float) + 15) & ~size_t(15));
+    const size_t terms = split ? 2 : 1;
+    return (terms * cols + cols / 256 * 16) * n * sizeof(__half) + ((n * sizeof(float) + 15) & ~size_t(15));
 }
 
 // Reductions over a block of THREADS and its cluster (`cluster` blocks share a row), every thread the
@@ -283,8 +283,9 @@ __device__ __noinline__ Terms terms_clamped(float f0, float f1, float f2, float 
 // kernel on larger operand magnitudes runs into the power limit earlier.)
 template <bool NORM, bool SPLIT, int THREADS, int R>
 __global__ void __launch_bounds__(THREADS, THREADS == 512 ? (R > 9 ? 1 : 2) : R > 3 ? 5 : 6) gemm_operand_kernel(const float *x, const float *__restrict__ weight, float eps, float *xout,
-                                                               size_t cols, size_t units, int cluster, __half *__restrict__ x16,
-                                                               __half *__restrict__ means, float *__restrict__ tok_scale) {
+                                                               size_t cols, size_t units, int cluster, size_t n,
+                                                               __half *__restrict__ x16, __half *__restrict__ means,
+                                                               float *__restrict__ tok_scale) {
     if (cluster > 1) cluster_arrive();
     // as the small-M prologues: let the product's kernel begin (it streams weights first),
     // wait for the kernel ahead, which may still read the operand or write x
@@ -341,7 +342,6 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? (R > 9 ? 1 : 2) : R 
     const int e = top ? max(-100, min(100, (int)(top >> 23) - 129)) : 0;
     const float down = __uint_as_float((uint32_t)(127 - e) << 23);
     if (rank == 0 && k == 0) tok_scale[t] = __uint_as_float((uint32_t)(127 + e) << 23);
-    const size_t col = SPLIT ? 2 * t : t;
 #pragma unroll
     for (int r = 0; r < R; r++) {
         const size_t at = place(r);
@@ -350,28 +350,18 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? (R > 9 ? 1 : 2) : R 
         Terms y;
         if (finite) y = terms_finite<SPLIT>(f);
         else y = terms_clamped(f[0], f[1], f[2], f[3]);
-        *reinterpret_cast<uint2 *>(x16 + col * cols + at) = y.hi;
-        if (SPLIT) *reinterpret_cast<uint2 *>(x16 + (col + 1) * cols + at) = y.lo;
+        *reinterpret_cast<uint2 *>(x16 + t * cols + at) = y.hi;
+        if (SPLIT) *reinterpret_cast<uint2 *>(x16 + (n + t) * cols + at) = y.lo;
         // sub-block sums over the eight threads that share it
+        float sum = SPLIT ? y.sh + y.sl : y.sh;
 #pragma unroll
-        for (int o = 1; o < 8; o <<= 1) {
-            y.sh += __shfl_xor_sync(0xffffffffu, y.sh, o);
-            if (SPLIT) y.sl += __shfl_xor_sync(0xffffffffu, y.sl, o);
-        }
+        for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         if ((k & 7) == 0) {
-            const size_t u = at >> 8;
-            const int j = (int)(at & 255) >> 5;
-            const float mh = y.sh * (1.0f / 32.0f), ml = y.sl * (1.0f / 32.0f);
-            __half *m = means + (col * units + u) * 16;
-            const __half a = to_f16_clamped(mh);
-            m[j] = a;
-            m[8 + j] = to_f16_clamped(mh - __half2float(a));
-            if (SPLIT) {
-                __half *m2 = m + units * 16;
-                const __half b = to_f16_clamped(ml);
-                m2[j] = b;
-                m2[8 + j] = to_f16_clamped(ml - __half2float(b));
-            }
+            const float mean = sum * (1.0f / 32.0f);
+            __half *m = means + (t * units + (at >> 8)) * 16 + ((at & 255) >> 5);
+            const __half hi = to_f16_clamped(mean);
+            m[0] = hi;
+            m[8] = to_f16_clamped(mean - __half2float(hi));
         }
     }
 }
@@ -382,9 +372,9 @@ int build_gemm_operand(dwim_b200_ctx *ctx, const float *x, size_t n, size_t cols
                        float eps, float *xout) {
     if (n == 0 || cols == 0) return 0;
     if (cols % 256) return fail(ctx, DWIM_B200_EINVAL, "GEMM operand: %zu columns are not whole 256-weight units", cols);
-    const size_t units = cols / 256, ncols = n * (split ? 2 : 1);
-    __half *means = out + ncols * cols;
-    float *tok_scale = reinterpret_cast<float *>(means + ncols * units * 16);
+    const size_t units = cols / 256, terms = split ? 2 : 1;
+    __half *means = out + terms * n * cols;
+    float *tok_scale = reinterpret_cast<float *>(means + n * units * 16);
     if (cols > OPERAND_MAX_COLS) return fail(ctx, DWIM_B200_EINVAL, "GEMM operand: rows of %zu activations are too long", cols);
     // A block a row once there are rows for every SM; below that as many blocks a row as there are SMs for.
     // Bound by a row's chain of load, reduction and store at few rows, by the bytes and the conversion's
@@ -418,7 +408,7 @@ int build_gemm_operand(dwim_b200_ctx *ctx, const float *x, size_t n, size_t cols
     using F = std::false_type;
     auto kern = weight ? (split ? pick(T(), T()) : pick(T(), F())) : (split ? pick(F(), T()) : pick(F(), F()));
     DWIM_CUDA(ctx, launch_clustered(!ctx->weights_written, (unsigned)cluster, kern, dim3((unsigned)(n * cluster)), dim3(wide ? 512 : 256), 0,
-                                    ctx->stream, x, weight, eps, xout, cols, units, (int)cluster, out, means, tok_scale));
+                                    ctx->stream, x, weight, eps, xout, cols, units, (int)cluster, n, out, means, tok_scale));
     DWIM_LAUNCHED(ctx);
     return 0;
 }

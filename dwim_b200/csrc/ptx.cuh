@@ -69,13 +69,24 @@ static __device__ __noinline__ void mbar_wait_slow(uint32_t bar, uint32_t parity
         }
     }
 }
-// Bounded wait built on the blocking form.
+// Bounded wait built on the blocking form.  (No call of a function: one that is not inlined would have to live
+// with the registers of the poorest of a kernel's warps, regs_dec below, and does not compile there.)
+__device__ __forceinline__ bool mbar_gave_up(uint64_t &start, uint32_t *status, uint32_t code) {
+    if (*(volatile uint32_t *)status != 0) return true;
+    const uint64_t now = globaltimer();
+    if (start == 0) start = now;
+    if (now - start <= WAIT_LIMIT_NS) return false;
+    atomicOr(status, code);
+    return true;
+}
 __device__ __forceinline__ void mbar_wait_parked(uint32_t bar, uint32_t parity, uint32_t *status, uint32_t code) {
     if (mbar_try(bar, parity)) return;
+    uint64_t start = 0;
 #pragma unroll 1
-    for (int i = 0; i < 4096; i++)
+    for (uint32_t i = 1;; i++) {
         if (mbar_try_suspend(bar, parity)) return;
-    mbar_wait_slow(bar, parity, status, code);
+        if (i % 1024 == 0 && mbar_gave_up(start, status, code)) return;
+    }
 }
 __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, uint32_t *status, uint32_t code) {
 #pragma unroll 1
@@ -90,6 +101,11 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, uint32_
 // launch was an ordinary one); griddep_launch() lets the next such launch begin.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// A warpgroup gives up registers of its threads', or takes some that others of its block gave up (and waits
+// until they did).  The shares must add up to no more than the block was launched with.
+template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // Thread-block clusters: all threads of the cluster meet (what they wrote to shared memory before is
 // visible to the others after), at once or in two halves; and loads and stores of another block's shared

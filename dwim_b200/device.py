@@ -124,7 +124,7 @@ class B200:
         self._check(self._L.dwim_b200_touch_bf16(self._ctx, buf._h))
 
     def activation_precision(self, mode: str) -> None:
-        """``"exact"`` (the default: f32 activations as two f16 columns) or ``"f16"`` (one column, the
+        """``"exact"`` (the default: f32 activations as two f16 terms) or ``"f16"`` (one term, the
         precision of the reference's CUDA device: worst error 3e-3 instead of 2e-6, twice the rate) for
         products of more than eight tokens."""
         self._check(self._L.dwim_b200_activation_precision(self._ctx, {"exact": 0, "f16": 1}[mode]))

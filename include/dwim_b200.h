@@ -135,7 +135,7 @@ DWIM_B200_API int dwim_b200_touch(dwim_b200_ctx *ctx, dwim_b200_buffer *buf);
 DWIM_B200_API int dwim_b200_touch_bf16(dwim_b200_ctx *ctx, dwim_b200_buffer *buf);
 /* How f32 activations reach the tensor-core kernels (products of more than
  * eight tokens; the small-M kernel's digit planes are exact either way).
- * EXACT, the default: a token travels as two f16 columns, value and rounding
+ * EXACT, the default: a token travels as two f16 terms, value and rounding
  * remainder, and the product's error stays near 2e-6 of its rms; twice the
  * tensor-core work of a bf16-exact buffer.  F16: one column, the activation
  * rounded to f16 after the token's power-of-two scaling, which is the

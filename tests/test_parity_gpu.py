@@ -842,6 +842,24 @@ def test_gemm_bf16_token_counts(dev, oracle, n):
     assert max_rel_err(dev.read(out).reshape(n, rows), oracle.matmul("q4_k", blocks, rows, cols, x)) <= 2e-5
 
 
+@pytest.mark.parametrize("fmt", FORMATS)
+@pytest.mark.parametrize("n", [9, 16, 17, 32, 33, 64, 65, 128, 129, 192, 193, 256, 257])
+def test_gemm_terms_at_tile_edges(dev, oracle, fmt, n):
+    """f32 activations' two terms side by side or in turn, bf16's one, at the edges of the tiles' token counts."""
+    rng = np.random.default_rng(n)
+    rows, cols = 129, 768
+    weight, w, _, _ = random_pair(dev, oracle, fmt, rows, cols, rng)
+    x = rng.standard_normal((n, cols)).astype(np.float32)
+    bits = oracle.to_bf16(x)
+    out, xb = dev.alloc(n * rows), dev.alloc(n * cols)
+    for bf16 in (False, True):
+        dev.write_bf16(xb, bits) if bf16 else dev.write(xb, x)
+        dev.matmul(out, weight, xb)
+        want = (oracle.bf16(bits).reshape(n, cols) if bf16 else x).astype(np.float64) @ w.T
+        # sums of 768 products in the tensor cores' fp32, f16 pairs for the activations: a few 2^-20 of the result
+        assert max_rel_err(dev.read(out).reshape(n, rows), want) <= 1e-5, bf16
+
+
 @pytest.mark.parametrize("rows,cols,n,bf16", [(1024, 5120, 70, False), (1024, 5120, 131, True), (129, 768, 70, True), (100, 2048, 300, False),
                                               (640, 2304, 600, True), (1024, 17408, 131, False), (5120, 4096, 90, True),
                                               (700, 1280, 161, True), (700, 1280, 192, True), (1500, 1024, 97, False), (2000, 512, 385, True)])
