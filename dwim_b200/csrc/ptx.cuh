@@ -88,6 +88,16 @@ __device__ __forceinline__ void mbar_wait_parked(uint32_t bar, uint32_t parity, 
         if (i % 1024 == 0 && mbar_gave_up(start, status, code)) return;
     }
 }
+// The whole warp waits until the barriers of all its lanes are through.
+__device__ __forceinline__ void mbar_wait_all(uint32_t bar, uint32_t parity, uint32_t *status, uint32_t code) {
+    if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return;
+    uint64_t start = 0;
+#pragma unroll 1
+    for (uint32_t i = 1;; i++) {
+        if (__all_sync(0xffffffffu, mbar_try_suspend(bar, parity))) return;
+        if (i % 1024 == 0 && __any_sync(0xffffffffu, mbar_gave_up(start, status, code))) return;
+    }
+}
 __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, uint32_t *status, uint32_t code) {
 #pragma unroll 1
     for (int i = 0; i < 64; i++)
@@ -197,6 +207,19 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void *tmap, int 
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
         "l"(tmap), "r"(c0), "r"(c1), "r"(bar)
+        : "memory");
+}
+
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void *tmap, int c0, int c1, int c2, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+        "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const void *tmap, int c0, int c1, int c2, int c3, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
+        "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
         : "memory");
 }
 

@@ -39,7 +39,7 @@ def functions(text):
 
 def test_every_function_is_found():
     names = [name for f in SOURCES for name, _ in functions(source(f))]
-    assert {"normalize_i8_kernel", "matmul_bf16_tile_kernel", "gemm_q4k_kernel", "gemm_dense_kernel", "dwim_smallm_kernel",
+    assert {"normalize_i8_kernel", "matmul_bf16_tile_kernel", "gemm_q4k_kernel", "gemm_dense_kernel", "gemm_few_kernel", "dwim_smallm_kernel",
             "push_shares"} <= set(names)
 
 

@@ -860,6 +860,38 @@ def test_gemm_terms_at_tile_edges(dev, oracle, fmt, n):
         assert max_rel_err(dev.read(out).reshape(n, rows), want) <= 1e-5, bf16
 
 
+@pytest.mark.parametrize("rows,cols,n,bf16", [(129, 256, 9, False), (1000, 512, 16, True), (77, 768, 17, False), (640, 1024, 32, True),
+                                              (1024, 5120, 12, False), (5121, 2304, 31, False), (300, 17408, 16, False), (19000, 512, 20, True)])
+def test_q4_k_few_tokens(dev, oracle, rows, cols, n, bf16):
+    """9 to 32 tokens: one to 68 units of K dealt to four groups and to a cluster's blocks, ragged rows, every epilogue."""
+    rng = np.random.default_rng(rows)
+    weight, w, other, w2 = random_pair(dev, oracle, "q4_k", rows, cols, rng)
+    x = rng.standard_normal((n, cols)).astype(np.float32)
+    x[1] *= 30.0
+    xb = dev.alloc(n * cols)
+    if bf16:
+        bits = oracle.to_bf16(x)
+        dev.write_bf16(xb, bits)
+        x = oracle.bf16(bits).reshape(n, cols)
+    else:
+        dev.write(xb, x)
+    x = x.astype(np.float64)
+    y, z = x @ w.T, x @ w2.T
+    out, scratch, h = dev.alloc(n * rows), dev.alloc(n * rows), rng.standard_normal((n, rows)).astype(np.float32)
+    res = dev.buffer(h)
+    dev.matmul(out, weight, xb)
+    got = dev.read(out).reshape(n, rows)
+    dev.matmul_add(res, weight, xb)
+    added = dev.read(res).reshape(n, rows)
+    dev.swiglu(out, weight, other, xb, scratch)
+    gated = dev.read(out).reshape(n, rows)
+    # the products' sums to 1e-5 of a token's typical result; silu(g) u by twice that of its factors
+    for t in range(n):
+        assert max_rel_err(got[t], y[t]) <= 1e-5
+        assert max_rel_err(added[t], h[t] + y[t]) <= 2e-5
+        assert np.abs(gated[t] - silu_times(y[t], z[t])).max() <= 3e-5 * np.sqrt((y[t] ** 2).mean()) * np.abs(z[t]).max()
+
+
 @pytest.mark.parametrize("rows,cols,n,bf16", [(1024, 5120, 70, False), (1024, 5120, 131, True), (129, 768, 70, True), (100, 2048, 300, False),
                                               (640, 2304, 600, True), (1024, 17408, 131, False), (5120, 4096, 90, True),
                                               (700, 1280, 161, True), (700, 1280, 192, True), (1500, 1024, 97, False), (2000, 512, 385, True)])
