@@ -20,7 +20,7 @@ static constexpr size_t WEIGHT_SLACK = 1024;
 
 namespace dwim {
 // gemm.cu
-bool gemm_supports(const WeightView &w);
+bool gemm_takes(const WeightView &w, size_t n, int terms);
 int gemm_large(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, size_t n, int terms, const OutSpec &out,
                const float *aux, int epilogue);
 
@@ -474,25 +474,62 @@ static int ensure_shadow(dwim_b200_ctx *ctx, dwim_b200_buffer *x, int kind, size
 
 constexpr size_t GROUPS_AT_ONCE = 64;
 
-// Room for the digit planes of all the groups of eight tokens that `x` can hold, up to GROUPS_AT_ONCE.  It spares
-// launches and no product needs it: it is never made anew at another length of the buffer (a graph captured at one
-// length may still read it), not allocated under a stream capture, and done without when memory is short.
+static bool capturing(dwim_b200_ctx *ctx) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) return false;
+    cudaGetLastError();
+    return true;
+}
+
+// Room for products of Q6_K and Q8_0 by nine tokens and more: the digit planes of all the groups of eight tokens that
+// `x` can hold, up to GROUPS_AT_ONCE, or its operand for the dense kernel, in one array.  It spares launches or time and
+// no product needs it: it is never made anew at another length of the buffer (a graph captured at one length may still
+// read it), not allocated under a stream capture, and done without when memory is short.
 static void reserve_groups(dwim_b200_ctx *ctx, dwim_b200_buffer *x, size_t cols, size_t group) {
     size_t most = x->cap / cols / I8_MAX_TOKENS;
     if (most > GROUPS_AT_ONCE) most = GROUPS_AT_ONCE;
-    if (x->groups_tried || most < 2) return;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        return;
-    }
+    if (x->groups_tried || most < 2 || capturing(ctx)) return;
+    // the dense kernel's: of all the tokens where it takes any number in this way, else of its tile's
+    size_t tokens = x->cap / cols;
+    if (tokens > 64 && cols <= 12288) tokens = 64;
+    const size_t planes = most * group, operand = cols % 256 ? 0 : gemm_operand_bytes(cols, tokens, 1);
     x->groups_tried = true;
-    if (cudaMalloc(&x->groups, most * group) == cudaSuccess) {
-        x->groups_cap = most * group;
-    } else {
+    for (size_t bytes = planes > operand ? planes : operand;; bytes = planes) {
+        if (cudaMalloc(&x->groups, bytes) == cudaSuccess) {
+            x->groups_cap = bytes;
+            return;
+        }
         x->groups = nullptr;
         cudaGetLastError();
+        if (bytes == planes) return;
     }
+}
+
+// The operand of a product that the groups of eight tokens could take as well: in the shadow where it fits, else in the
+// groups' array; null where there is no room.  (The shadow is not made longer for it: graphs captured with the groups'
+// planes in it would read freed memory.  Under a capture the conversion is part of the graph, as the groups' is.)
+static int operand_apart(dwim_b200_ctx *ctx, dwim_b200_buffer *x, size_t cols, size_t n, int split, const __half **operand) {
+    const size_t need = gemm_operand_bytes(cols, n, split);
+    *operand = nullptr;
+    const bool fits = need <= x->shadow_cap;
+    const int kind = x->shadow_kind;
+    if ((kind == SHADOW_GEMM || kind == SHADOW_GEMM_APART) && x->shadow_cols == cols && x->shadow_split == split && !capturing(ctx)) {
+        *operand = (const __half *)(kind == SHADOW_GEMM ? x->shadow : x->groups);
+        return 0;
+    }
+    if (!fits) {
+        reserve_groups(ctx, x, cols, panel_i8_bytes(cols, I8_MAX_TOKENS));
+        if (need > x->groups_cap) return 0;
+    }
+    void *place = fits ? x->shadow : x->groups;
+    x->shadow_kind = SHADOW_NONE;
+    int rc = build_gemm_operand(ctx, x->data, n, cols, split, (__half *)place);
+    if (rc) return rc;
+    x->shadow_kind = fits ? SHADOW_GEMM : SHADOW_GEMM_APART;
+    x->shadow_cols = cols;
+    x->shadow_split = split;
+    *operand = (const __half *)place;
+    return 0;
 }
 
 static int product(dwim_b200_ctx *ctx, const OutSpec &out, size_t out_len, const dwim_b200_weight *w, dwim_b200_buffer *x,
@@ -506,19 +543,21 @@ static int product(dwim_b200_ctx *ctx, const OutSpec &out, size_t out_len, const
     REQUIRE(ctx, out.dst[0] != x->data, DWIM_B200_EINVAL, "%s: output aliases input", what);
     // bf16 weights (the small gate matrices): f32 activations as they are, fp32 throughout
     if (v.fmt == BF16) return matmul_bf16(ctx, v, x->data, n, out, aux, epilogue);
-    // Up to eight tokens: the small-M kernel's int8 routines.  Above: the tensor-core kernels -- Q4_K
-    // from nine tokens on (measured on B200 at [17408, 5120]: 26 us at nine to sixteen tokens, against
-    // 57 us for sixteen through two small-M launches); Q6_K and Q8_0 from 65 on, and in groups of eight through
-    // the small-M kernel below that.  (Their dense kernel would be faster from 33 tokens, but sums in the tensor
-    // cores: 2.8e-7 to 6.7e-7 of the result in 2-norm, where the groups' integer products give 3e-7 by f32
-    // activations and 1.2e-7 by bf16 ones.)
-    const bool dense = gemm_supports(v) && n > (v.fmt == Q4_K ? (size_t)I8_MAX_TOKENS : (size_t)64);
-    if (dense) {
-        // bf16 activations are exact in one f16 term; f32 ones travel as two (value and rounding remainder)
-        int split = x->bf16_exact || ctx->act_f16 ? 0 : 1;
-        int rc = ensure_shadow(ctx, x, SHADOW_GEMM, v.cols, split);
+    // Up to eight tokens: the small-M kernel's int8 routines.  Above: the tensor-core kernels where they are the
+    // better ones (gemm_takes), the small-M kernel in groups of eight tokens elsewhere.
+    // bf16 activations are exact in one f16 term; f32 ones travel as two (value and rounding remainder).
+    const int split = x->bf16_exact || ctx->act_f16 ? 0 : 1;
+    if (gemm_takes(v, n, 1 + split)) {
+        const __half *operand;
+        int rc;
+        if (v.fmt != Q4_K && split && (n <= 64 || v.cols > 12288)) {
+            rc = operand_apart(ctx, x, v.cols, n, split, &operand);
+        } else {
+            rc = ensure_shadow(ctx, x, SHADOW_GEMM, v.cols, split);
+            operand = (const __half *)x->shadow;
+        }
         if (rc) return rc;
-        return gemm_large(ctx, v, (const __half *)x->shadow, n, split ? 2 : 1, out, aux, epilogue);
+        if (operand) return gemm_large(ctx, v, operand, n, split ? 2 : 1, out, aux, epilogue);
     }
     if (!gemv_takes_i8(v, n < (size_t)I8_MAX_TOKENS ? n : (size_t)I8_MAX_TOKENS))
         return fail(ctx, DWIM_B200_EFORMAT, "%s: no kernel takes format %d with %zu columns", what, v.fmt, v.cols);
@@ -540,7 +579,7 @@ static int product(dwim_b200_ctx *ctx, const OutSpec &out, size_t out_len, const
         if (groups > room) groups = room;
     }
     uint8_t *const panels = (uint8_t *)(groups * group > x->shadow_cap ? x->groups : x->shadow);
-    if (panels == x->shadow) x->shadow_kind = SHADOW_NONE;
+    if (panels == x->shadow || x->shadow_kind == SHADOW_GEMM_APART) x->shadow_kind = SHADOW_NONE;
     for (size_t t0 = 0; t0 < n;) {
         const size_t left = n - t0, g = left < (size_t)I8_MAX_TOKENS ? 1 : left / I8_MAX_TOKENS < groups ? left / I8_MAX_TOKENS : groups;
         const size_t nt = left < (size_t)I8_MAX_TOKENS ? left : (size_t)I8_MAX_TOKENS;

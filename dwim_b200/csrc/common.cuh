@@ -16,7 +16,8 @@
 enum ShadowKind : int {
     SHADOW_NONE = 0,
     SHADOW_GEMM,            // f16 rows, sub-block means and token scales, for the tensor-core kernels
-    SHADOW_PANEL_I8         // int8 digit planes per 256-wide unit, for the small-M kernel
+    SHADOW_PANEL_I8,        // int8 digit planes per 256-wide unit, for the small-M kernel
+    SHADOW_GEMM_APART       // as SHADOW_GEMM, in the groups' array
 };
 
 constexpr int DWIM_MAX_WORLD = 8;
@@ -40,8 +41,8 @@ struct dwim_b200_buffer {
     int shadow_kind = SHADOW_NONE;
     size_t shadow_cols = 0;      // K the shadow was built for
     int shadow_split = 0;        // 1: hi/lo column pairs, 0: single f16
-    // The digit planes of several groups of eight tokens (products of Q6_K and Q8_0 by nine tokens and more),
-    // where the shadow holds fewer.  Allocated once and kept to the buffer's end.
+    // The digit planes of several groups of eight tokens, or the dense kernel's operand (products of Q6_K and Q8_0 by
+    // nine tokens and more), where the shadow holds less.  Allocated once and kept to the buffer's end.
     void *groups = nullptr;
     size_t groups_cap = 0;       // bytes
     bool groups_tried = false;

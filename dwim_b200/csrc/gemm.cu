@@ -581,15 +581,17 @@ struct DenseArgs {
     const float *tok_scale, *aux;
     uint32_t *status;
 };
-// Two terms that take turns double the additions to an accumulator, so it is drained twice a unit.
+// Two terms that take turns double the additions to an accumulator, so it is drained twice a unit; tiles of 64 columns
+// take the place of exact sums and drain every K block.
 template <int FMT, int BN, int MODE> struct DenseCfg {
     static constexpr bool WIDE = MODE == SIDE_BY_SIDE;
-    static constexpr int DRAIN_KB = MODE == TWO_PASSES ? 2 : KBLOCKS;      // K blocks between drains
+    static constexpr int DRAIN_KB = BN <= 64 ? 1 : MODE == TWO_PASSES ? 2 : KBLOCKS;      // K blocks between drains
     static constexpr int TERM_BYTES = BN * BK * 2, ACC_COLS = BN * (WIDE ? 2 : 1);
-    static constexpr int A_STAGES = 2, A_STAGE = 2 * A_BYTES;
+    static constexpr int A_STAGES = BN <= 64 ? 4 : 2, A_STAGE = 2 * A_BYTES;
     static constexpr int STEPS = KBLOCKS / DRAIN_KB;                // drains of a unit
     // Accumulator buffers: two units' where tensor memory holds them, else two steps'.
     static constexpr int ACC_BUFS = 2 * STEPS * ACC_COLS <= 512 ? 2 * STEPS : 2;
+    static_assert(STEPS < 4 || (ACC_BUFS == 8 && BN == 64), "drain_unit");
     static_assert(ACC_BUFS == 2 * STEPS || STEPS == 2, "a unit of more steps than buffers would wait for itself");
     static constexpr int TMEM_COLS = ACC_BUFS * ACC_COLS > 256 ? 512 : 256;
     static constexpr int B_STAGES = ACC_COLS > 128 ? 3 : 4, B_BYTES = TERM_BYTES * (WIDE ? 2 : 1);
@@ -709,7 +711,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                     tc_fence_after();
                     if (elect_one()) {
                         // the weights' remainders first: they are too small for the accumulator's rounding to matter
-                        const uint32_t hi = a_lo + (g & 1) * (C::A_STAGE >> 4), lo = hi + (A_BYTES >> 4), bd = b_lo + bs * (C::B_BYTES >> 4);
+                        const uint32_t hi = a_lo + g % C::A_STAGES * (C::A_STAGE >> 4), lo = hi + (A_BYTES >> 4), bd = b_lo + bs * (C::B_BYTES >> 4);
 #pragma unroll
                         for (int k = 0; k < BK / 16; k++) {
                             if (g % DRAIN_KB == 0 && k == 0) umma_f16_lo(acc, lo, bd, DESC_HI_SW128, idesc, p != PASSES - 1);
@@ -733,7 +735,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         regs_inc<DENSE_WORKER_REGS>();
         const int quad = warp & 3, g = warp >> 2, rl = quad * 32 + lane;
         const uint32_t drain_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + g * C::DRAIN_COLS;
-        const uint32_t a_row_sw = (astage0 + (g & 1) * C::A_STAGE + rl * 128) | ((rl & 7) << 4);
+        const uint32_t a_row_sw = (astage0 + g % C::A_STAGES * C::A_STAGE + rl * 128) | ((rl & 7) << 4);
         const size_t row = (size_t)row0 + rl;
         uint64_t acc2[C::DRAIN_COLS / 2];
 #pragma unroll
@@ -764,6 +766,34 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             if (lane == 0) mbar_arrive(accempty0 + 8 * buf);
             if (++buf == C::ACC_BUFS) buf = 0, bufturn ^= 1;
         };
+        // All four steps of unit u: their sums meet before they reach the row's, which rounds once a unit so.
+        auto drain_unit = [&](int u) {
+            const uint32_t sc = __float_as_uint(lds32f(scale0 + ((u % SCALE_SLOTS) * TILE_M + rl) * 4));
+            const uint64_t sc2 = pack2(sc, sc);
+            uint64_t sum[C::DRAIN_COLS / 2];
+#pragma unroll
+            for (int half = 0; half < 2; half++) {
+                uint32_t v[2][16];
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    mbar_wait_parked(accfull0 + 8 * (buf + 2 * half + i), bufturn, a.status, 0x2000000u);
+                    tc_fence_after();
+                    tmem_ld16(drain_addr + (buf + 2 * half + i) * C::ACC_COLS, v[i]);
+                }
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < C::DRAIN_COLS / 2; j++) {
+                    const uint64_t two = fadd2(pack2(v[0][2 * j], v[0][2 * j + 1]), pack2(v[1][2 * j], v[1][2 * j + 1]));
+                    if (half == 0) sum[j] = two;
+                    else ffma2(acc2[j], sc2, fadd2(sum[j], two));
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane < 4) mbar_arrive(accempty0 + 8 * (buf + lane));
+            buf ^= 4;
+            if (buf == 0) bufturn ^= 1;
+        };
         // With two buffers for a unit's two steps the first of the unit before is drained ahead of the decode: its
         // buffer is the one that this unit's first step takes, which K blocks 2 and 3 wait for (their stages').
         constexpr int EARLY = C::ACC_BUFS == 2 * C::STEPS ? 0 : 1;
@@ -785,8 +815,10 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 const uint4 sc = fetch(u);
                 const int r = C::RAW_STEPS == 2 ? 2 * u + (g >> 1) : u, rs = r % C::RAW_STAGES;
                 mbar_wait_parked(rawfull0 + 8 * rs, (r / C::RAW_STAGES) & 1, a.status, 0x4000000u);
-                // the stage's last user, two K blocks back, is done (this warp has waited for the use before that one)
-                mbar_wait_parked(adone0 + 8 * (g ^ 2), (u & 1) ^ (g < 2 ? 1 : 0), a.status, 0x8000000u);
+    // the stage's last user is done: the K block of the unit before, or with two stages (this warp has waited for
+                // the use before that one) the one two K blocks back
+                if (C::A_STAGES == KBLOCKS) mbar_wait_parked(adone0 + 8 * g, (u & 1) ^ 1, a.status, 0x8000000u);
+                else mbar_wait_parked(adone0 + 8 * (g ^ 2), (u & 1) ^ (g < 2 ? 1 : 0), a.status, 0x8000000u);
                 const uint32_t raw = raw0 + rs * C::RAW_STAGE;
                 float unit_scale;
                 if constexpr (FMT == Q6_K) {
@@ -847,8 +879,12 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 __syncwarp();
             }
             if (u > 0) {
+                if constexpr (C::STEPS == 4) {
+                    drain_unit(u - 1);
+                } else {
 #pragma unroll 1
-                for (int i = EARLY; i < C::STEPS; i++) drain(u - 1);
+                    for (int i = EARLY; i < C::STEPS; i++) drain(u - 1);
+                }
             }
         }
         float acc[C::DRAIN_COLS];
@@ -1043,21 +1079,26 @@ int launch_dense(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand,
 
 }  // namespace
 
-// Formats the tensor-core kernels take: Q4_K, and the others up to 12288 columns.  Longer rows go through the
-// small-M kernel in groups of eight tokens at any token count.  The dense kernel could take them (its error and
-// shared memory do not depend on K; the operand's prologue ends at 51200 columns) and would be faster: [5120,
-// 17408] Q6_K by 65 bf16 tokens 212 us in groups, 70 dense, by 512 f32 ones 1445 and 336; Q8_0 193 and 72,
-// 1293 and 337.  But it sums in the tensor cores: 4.6e-7 (Q6_K) and 6.7e-7 (Q8_0) of the result in 2-norm by f32
-// activations where the groups give 3.1e-7, 2.8e-7 and 6.4e-7 by bf16 ones where they give 1.2e-7.  So the line
-// stays where the two paths' precision has been since the dense path was limited by its decoder to such rows.
-bool gemm_supports(const WeightView &w) {
+// Whether the tensor-core kernels take a product of n tokens by so many f16 terms: Q4_K from nine tokens on (25 us at
+// nine to sixteen in the kernel of many columns, [17408, 5120], against 57 for sixteen through two small-M launches).
+// Q6_K and Q8_0, whose alternative is the small-M kernel in groups of eight tokens, by time and by error:
+//   two terms (f32 activations): from 25 tokens on.  Drained every K block (up to 64 tokens, and rows above 12288) the
+//     dense kernel's error is 1.3e-7 to 1.5e-7 of the result in 2-norm, the groups' 2.9e-7 to 3.1e-7 (23-bit planes).
+//     Products with their operand, us, at 16, 24, 32 and 48 tokens: Q8_0 [5120, 5120] 21 31 32 51 in groups, 27 28 28 29
+//     dense; [12288, 5120] 37 53 64 96 and 58 58 58 58; [1024, 5120] 11 16 18 26 and 17; [20000, 1024] 20 29 38 54 and 30;
+//     [5120, 17408] by 32 88 and 73, by 512 1293 and 512; Q6_K within a tenth of these.
+//   one term (bf16 activations): from 65 tokens on, up to 12288 columns.  It would be faster from 17 on ([5120, 5120] by
+//     48 22 us, 51 in groups), but its error is 0.9e-7 to 1.3e-7 where the groups' is 0.6e-7 to 1.2e-7.
+constexpr size_t DENSE_FROM[2] = {65, 25};      // tokens, by one and two terms
+bool gemm_takes(const WeightView &w, size_t n, int terms) {
     if (w.cols % 256) return false;
-    return w.fmt == Q4_K || ((w.fmt == Q6_K || w.fmt == Q8_0) && w.cols <= 12288);
+    if (w.fmt == Q4_K) return n > (size_t)I8_MAX_TOKENS;
+    return (w.fmt == Q6_K || w.fmt == Q8_0) && n >= DENSE_FROM[terms - 1] && w.cols <= (terms == 2 ? 51200 : 12288);
 }
 
 int gemm_large(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, size_t n, int terms, const OutSpec &out,
                const float *aux, int epilogue) {
-    if (!gemm_supports(w)) return fail(ctx, DWIM_B200_EFORMAT, "the tensor-core GEMM does not take format %d", w.fmt);
+    if (!gemm_takes(w, n, terms)) return fail(ctx, DWIM_B200_EFORMAT, "the tensor-core GEMM does not take format %d, %zu tokens", w.fmt, n);
     if (w.fmt == Q4_K) {
         // (at 33 tokens and more a tile of 64 columns: tensor memory holds four groups' sums of 32)
         if (n <= 32 && (out.world == 1 || out.scatter_per)) return gemm_few(ctx, w, operand, n, terms, out, aux, epilogue);
@@ -1077,8 +1118,11 @@ int gemm_large(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, s
         };
         return terms == 1 ? wide(std::integral_constant<int, ONE_TERM>()) : wide(std::integral_constant<int, TWO_PASSES>());
     }
+    // few tokens, or long rows: drained every K block, for the groups' precision (gemm_takes)
     auto dense = [&](auto fmt) {
         constexpr int F = decltype(fmt)::value;
+        if (n <= 64 || w.cols > 12288)
+            return launch_dense<F, 64, TWO_PASSES>(ctx, w, operand, n, terms, out, aux, epilogue);
         if (n <= 128) return launch_dense<F, 128, SIDE_BY_SIDE>(ctx, w, operand, n, terms, out, aux, epilogue);
         return (terms == 1 ? launch_dense<F, 256, ONE_TERM> : launch_dense<F, 256, TWO_PASSES>)(ctx, w, operand, n, terms, out, aux, epilogue);
     };

@@ -1009,6 +1009,67 @@ def test_dense_kernel_shares_k_between_blocks(dev, oracle, fmt, rows, cols, n):
     assert np.abs(dev.read(out).reshape(n, rows) - silu).max() <= 4 * bar * max(1.0, np.abs(want).max())
 
 
+@pytest.mark.parametrize("fmt", ["q6_k", "q8_0"])
+@pytest.mark.parametrize("rows,cols,n", [(129, 256, 25), (300, 2304, 64), (2600, 1024, 33), (96, 17408, 30), (64, 12544, 130)])
+def test_dense_kernel_drained_every_k_block(dev, oracle, fmt, rows, cols, n):
+    """f32 activations of 25 to 64 tokens, and of rows above 12288: as exact as the digit planes that it replaces."""
+    rng = np.random.default_rng(cols)
+    weight, w, _, _ = random_pair(dev, oracle, fmt, rows, cols, rng)
+    x = rng.standard_normal((n, cols)).astype(np.float32)
+    want = x.astype(np.float64) @ w.T
+    out, xb, h = dev.alloc(n * rows), dev.buffer(x), rng.standard_normal((n, rows)).astype(np.float32)
+    dev.matmul(out, weight, xb)
+    got = dev.read(out).reshape(n, rows)
+    # three digit planes round an activation at 2^-23 of its unit's largest, three to four times its size: 3e-7 in 2-norm
+    assert np.linalg.norm(got - want) <= 3e-7 * np.linalg.norm(want)
+    res = dev.buffer(h)
+    dev.matmul_add(res, weight, xb)                       # the operand kept from the product before
+    assert max_rel_err(dev.read(res).reshape(n, rows), h + want) <= 1e-5
+    dev.write(xb, x[::-1])                                # and made anew after a write
+    dev.matmul(out, weight, xb)
+    assert np.array_equal(dev.read(out).reshape(n, rows), got[::-1])
+
+
+@pytest.mark.parametrize("fmt", ["q6_k", "q8_0"])
+def test_dense_kernel_of_few_tokens_under_capture(oracle, fmt):
+    """The operand is not the shadow's: captured after a product that left one, a graph makes its own at every replay,
+    and a shadow that an earlier graph reads stays where it is."""
+    import torch
+    from dwim_b200 import B200, Tensor
+    stream = torch.cuda.Stream()
+    d = B200(0, stream=stream.cuda_stream)
+    try:
+        rng = np.random.default_rng(73)
+        rows, cols, n = 96, 2048, 48
+        blocks = oracle.quantize(fmt, (0.02 * rng.standard_normal((rows, cols))).astype(np.float32))
+        weight = d.upload(Tensor(fmt, (rows, cols), blocks))
+        x = rng.standard_normal((3, n, cols)).astype(np.float32)
+        want = [oracle.matmul(fmt, blocks, rows, cols, y).reshape(n, rows) for y in x]
+        xb, out = d.buffer(x[0]), d.alloc(n * rows)
+        d.resize(xb, 8 * cols)
+        d.resize(out, 8 * rows)
+        d.matmul(out, weight, xb)                         # eight tokens' planes: all that the first graph has
+        d.resize(xb, n * cols)
+        d.resize(out, n * rows)
+        graphs = []
+        for i in range(2):
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                d.matmul(out, weight, xb)
+            graphs.append(graph)
+            d.write(xb, x[i])
+            d.matmul(out, weight, xb)
+            assert max_rel_err(d.read(out), want[i]) <= 2e-5
+        for i, graph in ((1, graphs[0]), (2, graphs[1]), (0, graphs[0])):
+            d.write(xb, x[i])
+            with torch.cuda.stream(stream):
+                graph.replay()
+            assert max_rel_err(d.read(out), want[i]) <= 2e-5
+        del graphs, graph
+    finally:
+        d.close()
+
+
 @pytest.mark.parametrize("bf16", [True, False])
 def test_gemm_fused_epilogues_at_256_columns(dev, oracle, bf16):
     """matmul_add and swiglu through the 256-column kernel (300 tokens of bf16
