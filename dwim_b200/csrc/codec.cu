@@ -22,15 +22,22 @@ __global__ void repack_q8_0(const uint16_t *__restrict__ file, size_t rows, size
         else quants[r * (qpitch / 2) + b * 16 + part - 1] = v;
     }
 }
-// Q6_K: a block is 105 halfwords (104 of ql|qh|scales, then d).
+// Q6_K: a block is 105 halfwords (96 of ql|qh, eight of sub-scales, d); the quants' bits are dealt out anew (formats.cuh).
 __global__ void repack_q6_k(const uint16_t *__restrict__ file, size_t rows, size_t nb, size_t srow, size_t qpitch,
                             uint16_t *__restrict__ quants, uint16_t *__restrict__ scales) {
     size_t total = rows * nb * 105;
     for (size_t u = blockIdx.x * (size_t)blockDim.x + threadIdx.x; u < total; u += (size_t)gridDim.x * blockDim.x) {
         size_t blk = u / 105, part = u % 105, r = blk / nb, b = blk % nb;
         uint16_t v = file[u];
-        if (part == 104) scales[r * srow + b] = v;
-        else quants[r * (qpitch / 2) + b * 104 + part] = v;
+        if (part == 104) {
+            scales[r * srow + b] = v;
+            continue;
+        }
+        if (part < 96) {
+            const uint8_t *bytes = reinterpret_cast<const uint8_t *>(file + blk * 105);
+            v = (uint16_t)(q6k_dev_byte(bytes, 2 * (int)part) | q6k_dev_byte(bytes, 2 * (int)part + 1) << 8);
+        }
+        quants[r * (qpitch / 2) + b * 104 + part] = v;
     }
 }
 

@@ -12,7 +12,11 @@
 // array, both row-major with rows padded to 16 bytes:
 //   Q8_0: quants [rows][cols] i8                scales [rows][pad8(cols/32)] f16
 //   Q6_K: quants [rows][cols/256][208]          scales [rows][pad8(cols/256)] f16
-//         (208 = ql 128 | qh 64 | sub-scales 16)
+//         (208 = quants 192 | sub-scales 16)
+// Q6_K's six bits are dealt out anew, bijectively, for the kernel that reads them most often (gemv.cu).  Of a set of
+// four scale groups (64 weights; t = 0..3) the weights 4c..4c+3 of each group are three words, at 64 j + 16 c + 4 t
+// for j = 0..2: byte b of word j holds u = q ^ 32 of weight 4c + b of the set's group j in bits 2..7 (so that the byte
+// without its low bits is the signed 4 * (q - 32)), and two bits of the same weight of its group 3 in bits 0..1.
 // Rows of every quant array sit `qpitch` bytes apart: the row's bytes rounded
 // up to an odd number of 16-byte steps.  A tile of consecutive rows is then
 // one contiguous run of HBM (one bulk copy into shared memory) and, once
@@ -109,12 +113,32 @@ __device__ __forceinline__ float q4k_weight(const uint8_t *blk, int i) {
     return __fsub_rn(__fmul_rn(__fmul_rn(d, (float)sc), (float)q), __fmul_rn(dmin, (float)m));
 }
 
-// ---- Q6_K (device block: ql[128] qh[64] sc[16]) ------------------------------
-__device__ __forceinline__ int q6k_quant(const uint8_t *blk, int i) {
+// ---- Q6_K -------------------------------------------------------------------
+// the six bits of weight i (0..255) of a file block (ql[128] qh[64] sc[16]; inference/quants.rs:73-104)
+__device__ __forceinline__ int q6k_file_bits(const uint8_t *blk, int i) {
     int half = i >> 7, r = i & 127, k = r >> 5, l = r & 31;
     int low = (blk[half * 64 + l + 32 * (k & 1)] >> (4 * (k >> 1))) & 0xf;
     int high = (blk[128 + half * 32 + l] >> (2 * k)) & 3;
-    return (low | (high << 4)) - 32;
+    return low | (high << 4);
+}
+// byte `at` (0..191) of the device block's quants
+__device__ __forceinline__ int q6k_dev_byte(const uint8_t *file_blk, int at) {
+    const int j = at >> 6, first = ((at >> 2) & 3) * 64 + ((at >> 4) & 3) * 4 + (at & 3);      // the weight of the set's group 0
+    const int own = q6k_file_bits(file_blk, first + 16 * j) ^ 32, last = q6k_file_bits(file_blk, first + 48) ^ 32;
+    return own << 2 | ((last >> (2 * j)) & 3);
+}
+// weight i's quant, -32..31, from the device block
+__device__ __forceinline__ int q6k_quant(const uint8_t *blk, int i) {
+    const int group = i >> 4, k = group & 3, at = ((i >> 2) & 3) * 16 + (group >> 2) * 4 + (i & 3);
+    const int u = k < 3 ? blk[64 * k + at] >> 2 : (blk[at] & 3) | (blk[64 + at] & 3) << 2 | (blk[128 + at] & 3) << 4;
+    return (u ^ 32) - 32;
+}
+// The four groups' bytes, signed 4 * (q - 32), from the three words of a set.
+__device__ __forceinline__ void q6k_bytes(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t (&q)[4]) {
+    q[0] = w0 & 0xfcfcfcfcu;
+    q[1] = w1 & 0xfcfcfcfcu;
+    q[2] = w2 & 0xfcfcfcfcu;
+    q[3] = ((w0 << 2) & 0x0c0c0c0cu) | ((w1 << 4) & 0x30303030u) | ((w2 << 6) & 0xc0c0c0c0u);
 }
 // inference/quants.rs:99: (d * scale) * q, left to right.
 __device__ __forceinline__ float q6k_weight(const uint8_t *blk, float d, int i) {

@@ -822,29 +822,24 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 const uint32_t raw = raw0 + rs * C::RAW_STAGE;
                 float unit_scale;
                 if constexpr (FMT == Q6_K) {
-                    const uint32_t rrow = raw + rl * Q6_K_DEV, ql = rrow + (g >> 1) * 64, qh = rrow + 128 + (g >> 1) * 32;
-                    const int nib = (g & 1) * 4;
-                    const uint32_t s4 = lds32(rrow + 192 + 4 * g) ^ 0x80808080u;      // the four groups' sub-scales + 128
-                    unit_scale = h2f_lo(sc.x);
+                    // The block's four groups (formats.cuh): word j of lane c for them at 64 j + 16 c + 4 g.
+                    const uint32_t rrow = raw + rl * Q6_K_DEV;
+                    const uint32_t s4 = lds32(rrow + 192 + 4 * g) ^ 0x80808080u;      // the groups' sub-scales + 128
+                    unit_scale = 0.25f * h2f_lo(sc.x);                                // the quants come four times as large
+                    uint32_t f[4];                                                    // 0x6480 = 1152 = 1024 + 128
 #pragma unroll
-                    for (int c = 0; c < 2; c++) {
-                        const uint4 h = lds128(qh + 16 * c), l0 = lds128(ql + 16 * c), l1 = lds128(ql + 32 + 16 * c);
-                        const uint32_t hw[4] = {h.x, h.y, h.z, h.w}, w0[4] = {l0.x, l0.y, l0.z, l0.w}, w1[4] = {l1.x, l1.y, l1.z, l1.w};
-                        // 0x6480 = 1152 = 1024 + 128
-                        const uint32_t f0 = hsub2(prmt(s4, 0x64006400u, 0x5050u + c * 0x0101u), 0x64806480u);
-                        const uint32_t f1 = hsub2(prmt(s4, 0x64006400u, 0x5252u + c * 0x0101u), 0x64806480u);
-                        uint32_t v0[4], v1[4];
+                    for (int k = 0; k < 4; k++) f[k] = hsub2(prmt(s4, 0x64006400u, 0x5050u + k * 0x0101u), 0x64806480u);
 #pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            const uint32_t hh = hw[i] >> nib;      // bits 0-1 of a byte: the first 32 weights, bits 2-3: the second
-                            v0[i] = ((w0[i] >> nib) & 0x0f0f0f0fu) | ((hh << 4) & 0x30303030u);
-                            v1[i] = ((w1[i] >> nib) & 0x0f0f0f0fu) | ((hh << 2) & 0x30303030u);
+                    for (int c = 0; c < 4; c += 2) {
+                        uint32_t q[2][4];
+#pragma unroll
+                        for (int i = 0; i < 2; i++) {
+                            const uint32_t at = rrow + 16 * (c + i) + 4 * g;
+                            q6k_bytes(lds32(at), lds32(at + 64), lds32(at + 128), q[i]);
                         }
 #pragma unroll
-                        for (int i = 0; i < 2; i++) {      // 0x6420 = 1056 = 1024 + 32
-                            store_terms(v0[2 * i], v0[2 * i + 1], 0x64206420u, f0, a_row_sw, 2 * c + i);
-                            store_terms(v1[2 * i], v1[2 * i + 1], 0x64206420u, f1, a_row_sw, 4 + 2 * c + i);
-                        }
+                        for (int k = 0; k < 4; k++)
+                            store_terms(q[0][k] ^ 0x80808080u, q[1][k] ^ 0x80808080u, 0x64806480u, f[k], a_row_sw, 2 * k + (c >> 1));
                     }
                 } else {
                     // the unit's power of two: its largest |d| to [64, 128)
@@ -1050,7 +1045,7 @@ int launch_dense(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand,
     const size_t units = w.cols / 256;
     CUtensorMap tw, tx;
     int rc;
-    // packed weights as bytes; rows past the end read as zeros (Q6_K's zero bytes are weights of -32 times a sub-scale of zero)
+    // packed weights as bytes; rows past the end read as zeros
     if ((rc = encode_2d(ctx, &tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, w.quants, w.qpitch, w.rows, w.qpitch, FMT == Q8_0 ? 128 : Q6_K_DEV, TILE_M,
                         FMT == Q8_0 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, "weight")))
         return rc;

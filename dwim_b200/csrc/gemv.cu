@@ -311,16 +311,12 @@ __device__ __forceinline__ void unit_q8_i8(const Lane &L, const I8Cols X, int ul
 
 // Q6_K.  One MMA of k = 16 per 16-weight scale group: lane c holds weights
 // 4c..4c+3 of the group as signed bytes; the group's i8 sub-scale weighs its
-// integer sums, d the unit's.  For (half, lh) the lane reads two ql words and
-// one qh word per row and makes the four groups k = 0..3 from them.  A weight's
-// six bits go to the top of its byte: flipping the uppermost makes them 4 * q
-// as a signed byte, no sign to spread; d takes the 4 back.  (Bound by issue:
-// 573 instructions a unit of 16 rows at one token with the sign spread, half of
-// them decode; the [151936, 5120] head at one token 199 us with its norm and
-// arg-max then, 170 now.)
-__device__ __forceinline__ uint32_t q6_bytes(uint32_t low, uint32_t high) {   // nibbles at bits 2-5, bit pairs at 6-7
-    return (low & 0x3c3c3c3cu) | ((high & 0xc0c0c0c0u) ^ 0x80808080u);
-}
+// integer sums, d the unit's.  A lane's share of a row is three 128-bit loads: word j of
+// the four sets of four groups, from which nine instructions a set make the groups' bytes,
+// 4 * q each (formats.cuh); d takes the 4 back.  (Bound by issue: with the file's nibbles and bit pairs, twelve
+// 32-bit loads and sixteen instructions, the [151936, 5120] product took 108 us at one token, 131 at two and 201 at
+// eight; 100, 118 and 194 like this.)
+__device__ __forceinline__ uint32_t word_of(const uint4 &v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 template <int NTILE, bool ONE>
 __device__ __forceinline__ void unit_q6k_i8(const Lane &L, const I8Cols X, int ul, int xu, int d_index, float (&acc)[NTILE == 2 ? 8 : 4]) {
     const uint32_t ba = L.row_a + ul * 208, bb = L.row_b + ul * 208;
@@ -334,34 +330,28 @@ __device__ __forceinline__ void unit_q6k_i8(const Lane &L, const I8Cols X, int u
     for (int p = 0; p < NTILE; p++)
 #pragma unroll
         for (int i = 0; i < 4; i++) is[p][i] = 0;
+    uint4 wa[3], wb[3];      // word j of the four sets of four groups
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        wa[j] = lds128(ba + 64 * j + 16 * L.c);
+        wb[j] = lds128(bb + 64 * j + 16 * L.c);
+    }
     if constexpr (ONE) {
         const uint32_t first = L.g < 4 ? 0xffffffffu : 0u, mine = 0x8880u + (uint32_t)(L.c >> 1) * 0x1111u;
         const uint32_t x0 = blob + (L.g & 3) * 32 + 16 * (L.g >> 2) + 4 * L.c;      // four columns: 128 bytes a sub-block
 #pragma unroll
-        for (int hf = 0; hf < 2; hf++) {
-            uint32_t la[2][2], lb[2][2], ha[2], hb[2];     // [lh][row of 32 weights]
+        for (int t = 0; t < 4; t++) {
+            uint32_t qa[4], qb[4];
+            q6k_bytes(word_of(wa[0], t), word_of(wa[1], t), word_of(wa[2], t), qa);
+            q6k_bytes(word_of(wb[0], t), word_of(wb[1], t), word_of(wb[2], t), qb);
 #pragma unroll
-            for (int lh = 0; lh < 2; lh++) {
-                const uint32_t o = 64 * hf + 16 * lh + 4 * L.c, oh = 128 + 32 * hf + 16 * lh + 4 * L.c;
-                la[lh][0] = lds32(ba + o); la[lh][1] = lds32(ba + o + 32); ha[lh] = lds32(ba + oh);
-                lb[lh][0] = lds32(bb + o); lb[lh][1] = lds32(bb + o + 32); hb[lh] = lds32(bb + oh);
-            }
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                uint32_t qa[2], qb[2];
-#pragma unroll
-                for (int lh = 0; lh < 2; lh++) {
-                    const uint32_t a = la[lh][k & 1], b = lb[lh][k & 1];
-                    qa[lh] = q6_bytes((k >> 1) ? a >> 2 : a << 2, ha[lh] << (6 - 2 * k));
-                    qb[lh] = q6_bytes((k >> 1) ? b >> 2 : b << 2, hb[lh] << (6 - 2 * k));
-                }
-                // the groups 8 hf + 2 k and + 1: this lane's results are of the one its columns belong to
-                const int word = 2 * hf + (k >> 1);
-                const int fa = (int)prmt(sca[word], 0u, mine + (2 * k & 3) * 0x1111u);
-                const int fb = (int)prmt(scb[word], 0u, mine + (2 * k & 3) * 0x1111u);
-                const uint32_t x = lds32(x0 + (4 * hf + k) * 128);
+            for (int k = 0; k < 2; k++) {
+                // the groups 4 t + 2 k and + 1: this lane's results are of the one its columns belong to
+                const int fa = (int)prmt(sca[t], 0u, mine + 2 * k * 0x1111u);
+                const int fb = (int)prmt(scb[t], 0u, mine + 2 * k * 0x1111u);
+                const uint32_t x = lds32(x0 + (2 * t + k) * 128);
                 int c[4];
-                imma_s8s8(c, qa[0], qb[0], qa[1], qb[1], x & first, x & ~first);
+                imma_s8s8(c, qa[2 * k], qb[2 * k], qa[2 * k + 1], qb[2 * k + 1], x & first, x & ~first);
                 is[0][0] += fa * c[0];
                 is[0][1] += fa * c[1];
                 is[0][2] += fb * c[2];
@@ -378,36 +368,30 @@ __device__ __forceinline__ void unit_q6k_i8(const Lane &L, const I8Cols X, int u
     const uint32_t xlane = blob + X.lane_col(L.g) * 32 + 4 * L.c;
     const uint32_t xstep = 32 * X.nc, tstep = 32 * X.tile_stride;
 #pragma unroll
-    for (int hf = 0; hf < 2; hf++)
+    for (int t = 0; t < 4; t++) {
+        uint32_t qa[4], qb[4];
+        q6k_bytes(word_of(wa[0], t), word_of(wa[1], t), word_of(wa[2], t), qa);
+        q6k_bytes(word_of(wb[0], t), word_of(wb[1], t), word_of(wb[2], t), qb);
 #pragma unroll
-        for (int lh = 0; lh < 2; lh++) {
-            const uint32_t o = 64 * hf + 16 * lh + 4 * L.c, oh = 128 + 32 * hf + 16 * lh + 4 * L.c;
-            const uint32_t la0 = lds32(ba + o), la1 = lds32(ba + o + 32), hha = lds32(ba + oh);
-            const uint32_t lb0 = lds32(bb + o), lb1 = lds32(bb + o + 32), hhb = lds32(bb + oh);
+        for (int k = 0; k < 4; k++) {
+            // byte k of the word, sign-extended (a selector nibble of 8 + b replicates byte b's sign)
+            constexpr uint32_t SEXT = 0x8880u;
+            const int fa = (int)prmt(sca[t], 0u, SEXT + k * 0x1111u);
+            const int fb = (int)prmt(scb[t], 0u, SEXT + k * 0x1111u);
+            // group 4 t + k: its half of the sub-block, digits 4c .. +3
+            const uint32_t xo = (2 * t + (k >> 1)) * xstep + 16 * (k & 1);
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const uint32_t la = (k & 1) ? la1 : la0, lb = (k & 1) ? lb1 : lb0;
-                const uint32_t qa = q6_bytes((k >> 1) ? la >> 2 : la << 2, hha << (6 - 2 * k));
-                const uint32_t qb = q6_bytes((k >> 1) ? lb >> 2 : lb << 2, hhb << (6 - 2 * k));
-                const int sidx = 8 * hf + 2 * k + lh;
-                // byte sidx & 3 of the word, sign-extended (a selector nibble of 8 + b replicates byte b's sign)
-                constexpr uint32_t SEXT = 0x8880u;
-                const int fa = (int)prmt(sca[sidx >> 2], 0u, SEXT + (sidx & 3) * 0x1111u);
-                const int fb = (int)prmt(scb[sidx >> 2], 0u, SEXT + (sidx & 3) * 0x1111u);
-                // sub-block 4*hf + k of the unit, digits 16*lh + 4c .. +3
-                const uint32_t xo = (4 * hf + k) * xstep + 16 * lh;
-#pragma unroll
-                for (int p = 0; p < NTILE; p++) {
-                    const uint32_t x = lds32(xlane + xo + p * tstep);
-                    int c[4];
-                    imma16_s8s8(c, qa, qb, x);
-                    is[p][0] += fa * c[0];
-                    is[p][1] += fa * c[1];
-                    is[p][2] += fb * c[2];
-                    is[p][3] += fb * c[3];
-                }
+            for (int p = 0; p < NTILE; p++) {
+                const uint32_t x = lds32(xlane + xo + p * tstep);
+                int c[4];
+                imma16_s8s8(c, qa[k], qb[k], x);
+                is[p][0] += fa * c[0];
+                is[p][1] += fa * c[1];
+                is[p][2] += fb * c[2];
+                is[p][3] += fb * c[3];
             }
         }
+    }
 #pragma unroll
     for (int p = 0; p < NTILE; p++)
 #pragma unroll
@@ -605,7 +589,7 @@ __global__ void __launch_bounds__((RT * KS + 1) * 32, 1) dwim_smallm_kernel(cons
     // of 16-byte steps apart, the four rows of a half-warp must be two steps
     // apart to cover all banks, so lanes g = 0..3 take rows 0, 2, 4, 6 of the
     // eight and g = 4..7 rows 1, 3, 5, 7.
-    const int grow = (FMT == Q4K_I8 || FMT == Q8_I8) ? ((L.g & 3) * 2 + (L.g >> 2)) : L.g;
+    const int grow = (FMT == Q4K_I8 || FMT == Q8_I8) ? ((L.g & 3) * 2 + (L.g >> 2)) : (L.g >> 1) + (L.g & 1) * 4;
     constexpr bool ONE = NT == 0, PACKED = NT <= 1;
     const I8Cols X = i8_cols<PACKED ? 1 : NT>(a.ncols, a.n_tokens);
 
