@@ -594,7 +594,7 @@ template <int FMT, int BN, int MODE> struct DenseCfg {
     static_assert(STEPS < 4 || (ACC_BUFS == 8 && BN == 64), "drain_unit");
     static_assert(ACC_BUFS == 2 * STEPS || STEPS == 2, "a unit of more steps than buffers would wait for itself");
     static constexpr int TMEM_COLS = ACC_BUFS * ACC_COLS > 256 ? 512 : 256;
-    static constexpr int B_STAGES = ACC_COLS > 128 ? 3 : 4, B_BYTES = TERM_BYTES * (WIDE ? 2 : 1);
+    static constexpr int B_STAGES = ACC_COLS > 192 ? 3 : 4, B_BYTES = TERM_BYTES * (WIDE ? 2 : 1);
     // raw weights: a unit of Q6_K, half a unit of Q8_0 (128 bytes a row, swizzled)
     static constexpr int RAW_STEPS = FMT == Q8_0 ? 2 : 1;           // ring stages per unit
     static constexpr int RAW_STAGES = FMT == Q8_0 ? 3 : 2, RAW_STAGE = FMT == Q8_0 ? TILE_M * 128 : TILE_M * Q6_K_DEV;
@@ -1039,6 +1039,20 @@ int launch_gemm(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, 
 }
 
 template <int FMT, int BN, int MODE>
+int dense_split(dwim_b200_ctx *ctx, const WeightView &w, size_t n, int terms, double *time = nullptr) {
+    using C = DenseCfg<FMT, BN, MODE>;
+    static std::atomic<int> known[64][MAX_SPLIT + 1] = {};
+    const long tiles = (long)((w.rows + TILE_M - 1) / TILE_M) * (long)((n + BN - 1) / BN);
+    return pick_split(ctx, gemm_dense_kernel<FMT, BN, MODE, false>, GEMM_THREADS, (size_t)C::SMEM, C::split_fits, SplitCost{2.0, 4.5}, known, tiles,
+                      (int)(w.cols / 256), terms == 1 ? 1.0 : 1.9, time);
+}
+template <int FMT, int BN, int MODE> double dense_time(dwim_b200_ctx *ctx, const WeightView &w, size_t n, int terms) {
+    double t = 0;
+    dense_split<FMT, BN, MODE>(ctx, w, n, terms, &t);
+    return t;
+}
+
+template <int FMT, int BN, int MODE>
 int launch_dense(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, size_t n, int terms, const OutSpec &out, const float *aux,
                  int epi) {
     using C = DenseCfg<FMT, BN, MODE>;
@@ -1060,9 +1074,7 @@ int launch_dense(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand,
     if ((rc = configure_gemm(ctx, kern, C::SMEM, GEMM_THREADS, 512 * DENSE_WORKER_REGS + 128 * DENSE_OTHER_REGS, configured[ctx->device & 63][shared]))) return rc;
     dim3 grid((unsigned)((w.rows + TILE_M - 1) / TILE_M), (unsigned)((n + BN - 1) / BN));
     if (!shared) {
-        static std::atomic<int> known[64][MAX_SPLIT + 1] = {};
-        a.split_k = pick_split(ctx, kern, GEMM_THREADS, (size_t)C::SMEM, C::split_fits, SplitCost{2.0, 4.5}, known, (long)grid.x * grid.y, (int)units,
-                               terms == 1 ? 1.0 : 1.9);
+        a.split_k = dense_split<FMT, BN, MODE>(ctx, w, n, terms);
         grid.x *= a.split_k;
     }
     const bool dependent = !ctx->weights_written;   // see dwim_b200_ctx::weights_written
@@ -1119,7 +1131,15 @@ int gemm_large(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, s
         if (n <= 64 || w.cols > 12288)
             return launch_dense<F, 64, TWO_PASSES>(ctx, w, operand, n, terms, out, aux, epilogue);
         if (n <= 128) return launch_dense<F, 128, SIDE_BY_SIDE>(ctx, w, operand, n, terms, out, aux, epilogue);
-        return (terms == 1 ? launch_dense<F, 256, ONE_TERM> : launch_dense<F, 256, TWO_PASSES>)(ctx, w, operand, n, terms, out, aux, epilogue);
+        // Tiles of 192 or 256 columns by their waves, as Q4_K's: [12288, 5120] Q6_K by 192 f32 tokens 128 us in tiles of 256,
+        // 100 of 192, by 384 206 and 165, by 256 129 and 166; [5120, 5120] Q8_0 by 130 52 and 40, by bf16 ones 31 and 29.
+        auto wide = [&](auto mode) {
+            constexpr int M = decltype(mode)::value;
+            if (0.82 * dense_time<F, 192, M>(ctx, w, n, terms) < dense_time<F, 256, M>(ctx, w, n, terms))
+                return launch_dense<F, 192, M>(ctx, w, operand, n, terms, out, aux, epilogue);
+            return launch_dense<F, 256, M>(ctx, w, operand, n, terms, out, aux, epilogue);
+        };
+        return terms == 1 ? wide(std::integral_constant<int, ONE_TERM>()) : wide(std::integral_constant<int, TWO_PASSES>());
     };
     return w.fmt == Q6_K ? dense(std::integral_constant<int, Q6_K>()) : dense(std::integral_constant<int, Q8_0>());
 }
