@@ -423,7 +423,7 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             const uint32_t raw_row = raw0 + rs * RAW_BYTES + rl * 144;
             const uint4 hdr = lds128(raw_row);
             Q4kBlock blk;
-            load_q4k_block(hdr, q4k_fold(hdr.x), raw_row, g, blk);
+            load_q4k_block(hdr, raw_row, g, blk);
             const int kb = KBLOCKS * u + g, stage = kb % C::A_STAGES;
             mbar_wait_parked(aempty0 + 8 * stage, ((kb / C::A_STAGES) & 1) ^ 1, a.status, 0x800u);   // the MMAs that read this stage are done
             store_q4k_block(blk, a_row_sw + stage * A_BYTES);
@@ -704,10 +704,23 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 #pragma unroll
             for (int g = 0; g < KBLOCKS; g++) {
                 const uint32_t acc = tm + buf * C::ACC_COLS;
-                if (g % DRAIN_KB == 0) mbar_wait_parked(accempty0 + 8 * buf, bufturn, a.status, 0x400000u);
-                mbar_wait_parked(afull0 + 8 * g, u & 1, a.status, 0x1000000u);
+                // What a K block needs: asked by lanes of the warp at once where its MMAs are so short that the 85 cycles
+                // of a test count ([5120, 5120] Q8_0 by 48 tokens 24.6 us one by one, 23.1 like this; wider tiles spill).
+                constexpr bool AT_ONCE = C::STEPS == 4;
+                if (!AT_ONCE) {
+                    if (g % DRAIN_KB == 0) mbar_wait_parked(accempty0 + 8 * buf, bufturn, a.status, 0x400000u);
+                    mbar_wait_parked(afull0 + 8 * g, u & 1, a.status, 0x1000000u);
+                }
+#pragma unroll AT_ONCE ? 2 : 1
                 for (int p = PASSES - 1; p >= 0; p--) {
-                    mbar_wait_parked(bfull0 + 8 * bs, bturn, a.status, 0x800000u);
+                    if (AT_ONCE) {
+                        uint32_t bar = bfull0 + 8 * bs, phase = bturn;
+                        if (p == PASSES - 1 && (lane & 1)) bar = afull0 + 8 * g, phase = u & 1;
+                        if (p == PASSES - 1 && (lane & 2)) bar = accempty0 + 8 * buf, phase = bufturn;
+                        mbar_wait_all(bar, phase, a.status, 0x800000u);
+                    } else {
+                        mbar_wait_parked(bfull0 + 8 * bs, bturn, a.status, 0x800000u);
+                    }
                     tc_fence_after();
                     if (elect_one()) {
                         // the weights' remainders first: they are too small for the accumulator's rounding to matter

@@ -149,11 +149,14 @@ struct Q4kFold {
     int e;        // the main operand is scaled by 2^-e
     bool zero;    // the main operand is dropped
 };
-__device__ __forceinline__ Q4kFold q4k_fold(uint32_t d_dmin, int more = 0) {
+template <bool CENTRED = false>
+__device__ __forceinline__ Q4kFold q4k_fold(uint32_t d_dmin) {
     const float d = h2f_lo(d_dmin), dmin = h2f_hi(d_dmin);
     const int ed = (int)((__float_as_uint(d) >> 23) & 0xffu), em = (int)((__float_as_uint(dmin) >> 23) & 0xffu);
     Q4kFold f;
-    f.e = max(0, em - ed - 4 + more);      // more: a smaller bound by so many powers of two
+    // (centred, and where d and dmin differ in sign, the minimums' two parts add up: twice the room)
+    if (CENTRED) f.e = max(0, em - ed - 4 + (int)((d_dmin ^ (d_dmin << 16)) >> 31));
+    else f.e = max(0, em - ed - 4);
     f.zero = d == 0.0f || f.e > 24;
     if (f.zero) f.e = 0;
     return f;
@@ -163,7 +166,7 @@ struct Q4kBlock {
     uint32_t words[8];                 // the 32 bytes of group g
     uint32_t mul[2], add[2];           // per nibble half: x*mul + add turns the magic-number halves into sc*q
 };
-__device__ __forceinline__ void load_q4k_block(const uint4 &hdr, const Q4kFold &f, uint32_t raw_row, int g, Q4kBlock &b) {
+__device__ __forceinline__ void load_q4k_block(const uint4 &hdr, uint32_t raw_row, int g, Q4kBlock &b) {
     const uint4 q0 = lds128(raw_row + 16 + 32 * g), q1 = lds128(raw_row + 32 + 32 * g);
     b.words[0] = q0.x; b.words[1] = q0.y; b.words[2] = q0.z; b.words[3] = q0.w;
     b.words[4] = q1.x; b.words[5] = q1.y; b.words[6] = q1.z; b.words[7] = q1.w;
@@ -171,6 +174,7 @@ __device__ __forceinline__ void load_q4k_block(const uint4 &hdr, const Q4kFold &
     const uint32_t y = (hdr.y >> sh) & 0xffffu, w = (hdr.w >> sh) & 0xffffu;
     const uint32_t sc2 = g < 2 ? (y & 0x3f3fu) : ((w & 0x0f0fu) | ((y >> 2) & 0x3030u));
     const uint32_t sa = sc2 & 0xffu, sb = sc2 >> 8;
+    const Q4kFold f = q4k_fold(hdr.x);      // (passed in instead, the 256-column form spills 96 bytes, 32 like this)
     // 2^-e as a half: normal down to 2^-14, subnormal below; zero drops the operand
     const uint32_t p1 = f.zero ? 0u : (f.e <= 14 ? (uint32_t)(15 - f.e) << 10 : 1u << (24 - f.e));
     const uint32_t p2 = p1 | (p1 << 16);

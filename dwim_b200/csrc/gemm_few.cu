@@ -91,8 +91,7 @@ struct FewScales {
     float by;                  // -32 * dmin / s
 };
 __device__ __forceinline__ FewScales few_scales(const uint4 &hdr) {
-    // (where d and dmin differ in sign the minimums' two parts add up: twice the room)
-    const Q4kFold f = q4k_fold(hdr.x, (hdr.x ^ (hdr.x << 16)) >> 31);
+    const Q4kFold f = q4k_fold<true>(hdr.x);
     const float dmin32 = 32.0f * h2f_hi(hdr.x);
     const float s = f.zero ? dmin32 : h2f_lo(hdr.x) * __uint_as_float((uint32_t)(127 + f.e) << 23);
     FewScales k;
