@@ -859,34 +859,45 @@ static int launch(dwim_b200_ctx *ctx, GemvArgs &a) {
 
 template <int FMT, int NT>
 static int launch_shape(dwim_b200_ctx *ctx, GemvArgs &a) {
-    // Row tiles per CTA (RT) x K-split warps per row tile (KS).  A CTA's tiles last rounds * (RT + 0.3)
-    // in times of 16 rows: every round has its reduction, epilogue and, where the planes travel with the
-    // stages, one load of all planes; wide tiles save rounds, narrow ones fill the last.  Measured, us,
-    // for RT = 1, 2, 3, 4: Q4_K by one token [17408, 5120] 17.8 15.7 17.1 15.5, [10240, 5120] 12.8 13.3
-    // 13.4 14.7, [5120, 6144] 9.7 10.4 9.2 10.0, [1024, 5120] 6.2 6.7 7.8 8.4; [5120, 17408] by five
-    // tokens 30.6 35.5 25.8 31.1; Q6_K [5120, 17408] by eight 42.9 46.3 34.2 45.5; the [151936, 5120] head
-    // by one 167 170 152 162, by eight 287 282 225 249.  Four is for Q4_K alone; Q8_0's
-    // whole rows, where they fit, by one or two tokens beat its boxes, two swizzled ones a unit, unless the boxes take a
-    // single round ([12288, 5120] 16.0 whole, 17.0 in boxes; [5120, 5120] 10.9 and 10.5; by eight 29.9 and
-    // 22.5, 18.1 and 12.9).  Rows beyond 65536 columns keep one row tile: the stage with the fewest units is the narrowest then.
+    // Row tiles per CTA (RT) x K-split warps per row tile (KS).  A CTA's tiles last rounds * (RT + c) in times of 16
+    // rows: every round has its reduction, epilogue and, where the planes travel with the stages, one load of all planes,
+    // which weigh the more the shorter the rows are; wide tiles save rounds, narrow ones fill the last.  c * cols was
+    // fitted to these and others, us for RT = 1, 2, 3, 4:
+    //   Q4_K, one token: [17408, 5120] 15.7 13.4 12.6 12.5, [10240, 5120] 11.1 10.4 8.8 10.2, [6144, 5120] 7.5 7.0 6.8
+    //   7.2, [5120, 6144] 7.3 7.9 7.2 8.3, [1024, 5120] 3.4 4.2 5.1 5.8, [5120, 17408] 15.7 19.5 14.6 16.7; five tokens
+    //   [17408, 5120] 22.5 19.2 18.6 18.4, [10240, 5120] 14.9 14.0 13.3 16.9, [5120, 17408] 24.6 24.0 16.8 21.5
+    //   Q6_K: the [151936, 5120] head by one 116 106 107 114, by five 232 168 173 156, by eight 230 209 197 180;
+    //   [12288, 5120] by one 12.3 12.1 11.4 13.2, by five 22.8 18.2 18.1 19.3
+    //   Q8_0: [17408, 2048] by one 12.6 9.5 9.4 8.8, by eight 16.5 11.8 13.8 11.9; [5120, 5120] by eight 14.3 14.7 10.3
+    // (with c = 0.3 throughout, [10240, 5120] took one row tile and [17408, 2048] whole rows of one).  Four K-split warps
+    // leave a thread more registers than five: Q4_K by one token with three row tiles [10240, 5120] 9.3 us with five,
+    // 8.8 with four, by five [5120, 6144] 10.8 and 9.5; two row tiles 20.1 and 19.2.  Q6_K and Q8_0 by three tokens and
+    // more are a percent better with five.  Q8_0 by one or two tokens: whole rows of one row tile, where those of two do
+    // not fit, beat its boxes, two swizzled ones a unit, unless the boxes take a single round ([12288, 5120] 13.0 and 14.0;
+    // [5120, 5120] 7.5 and 8.5 one product behind the other, but 10.1 and 9.4 with the conversion before each).
+    // Rows beyond 65536 columns keep one row tile: the stage with the fewest units is the narrowest then.
+    constexpr bool FEW = NT <= 1;
+    constexpr int MOST = FMT == Q4K_I8 || (FMT == Q6K_I8 && !FEW) ? 4 : 3;
+    constexpr int KS3 = FMT == Q4K_I8 || FEW ? 4 : 5, KS4 = FMT == Q4K_I8 ? 4 : 3;
     int rt = 1;
     if (a.w.cols <= 65536) {
-        const bool whole = FMT == Q8_I8 && NT == 1 && Smem<FMT, NT, 1, 8>::two_whole_fit(a);
+        const bool whole = FMT == Q8_I8 && FEW && Smem<FMT, NT, 1, 8>::two_whole_fit(a) && !Smem<FMT, NT, 2, 4>::two_whole_fit(a);
+        const double c = (FMT == Q4K_I8 ? 4300.0 : FMT == Q8_I8 ? 1900.0 : FEW ? 1540.0 : 2560.0) / (double)a.w.cols;
         double best = 0;
-        for (int t = 1; t <= (FMT == Q4K_I8 ? 4 : 3); t++) {
+        for (int t = 1; t <= MOST; t++) {
             const size_t tiles = (a.w.rows + 16 * t - 1) / (16 * t);
             const size_t rounds = (tiles + ctx->sm_count - 1) / ctx->sm_count;
-            const double cost = (double)rounds * (t + 0.3);
+            const double cost = (double)rounds * (t + c);
             if (t == 1 || (cost < best && !(whole && rounds > 1))) {
                 best = cost;
                 rt = t;
             }
         }
     }
-    if (rt == 2) return launch<FMT, NT, 2, 5>(ctx, a);
-    if (rt == 3) return launch<FMT, NT, 3, 5>(ctx, a);
-    if constexpr (FMT == Q4K_I8)
-        if (rt == 4) return launch<FMT, NT, 4, 4>(ctx, a);
+    if (rt == 2) return launch<FMT, NT, 2, 4>(ctx, a);
+    if (rt == 3) return launch<FMT, NT, 3, KS3>(ctx, a);
+    if constexpr (MOST == 4)
+        if (rt == 4) return launch<FMT, NT, 4, KS4>(ctx, a);
     return launch<FMT, NT, 1, 8>(ctx, a);
 }
 

@@ -207,7 +207,7 @@ def test_matmul_golden_cases(dev, fmt):
 
 @pytest.mark.parametrize("fmt", FORMATS)
 @pytest.mark.parametrize("rows,cols", [(2384, 1024), (2400, 5120), (7105, 768), (9500, 1280), (17, 6144), (2369, 6400), (65, 17408), (33, 30464),
-                                       (40, 70400), (7105, 5888)])
+                                       (40, 70400), (7105, 5888), (7200, 5120)])
 def test_small_m_row_tiles_and_boxes(dev, oracle, fmt, rows, cols):
     """One to four row tiles a CTA (ragged last tiles), whole rows and boxes of odd numbers of units (a last
     box that is part padding, part past the row), planes resident and travelling, up to a row too long for
