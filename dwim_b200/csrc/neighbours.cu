@@ -10,6 +10,7 @@
 //   - argmax over the vocabulary's logits on the device, instead of reading
 //     608 KB back per drafted token and scanning them on the host
 //     (inference/qwen35/mod.rs:702-710, 1066-1068).
+#include <atomic>
 #include <new>
 
 #include "common.cuh"
@@ -123,98 +124,122 @@ __global__ void __launch_bounds__(256) matmul_bf16_kernel(const __grid_constant_
     }
 }
 
-// More tokens: tiles of 32 rows by 32 or 64 tokens, K dealt to the eight blocks of a
+// More tokens: tiles of 32 rows by 32 tokens, K dealt to the eight blocks of a
 // cluster (the gate matrices have three row tiles: 512 tokens would otherwise
-// be 24 blocks), whose partial tiles are summed in rank order out of each
-// other's shared memory.  A thread keeps 4 x 2 or 4 x 4 sums as packed pairs over even
-// and odd k (fma.rn.f32x2), both operands from shared memory in f32, four k a
-// load; the next 64 of K wait in registers meanwhile.  (A warp per row and
-// eight tokens took 306 us for [96, 5120] by 512 tokens.)
-constexpr int BT_ROWS = 32, BT_K = 64, BT_PITCH = BT_K + 4, BT_SPLIT = 8;
+// be 48 blocks) and each chunk of it to a block's two groups of 128 threads, whose partial
+// tiles are summed in a fixed order, the blocks' out of each other's shared memory.  A thread
+// keeps 4 x 2 sums as packed pairs over even and odd k (fma.rn.f32x2), four k a load.  Bound
+// by the blocks' arithmetic and loads with few warps on an SM to hide either: chunks of 64 k
+// come by cp.async into a ring of four, weights as bf16.  [96, 5120] by 32, 64, 128, 256 and 512
+// tokens 10.6, 10.6, 16, 22 and 24 us; 14, 14, 18, 33 and 41 with one chunk ahead in registers, one
+// group and two barriers a chunk; 10.7, 16, 18, 18 and 33 with four groups; 15, 15, 23, 26 and 27 in
+// tiles of 64 tokens.  (A warp per row and eight tokens took 306 us by 512.)
+constexpr int BT_ROWS = 32, BT_TOK = 32, BT_K = 64, BT_PITCH = BT_K + 4, BT_WPITCH = BT_K + 8, BT_SPLIT = 8, BT_STAGES = 4, BT_GROUPS = 2, BT_THREADS = 128 * BT_GROUPS;
+constexpr int BT_X = BT_TOK * BT_PITCH * 4, BT_W = BT_ROWS * BT_WPITCH * 2, BT_SMEM = BT_STAGES * (BT_X + BT_W);      // a stage's bytes; all
+static_assert(BT_GROUPS * BT_ROWS * BT_TOK * 4 <= BT_STAGES * BT_X, "the partial tiles take the activations' place");
 __device__ __forceinline__ void ffma2_n(uint64_t &d, uint64_t a, uint64_t b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
-template <int BT_TOK>
-__global__ void __cluster_dims__(BT_SPLIT, 1, 1) __launch_bounds__(128) matmul_bf16_tile_kernel(const __grid_constant__ Bf16Args a) {
+// 16 bytes into shared memory, zeros where `there` is false (the address is not read then)
+__device__ __forceinline__ void copy16(uint32_t dst, const void *src, bool there) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(there ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ uint64_t bf16_pair(uint32_t w) { return (uint64_t)(w << 16) | (uint64_t)(w & 0xffff0000u) << 32; }
+__global__ void __cluster_dims__(BT_SPLIT, 1, 1) __launch_bounds__(BT_THREADS) matmul_bf16_tile_kernel(const __grid_constant__ Bf16Args a) {
     griddep_launch();
     griddep_wait();
-    __shared__ __align__(16) float xs[BT_TOK * BT_PITCH];
-    __shared__ __align__(16) float ws[BT_ROWS * BT_PITCH];
-    static_assert(BT_ROWS * BT_TOK <= BT_TOK * BT_PITCH, "the partial tile takes the activations' place");
+    extern __shared__ __align__(16) uint8_t bt_smem[];
+    float *const xs0 = reinterpret_cast<float *>(bt_smem);
+    const uint8_t *const ws0 = bt_smem + BT_STAGES * BT_X;
+    const uint32_t xa = smem_u32(bt_smem), wa = xa + BT_STAGES * BT_X;
     const int tid = threadIdx.x, rank = blockIdx.x % BT_SPLIT;
     const size_t r0 = (size_t)(blockIdx.x / BT_SPLIT) * BT_ROWS, t0 = (size_t)blockIdx.y * BT_TOK;
     const size_t chunks = (a.cols + BT_K - 1) / BT_K;
-    const size_t c0 = chunks * rank / BT_SPLIT, c1 = chunks * (rank + 1) / BT_SPLIT;
-    const int rg = tid & 7, tg = tid >> 3;      // rows rg + 8 i, tokens tg + 16 j
+    const size_t c0 = chunks * rank / BT_SPLIT;
+    const int n_chunks = (int)(chunks * (rank + 1) / BT_SPLIT - c0);
+    const int rg = tid & 7, tg = (tid >> 3) & 15, kg = tid >> 7;      // rows rg + 8 i, tokens tg + 16 j, quarter kg of a chunk
     constexpr int TJ = BT_TOK / 16;
     uint64_t acc[4][TJ];
 #pragma unroll
     for (int i = 0; i < 4; i++)
 #pragma unroll
         for (int j = 0; j < TJ; j++) acc[i][j] = 0ull;
-    float4 xv[BT_TOK / 8];
-    uint4 wv[2];
     // a chunk's activations: rows of sixteen float4; its weights: 32 rows of eight 16-byte groups
-    auto fetch = [&](size_t c) {
-        const size_t k0 = c * BT_K;
+    auto fetch = [&](int c) {
+        const int s = c % BT_STAGES;
+        const size_t k0 = (c0 + c) * BT_K;
 #pragma unroll
-        for (int i = 0; i < BT_TOK / 8; i++) {
-            const size_t t = t0 + (size_t)(tid >> 4) + 8 * i, k = k0 + (size_t)(tid & 15) * 4;
-            xv[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (t < a.n && k < a.cols) xv[i] = *reinterpret_cast<const float4 *>(a.x + t * a.cols + k);
+        for (int i = 0; i < BT_TOK * 16 / BT_THREADS; i++) {
+            const int row = (tid >> 4) + BT_THREADS / 16 * i;
+            const size_t t = t0 + row, k = k0 + (size_t)(tid & 15) * 4;
+            const bool there = t < a.n && k < a.cols;
+            copy16(xa + s * BT_X + (row * BT_PITCH + (tid & 15) * 4) * 4, there ? a.x + t * a.cols + k : a.x, there);
         }
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const size_t r = r0 + (size_t)(tid >> 3) + 16 * i, k = k0 + (size_t)(tid & 7) * 8;
-            wv[i] = make_uint4(0, 0, 0, 0);
-            if (r < a.rows && k < a.cols) wv[i] = *reinterpret_cast<const uint4 *>(a.w + r * a.cols + k);
+        if (tid < BT_ROWS * 8) {
+            const int row = tid >> 3;
+            const size_t r = r0 + row, k = k0 + (size_t)(tid & 7) * 8;
+            const bool there = r < a.rows && k < a.cols;
+            copy16(wa + s * BT_W + (row * BT_WPITCH + (tid & 7) * 8) * 2, there ? a.w + r * a.cols + k : a.w, there);
         }
     };
-    if (c0 < c1) fetch(c0);
-    for (size_t c = c0; c < c1; c++) {
-        __syncthreads();      // the chunk before has been read
 #pragma unroll
-        for (int i = 0; i < BT_TOK / 8; i++) *reinterpret_cast<float4 *>(xs + ((tid >> 4) + 8 * i) * BT_PITCH + (tid & 15) * 4) = xv[i];
+    for (int c = 0; c < BT_STAGES - 1; c++) {
+        if (c < n_chunks) fetch(c);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int c = 0; c < n_chunks; c++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(BT_STAGES - 2) : "memory");      // this thread's part of chunk c is there
+        __syncthreads();                                                             // everyone's is, and chunk c - 1 has been read
+        if (c + BT_STAGES - 1 < n_chunks) fetch(c + BT_STAGES - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float *xs = xs0 + c % BT_STAGES * (BT_X / 4);
+        const uint8_t *ws = ws0 + c % BT_STAGES * BT_W;
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
-            float *d = ws + ((tid >> 3) + 16 * i) * BT_PITCH + (tid & 7) * 8;
-            *reinterpret_cast<float4 *>(d) = make_float4(bf16_lo(wv[i].x), bf16_hi(wv[i].x), bf16_lo(wv[i].y), bf16_hi(wv[i].y));
-            *reinterpret_cast<float4 *>(d + 4) = make_float4(bf16_lo(wv[i].z), bf16_hi(wv[i].z), bf16_lo(wv[i].w), bf16_hi(wv[i].w));
-        }
-        __syncthreads();
-        if (c + 1 < c1) fetch(c + 1);
-#pragma unroll 4
-        for (int k = 0; k < BT_K; k += 4) {
-            ulonglong2 wq[4], xq[TJ];
+        for (int i4 = 0; i4 < BT_K / BT_GROUPS / 4; i4++) {
+            const int k = kg * (BT_K / BT_GROUPS) + 4 * i4;
+            uint2 wq[4];
+            ulonglong2 xq[TJ];
 #pragma unroll
-            for (int i = 0; i < 4; i++) wq[i] = *reinterpret_cast<const ulonglong2 *>(ws + (rg + 8 * i) * BT_PITCH + k);
+            for (int i = 0; i < 4; i++) wq[i] = *reinterpret_cast<const uint2 *>(ws + ((rg + 8 * i) * BT_WPITCH + k) * 2);
 #pragma unroll
             for (int j = 0; j < TJ; j++) xq[j] = *reinterpret_cast<const ulonglong2 *>(xs + (tg + 16 * j) * BT_PITCH + k);
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < 4; i++) {
+                const uint64_t w01 = bf16_pair(wq[i].x), w23 = bf16_pair(wq[i].y);
 #pragma unroll
                 for (int j = 0; j < TJ; j++) {
-                    ffma2_n(acc[i][j], wq[i].x, xq[j].x);
-                    ffma2_n(acc[i][j], wq[i].y, xq[j].y);
+                    ffma2_n(acc[i][j], w01, xq[j].x);
+                    ffma2_n(acc[i][j], w23, xq[j].y);
                 }
+            }
         }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    // the partial tile [token][row] in the activations' place
+    // the groups' partial tiles [token][row] in the activations' place, their sum in the first's
+    float *const part = xs0;
+    constexpr int TILE = BT_TOK * BT_ROWS;
 #pragma unroll
     for (int i = 0; i < 4; i++)
 #pragma unroll
         for (int j = 0; j < TJ; j++)
-            xs[(tg + 16 * j) * BT_ROWS + rg + 8 * i] = __uint_as_float((uint32_t)acc[i][j]) + __uint_as_float((uint32_t)(acc[i][j] >> 32));
-    cluster_sync();
-    // this rank's share of the tile: a warp its tokens, a lane a row
-    const uint32_t mine = smem_u32(xs);
+            part[kg * TILE + (tg + 16 * j) * BT_ROWS + rg + 8 * i] = __uint_as_float((uint32_t)acc[i][j]) + __uint_as_float((uint32_t)(acc[i][j] >> 32));
+    __syncthreads();
 #pragma unroll
-    for (int i = 0; i < BT_TOK / BT_SPLIT / 4; i++) {
-        const int t = rank * (BT_TOK / BT_SPLIT) + (tid >> 5) * (BT_TOK / BT_SPLIT / 4) + i, r = tid & 31;
+    for (int i = tid; i < TILE; i += BT_THREADS) {
+        float v = part[i];
+#pragma unroll
+        for (int g = 1; g < BT_GROUPS; g++) v += part[g * TILE + i];
+        part[i] = v;
+    }
+    cluster_sync();
+    // this rank's share of the tile: a warp a token, a lane a row
+    static_assert(BT_TOK / BT_SPLIT <= BT_THREADS / 32, "a warp a token");
+    const int t = rank * (BT_TOK / BT_SPLIT) + (tid >> 5), r = tid & 31;
+    if (tid >> 5 < BT_TOK / BT_SPLIT) {
         float v = 0.0f;
 #pragma unroll
-        for (int p = 0; p < BT_SPLIT; p++) v += ld_cluster_f32(mine + (t * BT_ROWS + r) * 4, p);
+        for (int p = 0; p < BT_SPLIT; p++) v += ld_cluster_f32(xa + (t * BT_ROWS + r) * 4, p);
         if (t0 + t < a.n && r0 + r < a.rows) bf16_emit(a, t0 + t, r0 + r, v);
     }
     cluster_sync();      // a block's shared memory is read until here
@@ -273,11 +298,13 @@ int matmul_bf16(dwim_b200_ctx *ctx, const WeightView &w, const float *x, size_t 
     // counts whose activations are small beside a launch; the other wants whole tiles of tokens.
     const bool dependent = !ctx->weights_written;
     if (n > (size_t)BF16_FEW) {
-        // narrow token tiles while there are few of them: 14 us against 19 for [96, 5120] by 64 tokens, 56 against 39 by 512
-        const size_t tok = n <= 128 ? 32 : 64;
-        auto kern = tok == 32 ? matmul_bf16_tile_kernel<32> : matmul_bf16_tile_kernel<64>;
-        const dim3 grid((unsigned)((w.rows + BT_ROWS - 1) / BT_ROWS * BT_SPLIT), (unsigned)((n + tok - 1) / tok));
-        DWIM_CUDA(ctx, launch_dependent(dependent, kern, grid, dim3(128), 0, ctx->stream, a));
+        static std::atomic<bool> configured[64] = {};
+        if (!configured[ctx->device & 63]) {
+            DWIM_CUDA(ctx, cudaFuncSetAttribute(matmul_bf16_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_SMEM));
+            configured[ctx->device & 63] = true;
+        }
+        const dim3 grid((unsigned)((w.rows + BT_ROWS - 1) / BT_ROWS * BT_SPLIT), (unsigned)((n + BT_TOK - 1) / BT_TOK));
+        DWIM_CUDA(ctx, launch_dependent(dependent, matmul_bf16_tile_kernel, grid, dim3(BT_THREADS), (size_t)BT_SMEM, ctx->stream, a));
     } else {
         auto kern = n == 1 ? matmul_bf16_kernel<1> : n == 2 ? matmul_bf16_kernel<2> : n <= 4 ? matmul_bf16_kernel<4> : matmul_bf16_kernel<8>;
         const dim3 grid((unsigned)w.rows, (unsigned)((n + 7) / 8));
