@@ -86,6 +86,9 @@ template <int BN, int MODE> struct Cfg {
     static constexpr int RAW_STAGES = BN == 32 ? 3 : 2;
     static constexpr int MIN_STAGES = BN > 128 ? 1 : 2;
     static constexpr bool WIDE = MODE == SIDE_BY_SIDE;
+    // Whether the warpgroups trade registers: at 192 columns and less 96 are enough ([2090, 16896] by 571 bf16 tokens 57.0 us
+    // with the trade, 55.1 without).
+    static constexpr bool TRADE = BN > 192;
     static constexpr int TERM_BYTES = BN * BK * 2, B_BYTES = TERM_BYTES * (WIDE ? 2 : 1), ACC_COLS = BN * (WIDE ? 2 : 1);
     static constexpr int BMIN_BYTES = BN * 16 * 2;                 // [K group of 8][column][16 B]: the means' hi and lo parts
     static constexpr int MIN_BYTES = AMIN_BYTES + ((BMIN_BYTES + 1023) / 1024) * 1024;
@@ -206,6 +209,7 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     // One pass over a unit's K blocks: a K block's A and B stages are handed over and released together.
     constexpr int PASSES = MODE == TWO_PASSES ? 2 : 1;
     constexpr bool JOINT = PASSES == 1;
+    constexpr bool TRADE = C::TRADE;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;   // the swizzled tiles want 1024-byte alignment
     // barriers, 8 bytes each
@@ -260,7 +264,7 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     griddep_launch();
 
     if (warp == X_WARP) {
-        regs_dec<OTHER_REGS>();
+        if constexpr (TRADE) regs_dec<OTHER_REGS>();
         // ------------------------------ TMA producer ------------------------------
         griddep_wait();   // the operand comes from the prologue kernel just ahead
         if (elect_one()) {
@@ -298,7 +302,7 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             }
         }
     } else if (warp == RAW_WARP) {
-        regs_dec<OTHER_REGS>();
+        if constexpr (TRADE) regs_dec<OTHER_REGS>();
         // ------------------------------ packed weights' producer ------------------------------
         // Its own warp: the blocks come from HBM and must run as far ahead as the
         // ring allows, whatever the activations' producer is waiting for.
@@ -311,7 +315,7 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             }
         }
     } else if (warp == MMA_WARP) {
-        regs_dec<OTHER_REGS>();
+        if constexpr (TRADE) regs_dec<OTHER_REGS>();
         // ------------------------------ MMA issuer ------------------------------
         // The whole warp runs the loop (uniform control flow keeps addresses
         // and descriptors on the uniform data path) and one lane issues.  Units
@@ -374,7 +378,7 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             }
         }
     } else if (warp < N_WORKERS) {
-        regs_inc<WORKER_REGS>();
+        if constexpr (TRADE) regs_inc<WORKER_REGS>();
         // ------------------------------ workers ------------------------------
         // Warp w owns TMEM lane quadrant w % 4 (weight rows 32*(w % 4) + lane)
         // and K block g = w / 4 of every unit: it decodes that block of
@@ -541,7 +545,7 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             cluster_sync();
         }
     }
-    if (warp > RAW_WARP) regs_dec<OTHER_REGS>();      // (the warpgroup takes part as a whole)
+    if constexpr (TRADE) { if (warp > RAW_WARP) regs_dec<OTHER_REGS>(); }      // (the warpgroup takes part as a whole)
     if (warp >= N_WORKERS) {
         __syncwarp();
         if (split_k > 1) {      // the workers' two meetings are the whole cluster's
@@ -1035,7 +1039,7 @@ int launch_gemm(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, 
         if (shared == 1) kern = gemm_q4k_kernel<BN, 1, MODE>;
     }
     static std::atomic<bool> configured[64][3] = {};
-    if ((rc = configure_gemm(ctx, kern, C::SMEM, GEMM_THREADS, 512 * WORKER_REGS + 128 * OTHER_REGS, configured[ctx->device & 63][shared]))) return rc;
+    if ((rc = configure_gemm(ctx, kern, C::SMEM, GEMM_THREADS, C::TRADE ? 512 * WORKER_REGS + 128 * OTHER_REGS : 0, configured[ctx->device & 63][shared]))) return rc;
     dim3 grid((unsigned)((w.rows + TILE_M - 1) / TILE_M), (unsigned)((n + BN - 1) / BN));
     if constexpr (ONE) {
         if (!shared) {
