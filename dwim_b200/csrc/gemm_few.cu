@@ -21,8 +21,8 @@
 //   warp 23      packed weights' producer
 // All rings are dealt to the groups in turn (stage % 4), so that a group waits for phases of its own alone: of a
 // barrier that others' phases pass it could miss two, and take an old one for the one it waits for.
-// Bound by instruction issue (about 1100 a worker and unit, 410 of them on the ALU pipe; DRAM at 40 %).  [17408, 5120] by
-// 16 f32 tokens 24.2 us in gemm.cu's kernel, 18.4 here (31.7 with one MMA warp), by 32 25.5 and 23.0; [5120, 17408] by 16
+// Bound by the workers' chain and issue (1053 instructions a worker and unit; issue slots 61 %, ALU 39 %, DRAM 2.8 TB/s).
+// [17408, 5120] by 16 f32 tokens 24.2 us in gemm.cu's kernel, 18.4 here (31.7 with one MMA warp), by 32 25.5 and 23.0; [5120, 17408] by 16
 // 28.6 and 20.7; a layer of 16 tokens 156 and 122.
 // Every mbarrier wait is bounded (ptx.cuh).
 #include "gemm.cuh"
