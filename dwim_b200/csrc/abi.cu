@@ -36,6 +36,41 @@ int reserve_shadow(dwim_b200_ctx *ctx, dwim_b200_buffer *b, size_t need) {
     b->shadow_cap = need;
     return 0;
 }
+
+// The capture that the context's stream is under (an id that no other has), 0 when it is under none.
+static unsigned long long capture_id(dwim_b200_ctx *ctx) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (cudaStreamGetCaptureInfo(ctx->stream, &status, &id) != cudaSuccess) {
+        cudaGetLastError();
+        return ~0ull;
+    }
+    return status == cudaStreamCaptureStatusNone ? 0 : status == cudaStreamCaptureStatusActive ? id : ~0ull;
+}
+
+// A conversion that was recorded under a capture is made when its graph runs, so it is there for the rest of that
+// capture alone; one that was launched is there until a graph that makes another form runs, which nothing says.
+bool shadow_holds(dwim_b200_ctx *ctx, const dwim_b200_buffer *b, int kind, size_t cols, int split) {
+    if (b->shadow_kind != kind || b->shadow_cols != cols || b->shadow_split != split) return false;
+    const unsigned long long id = capture_id(ctx);
+    if (id != b->shadow_capture || id == ~0ull) return false;
+    const ShadowForm &r = b->replayed;
+    return id != 0 || r.kind == SHADOW_NONE || (r.kind == kind && r.cols == cols && r.split == split && r.len == b->len);
+}
+void shadow_made(dwim_b200_ctx *ctx, dwim_b200_buffer *b, int kind, size_t cols, int split) {
+    b->shadow_kind = kind;
+    b->shadow_cols = cols;
+    b->shadow_split = split;
+    b->shadow_capture = capture_id(ctx);
+    if (b->shadow_capture == 0) return;
+    ShadowForm &r = b->replayed;
+    const bool first = r.kind == SHADOW_NONE && kind != SHADOW_NONE;
+    if (!first && (r.kind != kind || r.cols != cols || r.split != split || r.len != b->len)) kind = SHADOW_MIXED;
+    r.kind = kind;
+    r.cols = cols;
+    r.split = split;
+    r.len = b->len;
+}
 }  // namespace dwim
 
 extern "C" {
@@ -457,7 +492,7 @@ int dwim_b200_quantize(dwim_b200_ctx *ctx, int fmt, size_t rows, size_t cols, co
 // Makes sure `x` has a shadow of the given kind for K = cols, (re)building it
 // if the buffer was written since.
 static int ensure_shadow(dwim_b200_ctx *ctx, dwim_b200_buffer *x, int kind, size_t cols, int split) {
-    if (x->shadow_kind == kind && x->shadow_cols == cols && x->shadow_split == split) return 0;
+    if (shadow_holds(ctx, x, kind, cols, split)) return 0;
     size_t n = x->len / cols;
     size_t need = kind == SHADOW_GEMM ? gemm_operand_bytes(cols, n, split) : panel_i8_bytes(cols, n);
     int rc = reserve_shadow(ctx, x, need);
@@ -466,20 +501,11 @@ static int ensure_shadow(dwim_b200_ctx *ctx, dwim_b200_buffer *x, int kind, size
     rc = kind == SHADOW_GEMM ? build_gemm_operand(ctx, x->data, n, cols, split, (__half *)x->shadow)
                              : build_panels_i8(ctx, x->data, n, cols, (uint8_t *)x->shadow);
     if (rc) return rc;
-    x->shadow_kind = kind;
-    x->shadow_cols = cols;
-    x->shadow_split = split;
+    shadow_made(ctx, x, kind, cols, split);
     return 0;
 }
 
 constexpr size_t GROUPS_AT_ONCE = 64;
-
-static bool capturing(dwim_b200_ctx *ctx) {
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(ctx->stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) return false;
-    cudaGetLastError();
-    return true;
-}
 
 // Room for products of Q6_K and Q8_0 by nine tokens and more: the digit planes of all the groups of eight tokens that
 // `x` can hold, up to GROUPS_AT_ONCE, or its operand for the dense kernel, in one array.  It spares launches or time and
@@ -488,7 +514,7 @@ static bool capturing(dwim_b200_ctx *ctx) {
 static void reserve_groups(dwim_b200_ctx *ctx, dwim_b200_buffer *x, size_t cols, size_t group) {
     size_t most = x->cap / cols / I8_MAX_TOKENS;
     if (most > GROUPS_AT_ONCE) most = GROUPS_AT_ONCE;
-    if (x->groups_tried || most < 2 || capturing(ctx)) return;
+    if (x->groups_tried || most < 2 || capture_id(ctx)) return;
     // the dense kernel's: of all the tokens where it takes any number in this way, else of its tile's
     size_t tokens = x->cap / cols;
     if (tokens > 64 && cols <= 12288) tokens = 64;
@@ -512,11 +538,11 @@ static int operand_apart(dwim_b200_ctx *ctx, dwim_b200_buffer *x, size_t cols, s
     const size_t need = gemm_operand_bytes(cols, n, split);
     *operand = nullptr;
     const bool fits = need <= x->shadow_cap;
-    const int kind = x->shadow_kind;
-    if ((kind == SHADOW_GEMM || kind == SHADOW_GEMM_APART) && x->shadow_cols == cols && x->shadow_split == split && !capturing(ctx)) {
-        *operand = (const __half *)(kind == SHADOW_GEMM ? x->shadow : x->groups);
-        return 0;
-    }
+    for (int kind : {SHADOW_GEMM, SHADOW_GEMM_APART})
+        if (shadow_holds(ctx, x, kind, cols, split)) {
+            *operand = (const __half *)(kind == SHADOW_GEMM ? x->shadow : x->groups);
+            return 0;
+        }
     if (!fits) {
         reserve_groups(ctx, x, cols, panel_i8_bytes(cols, I8_MAX_TOKENS));
         if (need > x->groups_cap) return 0;
@@ -525,9 +551,7 @@ static int operand_apart(dwim_b200_ctx *ctx, dwim_b200_buffer *x, size_t cols, s
     x->shadow_kind = SHADOW_NONE;
     int rc = build_gemm_operand(ctx, x->data, n, cols, split, (__half *)place);
     if (rc) return rc;
-    x->shadow_kind = fits ? SHADOW_GEMM : SHADOW_GEMM_APART;
-    x->shadow_cols = cols;
-    x->shadow_split = split;
+    shadow_made(ctx, x, fits ? SHADOW_GEMM : SHADOW_GEMM_APART, cols, split);
     *operand = (const __half *)place;
     return 0;
 }
@@ -579,7 +603,8 @@ static int product(dwim_b200_ctx *ctx, const OutSpec &out, size_t out_len, const
         if (groups > room) groups = room;
     }
     uint8_t *const panels = (uint8_t *)(groups * group > x->shadow_cap ? x->groups : x->shadow);
-    if (panels == x->shadow || x->shadow_kind == SHADOW_GEMM_APART) x->shadow_kind = SHADOW_NONE;
+    if (panels == x->shadow || x->shadow_kind == SHADOW_GEMM_APART) shadow_made(ctx, x, SHADOW_NONE, 0, 0);
+    else if (capture_id(ctx)) x->replayed.kind = SHADOW_MIXED;
     for (size_t t0 = 0; t0 < n;) {
         const size_t left = n - t0, g = left < (size_t)I8_MAX_TOKENS ? 1 : left / I8_MAX_TOKENS < groups ? left / I8_MAX_TOKENS : groups;
         const size_t nt = left < (size_t)I8_MAX_TOKENS ? left : (size_t)I8_MAX_TOKENS;

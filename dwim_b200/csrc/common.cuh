@@ -20,6 +20,13 @@ enum ShadowKind : int {
     SHADOW_GEMM_APART       // as SHADOW_GEMM, in the groups' array
 };
 
+// What graphs make of a buffer: nothing, one form of its contents, or several (SHADOW_MIXED).
+constexpr int SHADOW_MIXED = -1;
+struct ShadowForm {
+    int kind = SHADOW_NONE, split = 0;
+    size_t cols = 0, len = 0;
+};
+
 constexpr int DWIM_MAX_WORLD = 8;
 
 struct dwim_b200_buffer {
@@ -40,7 +47,9 @@ struct dwim_b200_buffer {
     size_t shadow_cap = 0;       // bytes
     int shadow_kind = SHADOW_NONE;
     size_t shadow_cols = 0;      // K the shadow was built for
-    int shadow_split = 0;        // 1: hi/lo column pairs, 0: single f16
+    int shadow_split = 0;        // f16 terms of an activation less one
+    unsigned long long shadow_capture = 0;   // the stream capture that the conversion is part of; 0: it was launched
+    ShadowForm replayed;         // what captured graphs make there whenever they run
     // The digit planes of several groups of eight tokens, or the dense kernel's operand (products of Q6_K and Q8_0 by
     // nine tokens and more), where the shadow holds less.  Allocated once and kept to the buffer's end.
     void *groups = nullptr;
@@ -214,6 +223,10 @@ void shared_release(dwim_b200_buffer *buf);
 // abi.cu
 // The buffer's shadow made at least `need` bytes long (a longer one takes the place of the old).
 int reserve_shadow(dwim_b200_ctx *ctx, dwim_b200_buffer *b, size_t need);
+// Whether that form of the buffer's contents is there for the next launch on the stream; and that it is now
+// (SHADOW_NONE: that something else is).
+bool shadow_holds(dwim_b200_ctx *ctx, const dwim_b200_buffer *b, int kind, size_t cols, int split);
+void shadow_made(dwim_b200_ctx *ctx, dwim_b200_buffer *b, int kind, size_t cols, int split);
 // neighbours.cu
 int matmul_bf16(dwim_b200_ctx *ctx, const WeightView &w, const float *x, size_t n, const OutSpec &out, const float *aux, int epi);
 // static_scratch.cu

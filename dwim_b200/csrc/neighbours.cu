@@ -337,9 +337,7 @@ extern "C" int dwim_b200_normalize(dwim_b200_ctx *ctx, dwim_b200_buffer *out, co
         if (rc) return rc;
         rc = build_gemm_operand(ctx, x->data, n, dim, split, (__half *)out->shadow, weight->data, eps, out->data);
         if (rc) return rc;
-        out->shadow_kind = SHADOW_GEMM;
-        out->shadow_cols = dim;
-        out->shadow_split = split;
+        shadow_made(ctx, out, SHADOW_GEMM, dim, split);
         return 0;
     }
     if (dim % 256 == 0 && n <= (size_t)I8_MAX_TOKENS) {
@@ -348,9 +346,7 @@ extern "C" int dwim_b200_normalize(dwim_b200_ctx *ctx, dwim_b200_buffer *out, co
         if (rc) return rc;
         rc = build_panels_i8(ctx, x->data, n, dim, (uint8_t *)out->shadow, weight->data, eps, out->data);
         if (rc) return rc;
-        out->shadow_kind = SHADOW_PANEL_I8;
-        out->shadow_cols = dim;
-        out->shadow_split = 0;
+        shadow_made(ctx, out, SHADOW_PANEL_I8, dim, 0);
         return 0;
     }
     DWIM_CUDA(ctx, launch_dependent(!ctx->weights_written, rmsnorm_rows_kernel, dim3((unsigned)n), dim3(256), 0, ctx->stream,

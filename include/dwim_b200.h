@@ -124,9 +124,12 @@ DWIM_B200_API int dwim_b200_resize(dwim_b200_ctx *ctx, dwim_b200_buffer *buf, si
  * which the reference invalidates in its own write paths, :313-384).  This
  * library drops the cache whenever one of its own calls writes the buffer; a
  * write it cannot see (a kernel of the caller's through dwim_b200_buffer_ptr, a
- * collective into a wrapped buffer) must be followed by touch before the next
- * product reads the buffer, or that product multiplies the old contents.  It
- * also forgets that the contents were exact in 16 bits (write_bf16). */
+ * collective into a wrapped buffer, a captured graph's run for the buffers that
+ * its calls write) must be followed by touch before the next product reads the
+ * buffer, or that product multiplies the old contents.  (A captured product
+ * converts its input within its graph; what graphs do to the cached form of a
+ * buffer they only read is accounted for.)  It also forgets that the contents
+ * were exact in 16 bits (write_bf16). */
 DWIM_B200_API int dwim_b200_touch(dwim_b200_ctx *ctx, dwim_b200_buffer *buf);
 /* The same, where the caller vouches that every value it wrote is exactly a
  * bf16 (the output of a bf16 kernel widened to f32): the next product then

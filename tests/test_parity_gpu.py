@@ -1070,6 +1070,83 @@ def test_dense_kernel_of_few_tokens_under_capture(oracle, fmt):
         d.close()
 
 
+@pytest.mark.parametrize("fmt", FORMATS)
+@pytest.mark.parametrize("n", [5, 16, 48])
+def test_a_captured_conversion_is_not_taken_for_a_made_one(oracle, fmt, n):
+    """A conversion recorded into a graph has not run, and one that a graph makes again at another length of the buffer
+    takes its place: an eager product multiplies the buffer's contents all the same.  A captured norm still spares its
+    product the conversion."""
+    import torch
+    from dwim_b200 import B200, Tensor
+    stream = torch.cuda.Stream()
+    d = B200(0, stream=stream.cuda_stream)
+    try:
+        rng = np.random.default_rng(79)
+        rows, cols, other = 96, 2048, n + 3      # (longer: no array that a graph reads is made anew)
+        blocks = oracle.quantize(fmt, (0.02 * rng.standard_normal((rows, cols))).astype(np.float32))
+        weight = d.upload(Tensor(fmt, (rows, cols), blocks))
+        x = rng.standard_normal((3, other, cols)).astype(np.float32)
+        want = [oracle.matmul(fmt, blocks, rows, cols, y).reshape(-1, rows) for y in x]
+        xb, out, gain = d.buffer(x[0]), d.alloc(other * rows), d.buffer(np.ones(cols, np.float32))
+
+        def at(tokens):
+            d.resize(xb, tokens * cols)
+            d.resize(out, tokens * rows)
+
+        def captured(call):
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                call()
+            return graph
+
+        def product():
+            d.matmul(out, weight, xb)
+
+        def right(y, tokens):
+            got = d.read(out).reshape(tokens, rows)
+            d.write(out, np.zeros(tokens * rows, np.float32))
+            return max_rel_err(got, want[y][:tokens]) <= 2e-5
+
+        at(other)
+        product()
+        graphs = [captured(product)]                      # at the other length
+        at(n)
+        product()
+        d.write(xb, x[1][:n])
+        graphs.append(captured(product))
+        product()
+        assert right(1, n), "an eager product after a capture that has not run"
+        for graph in (graphs[0], graphs[1], graphs[0]):
+            with torch.cuda.stream(stream):
+                graph.replay()
+            product()
+            assert right(1, n), "an eager product after a graph of another length"
+        # the norm's operand: made by its launch under the capture, not there before the graph has run
+        normed = d.alloc(n * cols)
+        d.normalize(normed, xb, gain, n * cols, 1e-6)
+        d.matmul(out, weight, normed)
+        d.write(normed, x[0][:n])
+        launches = d.launches
+        graphs.append(captured(lambda: (d.normalize(normed, xb, gain, n * cols, 1e-6), d.matmul(out, weight, normed))))
+        if fmt == "q4_k" or n != 16:                      # (groups of eight convert for themselves)
+            assert d.launches - launches == 2, "the product ran a conversion of its own"
+        d.matmul(out, weight, normed)
+        assert right(0, n), "an eager product after a captured norm that has not run"
+        for i in (2, 0):
+            d.write(xb, x[i][:n])
+            with torch.cuda.stream(stream):
+                graphs[1].replay()
+            assert right(i, n)
+        at(other)
+        d.write(xb, x[2])
+        with torch.cuda.stream(stream):
+            graphs[0].replay()
+        assert right(2, other), "captured while an eager product's operand was there"
+        del graphs, graph
+    finally:
+        d.close()
+
+
 @pytest.mark.parametrize("bf16", [True, False])
 def test_gemm_fused_epilogues_at_256_columns(dev, oracle, bf16):
     """matmul_add and swiglu through the 256-column kernel (300 tokens of bf16
