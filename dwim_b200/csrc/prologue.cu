@@ -273,7 +273,7 @@ __device__ __noinline__ Terms terms_clamped(float f0, float f1, float f2, float 
 //   by `weight` (Cpu::rmsnorm, gpu/cpu.rs:157-166: v * (scale * w) with
 //   scale = 1 / sqrt(sum(v^2) / dim + eps)); the f32 result goes to `xout`.
 // Then the row is scaled by a power of two 2^-e, chosen per token so that its
-// largest magnitude lands in [4, 8): whatever the activations' range, nothing
+// largest magnitude lands in [4, 8): whatever finite activations' range, nothing
 // is clamped, an activation down to 2^-16 of the token's largest keeps its
 // full f16 precision (and, for f32 inputs, the f16 remainder its share), and
 // the product's epilogue multiplies the token's results by 2^e (tok_scale)
@@ -337,9 +337,11 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? (R > 9 ? 1 : 2) : R 
     uint32_t top = row_max<THREADS>(largest(0x80000000u), s[1], rank, cluster, NORM);
     const bool finite = top < 0x7f800000u;
     if (!finite) top = row_max<THREADS>(largest(0x7f800001u), s[2], rank, cluster, true);     // a NaN is passed over
-    // the largest in [2^(b-127), 2^(b-126)) for its biased exponent b; e = b - 127 - 2, kept where 2^e and
-    // 2^-e are normal floats (a row of zeros, subnormals or infinities takes the nearest end)
-    const int e = top ? max(-100, min(100, (int)(top >> 23) - 129)) : 0;
+    // the largest in [2^(b-127), 2^(b-126)) for its biased exponent b; e = b - 127 - 2, at most 125 for a finite row;
+    // 2^e and 2^-e are normal floats then (a row whose largest is below 2^-123 takes the nearest end).  A row with an
+    // infinity or a NaN is clamped and stops at 2^100 either way.
+    const int most = finite ? 125 : 100;
+    const int e = top ? max(-most, min(most, (int)(top >> 23) - 129)) : 0;
     const float down = __uint_as_float((uint32_t)(127 - e) << 23);
     if (rank == 0 && k == 0) tok_scale[t] = __uint_as_float((uint32_t)(127 + e) << 23);
 #pragma unroll

@@ -1147,6 +1147,26 @@ def test_a_captured_conversion_is_not_taken_for_a_made_one(oracle, fmt, n):
         d.close()
 
 
+@pytest.mark.parametrize("fmt,n", [("q4_k", 16), ("q4_k", 40), ("q4_k", 150), ("q6_k", 40), ("q6_k", 80), ("q6_k", 150), ("q8_0", 40), ("q8_0", 150)])
+def test_gemm_activations_at_the_ends_of_f32(dev, oracle, fmt, n):
+    """Rows whose largest activation is near the ends of f32's exponents: the token's power of two reaches both, so that
+    such a row's result is as exact as an ordinary one's (the smallest here a little above the subnormals)."""
+    rng = np.random.default_rng(n)
+    rows, cols = 129, 768
+    weight, w, _, _ = random_pair(dev, oracle, fmt, rows, cols, rng)
+    x = rng.standard_normal((n, cols)).astype(np.float32)
+    sizes = (1.0, 1e36, 1e-34, 8e34, 3e37, 1e-30)
+    for i, size in enumerate(sizes):
+        x[i::len(sizes)] *= np.float32(size)
+    want = x.astype(np.float64) @ w.T
+    out = dev.alloc(n * rows)
+    dev.matmul(out, weight, dev.buffer(x))
+    got = dev.read(out).reshape(n, rows)
+    assert np.isfinite(got).all()
+    for t in range(n):
+        assert np.abs(got[t] - want[t]).max() <= 1e-5 * np.sqrt((want[t] ** 2).mean()), (t, sizes[t % len(sizes)])
+
+
 @pytest.mark.parametrize("bf16", [True, False])
 def test_gemm_fused_epilogues_at_256_columns(dev, oracle, bf16):
     """matmul_add and swiglu through the 256-column kernel (300 tokens of bf16
