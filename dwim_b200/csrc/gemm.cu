@@ -263,121 +263,7 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     // before their first store.
     griddep_launch();
 
-    if (warp == X_WARP) {
-        if constexpr (TRADE) regs_dec<OTHER_REGS>();
-        // ------------------------------ TMA producer ------------------------------
-        griddep_wait();   // the operand comes from the prologue kernel just ahead
-        if (elect_one()) {
-            int bs = 0, bturn = 1;
-            for (int u = 0; u < units; u++) {
-                const int ms = u % C::MIN_STAGES;
-                for (int p = PASSES - 1; p >= 0; p--)      // the remainders first
-                    for (int h = 0; h < KBLOCKS; h++) {
-                        uint32_t full = bfull0 + 8 * bs;
-                        if (JOINT) {
-                            // B stage kb % B_STAGES was last read by K block kb - B_STAGES
-                            const int kb = KBLOCKS * u + h, prev = kb - C::B_STAGES;
-                            if (prev >= 0)
-                                mbar_wait_parked(aempty0 + 8 * (prev % C::A_STAGES), (prev / C::A_STAGES) & 1, a.status, 0x20u);
-                            full = afull0 + 8 * (kb % C::A_STAGES);
-                        } else {
-                            mbar_wait_parked(bempty0 + 8 * bs, bturn, a.status, 0x20u);
-                        }
-                        mbar_expect_tx(full, C::TERM_BYTES * (C::WIDE ? a.terms : 1));
-                        const uint32_t to = bstage0 + bs * C::B_BYTES;
-                        const int k = (KBLOCKS * (ub + u) + h) * BK;
-                        tma_load_2d(to, &tmap_x, k, p * (int)a.n + col0, full);
-                        if (C::WIDE && a.terms == 2) tma_load_2d(to + C::TERM_BYTES, &tmap_x, k, (int)a.n + col0, full);
-                        if (++bs == C::B_STAGES) bs = 0, bturn ^= 1;
-                    }
-                // the minimums' stage was last read by unit u - MIN_STAGES
-                if (u >= C::MIN_STAGES) {
-                    const int uu = u - C::MIN_STAGES;
-                    mbar_wait_parked(accfull0 + 8 * (uu & 1), (uu >> 1) & 1, a.status, 0x40u);
-                }
-                mbar_expect_tx(minfull0 + 8 * ms, C::BMIN_BYTES);
-                const uint32_t bm = min0 + ms * C::MIN_BYTES + AMIN_BYTES;
-                tma_load_2d(bm, &tmap_m, (ub + u) * 16, col0, minfull0 + 8 * ms);                 // the means' hi parts
-                tma_load_2d(bm + BN * 16, &tmap_m, (ub + u) * 16 + 8, col0, minfull0 + 8 * ms);   // and lo parts
-            }
-        }
-    } else if (warp == RAW_WARP) {
-        if constexpr (TRADE) regs_dec<OTHER_REGS>();
-        // ------------------------------ packed weights' producer ------------------------------
-        // Its own warp: the blocks come from HBM and must run as far ahead as the
-        // ring allows, whatever the activations' producer is waiting for.
-        if (elect_one()) {
-            for (int u = 0; u < units; u++) {
-                const int rs = u % C::RAW_STAGES;
-                mbar_wait_parked(rawempty0 + 8 * rs, ((u / C::RAW_STAGES) & 1) ^ 1, a.status, 0x10u);
-                mbar_expect_tx(rawfull0 + 8 * rs, TILE_M * 144);
-                tma_load_2d(raw0 + rs * RAW_BYTES, &tmap_w, (ub + u) * 144, row0, rawfull0 + 8 * rs);
-            }
-        }
-    } else if (warp == MMA_WARP) {
-        if constexpr (TRADE) regs_dec<OTHER_REGS>();
-        // ------------------------------ MMA issuer ------------------------------
-        // The whole warp runs the loop (uniform control flow keeps addresses
-        // and descriptors on the uniform data path) and one lane issues.  Units
-        // are taken two at a time so that the accumulator buffer is static.
-        constexpr uint32_t idesc_min = idesc_f16(TILE_M, BN);
-        const uint32_t idesc = C::WIDE && a.terms == 2 ? idesc_f16(TILE_M, C::ACC_COLS) : idesc_min;
-        constexpr uint32_t desc_hi = DESC_HI_SW128;
-        const uint32_t a_lo = desc_lo_sw128(astage0), b_lo = desc_lo_sw128(bstage0);
-        const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
-        int bs = 0;                                                   // the next B stage
-        uint32_t bturn = 0, slot = 0, turn = 0;                       // its phase; the next A stage and its phase
-        for (int u0 = 0; u0 < units; u0 += 2) {
-#pragma unroll 1
-            for (int ab = 0; ab < 2; ab++) {      // (unrolled, the 256-column form spilled more and took 475 us instead of 403)
-                const int u = u0 + ab;
-                if (u >= units) break;
-                const uint32_t s1 = tm + ab * C::ACC_COLS;
-                const uint32_t upar = (u0 >> 1) & 1;
-                mbar_wait_parked(accempty0 + 8 * ab, upar ^ 1, a.status, 0x80u);   // the drain of unit u-2 is done
-                const uint32_t slot0 = slot, turn0 = turn;
-                // All of the unit's remainders, then its values: the sum grows to its size in the second pass only,
-                // whose additions alone the accumulator rounds at that size.
-                for (int p = PASSES - 1; p >= 0; p--) {
-                    const bool first = p == PASSES - 1;
-                    slot = slot0, turn = turn0;
-#pragma unroll
-                    for (int g = 0; g < KBLOCKS; g++) {
-                        if (C::A_STAGES == KBLOCKS) slot = g, turn = ab;
-                        if (first) mbar_wait_parked(afull0 + 8 * slot, turn, a.status, 0x100u);
-                        if (!JOINT) mbar_wait_parked(bfull0 + 8 * bs, bturn, a.status, 0x8000u);
-                        tc_fence_after();
-                        const uint32_t ad = a_lo + slot * (A_BYTES >> 4), bd = b_lo + bs * (C::B_BYTES >> 4);
-                        if (elect_one()) {
-#pragma unroll
-                            for (int k = 0; k < BK / 16; k++) {   // 32 bytes further along the swizzled row per K=16
-                                if (g == 0 && k == 0) umma_f16_lo(s1, ad, bd, desc_hi, idesc, !first);
-                                else umma_f16_lo<1>(s1, ad + 2 * k, bd + 2 * k, desc_hi, idesc);
-                            }
-                            // the stages may be refilled once these finish
-                            if (!JOINT) umma_commit(bempty0 + 8 * bs);
-                            if (p == 0) umma_commit(aempty0 + 8 * slot);
-                        }
-                        __syncwarp();
-                        if (++bs == C::B_STAGES) bs = 0, bturn ^= 1;
-                        if (C::A_STAGES != KBLOCKS && ++slot == C::A_STAGES) slot = 0, turn ^= 1;
-                    }
-                }
-                const int ms = u % C::MIN_STAGES;
-                mbar_wait_parked(minfull0 + 8 * ms, (u / C::MIN_STAGES) & 1, a.status, 0x200u);
-                tc_fence_after();
-                if (elect_one()) {
-                    // the minimums: terms (hi, hi | lo, lo) against the means' (hi, lo) twice
-                    const uint32_t am = min0 + ms * C::MIN_BYTES;
-                    const uint64_t bdm = smem_desc_plain(am + AMIN_BYTES, BN * 16);
-                    umma_f16(s1, smem_desc_plain(am, TILE_M * 16), bdm, idesc_min, 1);
-                    umma_f16(s1, smem_desc_plain(am + 2 * TILE_M * 16, TILE_M * 16), bdm, idesc_min, 1);
-                    umma_commit(accfull0 + 8 * ab);     // the unit's sum is complete
-                }
-                __syncwarp();
-            }
-        }
-    } else if (warp < N_WORKERS) {
+    if (warp < N_WORKERS) {
         if constexpr (TRADE) regs_inc<WORKER_REGS>();
         // ------------------------------ workers ------------------------------
         // Warp w owns TMEM lane quadrant w % 4 (weight rows 32*(w % 4) + lane)
@@ -544,8 +430,121 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             cluster_sync();
             cluster_sync();
         }
+    } else {
+        if constexpr (TRADE) regs_dec<OTHER_REGS>();      // (a warpgroup's warps at one instruction)
+        if (warp == X_WARP) {
+            // ------------------------------ TMA producer ------------------------------
+            griddep_wait();   // the operand comes from the prologue kernel just ahead
+            if (elect_one()) {
+                int bs = 0, bturn = 1;
+                for (int u = 0; u < units; u++) {
+                    const int ms = u % C::MIN_STAGES;
+                    for (int p = PASSES - 1; p >= 0; p--)      // the remainders first
+                        for (int h = 0; h < KBLOCKS; h++) {
+                            uint32_t full = bfull0 + 8 * bs;
+                            if (JOINT) {
+                                // B stage kb % B_STAGES was last read by K block kb - B_STAGES
+                                const int kb = KBLOCKS * u + h, prev = kb - C::B_STAGES;
+                                if (prev >= 0)
+                                    mbar_wait_parked(aempty0 + 8 * (prev % C::A_STAGES), (prev / C::A_STAGES) & 1, a.status, 0x20u);
+                                full = afull0 + 8 * (kb % C::A_STAGES);
+                            } else {
+                                mbar_wait_parked(bempty0 + 8 * bs, bturn, a.status, 0x20u);
+                            }
+                            mbar_expect_tx(full, C::TERM_BYTES * (C::WIDE ? a.terms : 1));
+                            const uint32_t to = bstage0 + bs * C::B_BYTES;
+                            const int k = (KBLOCKS * (ub + u) + h) * BK;
+                            tma_load_2d(to, &tmap_x, k, p * (int)a.n + col0, full);
+                            if (C::WIDE && a.terms == 2) tma_load_2d(to + C::TERM_BYTES, &tmap_x, k, (int)a.n + col0, full);
+                            if (++bs == C::B_STAGES) bs = 0, bturn ^= 1;
+                        }
+                    // the minimums' stage was last read by unit u - MIN_STAGES
+                    if (u >= C::MIN_STAGES) {
+                        const int uu = u - C::MIN_STAGES;
+                        mbar_wait_parked(accfull0 + 8 * (uu & 1), (uu >> 1) & 1, a.status, 0x40u);
+                    }
+                    mbar_expect_tx(minfull0 + 8 * ms, C::BMIN_BYTES);
+                    const uint32_t bm = min0 + ms * C::MIN_BYTES + AMIN_BYTES;
+                    tma_load_2d(bm, &tmap_m, (ub + u) * 16, col0, minfull0 + 8 * ms);                 // the means' hi parts
+                    tma_load_2d(bm + BN * 16, &tmap_m, (ub + u) * 16 + 8, col0, minfull0 + 8 * ms);   // and lo parts
+                }
+            }
+        } else if (warp == RAW_WARP) {
+            // ------------------------------ packed weights' producer ------------------------------
+            // Its own warp: the blocks come from HBM and must run as far ahead as the
+            // ring allows, whatever the activations' producer is waiting for.
+            if (elect_one()) {
+                for (int u = 0; u < units; u++) {
+                    const int rs = u % C::RAW_STAGES;
+                    mbar_wait_parked(rawempty0 + 8 * rs, ((u / C::RAW_STAGES) & 1) ^ 1, a.status, 0x10u);
+                    mbar_expect_tx(rawfull0 + 8 * rs, TILE_M * 144);
+                    tma_load_2d(raw0 + rs * RAW_BYTES, &tmap_w, (ub + u) * 144, row0, rawfull0 + 8 * rs);
+                }
+            }
+        } else if (warp == MMA_WARP) {
+            // ------------------------------ MMA issuer ------------------------------
+            // The whole warp runs the loop (uniform control flow keeps addresses
+            // and descriptors on the uniform data path) and one lane issues.  Units
+            // are taken two at a time so that the accumulator buffer is static.
+            constexpr uint32_t idesc_min = idesc_f16(TILE_M, BN);
+            const uint32_t idesc = C::WIDE && a.terms == 2 ? idesc_f16(TILE_M, C::ACC_COLS) : idesc_min;
+            constexpr uint32_t desc_hi = DESC_HI_SW128;
+            const uint32_t a_lo = desc_lo_sw128(astage0), b_lo = desc_lo_sw128(bstage0);
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
+            int bs = 0;                                                   // the next B stage
+            uint32_t bturn = 0, slot = 0, turn = 0;                       // its phase; the next A stage and its phase
+            for (int u0 = 0; u0 < units; u0 += 2) {
+    #pragma unroll 1
+                for (int ab = 0; ab < 2; ab++) {      // (unrolled, the 256-column form spilled more and took 475 us instead of 403)
+                    const int u = u0 + ab;
+                    if (u >= units) break;
+                    const uint32_t s1 = tm + ab * C::ACC_COLS;
+                    const uint32_t upar = (u0 >> 1) & 1;
+                    mbar_wait_parked(accempty0 + 8 * ab, upar ^ 1, a.status, 0x80u);   // the drain of unit u-2 is done
+                    const uint32_t slot0 = slot, turn0 = turn;
+                    // All of the unit's remainders, then its values: the sum grows to its size in the second pass only,
+                    // whose additions alone the accumulator rounds at that size.
+                    for (int p = PASSES - 1; p >= 0; p--) {
+                        const bool first = p == PASSES - 1;
+                        slot = slot0, turn = turn0;
+    #pragma unroll
+                        for (int g = 0; g < KBLOCKS; g++) {
+                            if (C::A_STAGES == KBLOCKS) slot = g, turn = ab;
+                            if (first) mbar_wait_parked(afull0 + 8 * slot, turn, a.status, 0x100u);
+                            if (!JOINT) mbar_wait_parked(bfull0 + 8 * bs, bturn, a.status, 0x8000u);
+                            tc_fence_after();
+                            const uint32_t ad = a_lo + slot * (A_BYTES >> 4), bd = b_lo + bs * (C::B_BYTES >> 4);
+                            if (elect_one()) {
+    #pragma unroll
+                                for (int k = 0; k < BK / 16; k++) {   // 32 bytes further along the swizzled row per K=16
+                                    if (g == 0 && k == 0) umma_f16_lo(s1, ad, bd, desc_hi, idesc, !first);
+                                    else umma_f16_lo<1>(s1, ad + 2 * k, bd + 2 * k, desc_hi, idesc);
+                                }
+                                // the stages may be refilled once these finish
+                                if (!JOINT) umma_commit(bempty0 + 8 * bs);
+                                if (p == 0) umma_commit(aempty0 + 8 * slot);
+                            }
+                            __syncwarp();
+                            if (++bs == C::B_STAGES) bs = 0, bturn ^= 1;
+                            if (C::A_STAGES != KBLOCKS && ++slot == C::A_STAGES) slot = 0, turn ^= 1;
+                        }
+                    }
+                    const int ms = u % C::MIN_STAGES;
+                    mbar_wait_parked(minfull0 + 8 * ms, (u / C::MIN_STAGES) & 1, a.status, 0x200u);
+                    tc_fence_after();
+                    if (elect_one()) {
+                        // the minimums: terms (hi, hi | lo, lo) against the means' (hi, lo) twice
+                        const uint32_t am = min0 + ms * C::MIN_BYTES;
+                        const uint64_t bdm = smem_desc_plain(am + AMIN_BYTES, BN * 16);
+                        umma_f16(s1, smem_desc_plain(am, TILE_M * 16), bdm, idesc_min, 1);
+                        umma_f16(s1, smem_desc_plain(am + 2 * TILE_M * 16, TILE_M * 16), bdm, idesc_min, 1);
+                        umma_commit(accfull0 + 8 * ab);     // the unit's sum is complete
+                    }
+                    __syncwarp();
+                }
+            }
+        }
     }
-    if constexpr (TRADE) { if (warp > RAW_WARP) regs_dec<OTHER_REGS>(); }      // (the warpgroup takes part as a whole)
     if (warp >= N_WORKERS) {
         __syncwarp();
         if (split_k > 1) {      // the workers' two meetings are the whole cluster's
@@ -673,82 +672,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     const uint32_t tmem_base = lds32(tmem_slot);
     griddep_launch();
 
-    if (warp == X_WARP) {
-        regs_dec<DENSE_OTHER_REGS>();
-        griddep_wait();   // the operand comes from the prologue kernel just ahead
-        if (elect_one()) {
-            int s = 0, turn = 1;
-            for (int kb = 0; kb < KBLOCKS * units; kb++)
-                for (int p = PASSES - 1; p >= 0; p--) {      // the remainders first
-                    mbar_wait_parked(bempty0 + 8 * s, turn, a.status, 0x100000u);
-                    mbar_expect_tx(bfull0 + 8 * s, C::TERM_BYTES * (C::WIDE ? a.terms : 1));
-                    const uint32_t to = bstage0 + s * C::B_BYTES;
-                    tma_load_2d(to, &tmap_x, (KBLOCKS * ub + kb) * BK, p * (int)a.n + col0, bfull0 + 8 * s);
-                    if (C::WIDE && a.terms == 2) tma_load_2d(to + C::TERM_BYTES, &tmap_x, (KBLOCKS * ub + kb) * BK, (int)a.n + col0, bfull0 + 8 * s);
-                    if (++s == C::B_STAGES) s = 0, turn ^= 1;
-                }
-        }
-    } else if (warp == RAW_WARP) {
-        regs_dec<DENSE_OTHER_REGS>();
-        if (elect_one()) {
-            for (int r = 0; r < C::RAW_STEPS * units; r++) {
-                const int s = r % C::RAW_STAGES;
-                mbar_wait_parked(rawempty0 + 8 * s, ((r / C::RAW_STAGES) & 1) ^ 1, a.status, 0x200000u);
-                mbar_expect_tx(rawfull0 + 8 * s, C::RAW_STAGE);
-                tma_load_2d(raw0 + s * C::RAW_STAGE, &tmap_w, FMT == Q8_0 ? (2 * ub + r) * 128 : (ub + r) * Q6_K_DEV, row0, rawfull0 + 8 * s);
-            }
-        }
-    } else if (warp == MMA_WARP) {
-        regs_dec<DENSE_OTHER_REGS>();
-        const uint32_t idesc = idesc_f16(TILE_M, C::WIDE && a.terms == 2 ? C::ACC_COLS : BN);
-        const uint32_t a_lo = desc_lo_sw128(astage0), b_lo = desc_lo_sw128(bstage0);
-        const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
-        int bs = 0, bturn = 0, buf = 0, bufturn = 1;
-        for (int u = 0; u < units; u++) {
-#pragma unroll
-            for (int g = 0; g < KBLOCKS; g++) {
-                const uint32_t acc = tm + buf * C::ACC_COLS;
-                // What a K block needs: asked by lanes of the warp at once where its MMAs are so short that the 85 cycles
-                // of a test count ([5120, 5120] Q8_0 by 48 tokens 24.6 us one by one, 23.1 like this; wider tiles spill).
-                constexpr bool AT_ONCE = C::STEPS == 4;
-                if (!AT_ONCE) {
-                    if (g % DRAIN_KB == 0) mbar_wait_parked(accempty0 + 8 * buf, bufturn, a.status, 0x400000u);
-                    mbar_wait_parked(afull0 + 8 * g, u & 1, a.status, 0x1000000u);
-                }
-#pragma unroll AT_ONCE ? 2 : 1
-                for (int p = PASSES - 1; p >= 0; p--) {
-                    if (AT_ONCE) {
-                        uint32_t bar = bfull0 + 8 * bs, phase = bturn;
-                        if (p == PASSES - 1 && (lane & 1)) bar = afull0 + 8 * g, phase = u & 1;
-                        if (p == PASSES - 1 && (lane & 2)) bar = accempty0 + 8 * buf, phase = bufturn;
-                        mbar_wait_all(bar, phase, a.status, 0x800000u);
-                    } else {
-                        mbar_wait_parked(bfull0 + 8 * bs, bturn, a.status, 0x800000u);
-                    }
-                    tc_fence_after();
-                    if (elect_one()) {
-                        // the weights' remainders first: they are too small for the accumulator's rounding to matter
-                        const uint32_t hi = a_lo + g % C::A_STAGES * (C::A_STAGE >> 4), lo = hi + (A_BYTES >> 4), bd = b_lo + bs * (C::B_BYTES >> 4);
-#pragma unroll
-                        for (int k = 0; k < BK / 16; k++) {
-                            if (g % DRAIN_KB == 0 && k == 0) umma_f16_lo(acc, lo, bd, DESC_HI_SW128, idesc, p != PASSES - 1);
-                            else umma_f16_lo<1>(acc, lo + 2 * k, bd + 2 * k, DESC_HI_SW128, idesc);
-                        }
-#pragma unroll
-                        for (int k = 0; k < BK / 16; k++) umma_f16_lo<1>(acc, hi + 2 * k, bd + 2 * k, DESC_HI_SW128, idesc);
-                        umma_commit(bempty0 + 8 * bs);
-                        if (p == 0) {
-                            umma_commit(adone0 + 8 * g);
-                            if (g % DRAIN_KB == DRAIN_KB - 1) umma_commit(accfull0 + 8 * buf);
-                        }
-                    }
-                    __syncwarp();
-                    if (++bs == C::B_STAGES) bs = 0, bturn ^= 1;
-                }
-                if (g % DRAIN_KB == DRAIN_KB - 1 && ++buf == C::ACC_BUFS) buf = 0, bufturn ^= 1;
-            }
-        }
-    } else if (warp < N_WORKERS) {
+    if (warp < N_WORKERS) {
         regs_inc<DENSE_WORKER_REGS>();
         const int quad = warp & 3, g = warp >> 2, rl = quad * 32 + lane;
         const uint32_t drain_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + g * C::DRAIN_COLS;
@@ -920,8 +844,82 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             for (int j = 0; j < 8; j++) v[j] *= lds32f(tk + (8 * q + j) * 4);
             gemm_emit<SHARED>(to, a.rows, a.n, (size_t)col0 + g * C::DRAIN_COLS + 8 * q, v);
         }
+    } else {
+        regs_dec<DENSE_OTHER_REGS>();      // (a warpgroup's warps at one instruction)
+        if (warp == X_WARP) {
+            griddep_wait();   // the operand comes from the prologue kernel just ahead
+            if (elect_one()) {
+                int s = 0, turn = 1;
+                for (int kb = 0; kb < KBLOCKS * units; kb++)
+                    for (int p = PASSES - 1; p >= 0; p--) {      // the remainders first
+                        mbar_wait_parked(bempty0 + 8 * s, turn, a.status, 0x100000u);
+                        mbar_expect_tx(bfull0 + 8 * s, C::TERM_BYTES * (C::WIDE ? a.terms : 1));
+                        const uint32_t to = bstage0 + s * C::B_BYTES;
+                        tma_load_2d(to, &tmap_x, (KBLOCKS * ub + kb) * BK, p * (int)a.n + col0, bfull0 + 8 * s);
+                        if (C::WIDE && a.terms == 2) tma_load_2d(to + C::TERM_BYTES, &tmap_x, (KBLOCKS * ub + kb) * BK, (int)a.n + col0, bfull0 + 8 * s);
+                        if (++s == C::B_STAGES) s = 0, turn ^= 1;
+                    }
+            }
+        } else if (warp == RAW_WARP) {
+            if (elect_one()) {
+                for (int r = 0; r < C::RAW_STEPS * units; r++) {
+                    const int s = r % C::RAW_STAGES;
+                    mbar_wait_parked(rawempty0 + 8 * s, ((r / C::RAW_STAGES) & 1) ^ 1, a.status, 0x200000u);
+                    mbar_expect_tx(rawfull0 + 8 * s, C::RAW_STAGE);
+                    tma_load_2d(raw0 + s * C::RAW_STAGE, &tmap_w, FMT == Q8_0 ? (2 * ub + r) * 128 : (ub + r) * Q6_K_DEV, row0, rawfull0 + 8 * s);
+                }
+            }
+        } else if (warp == MMA_WARP) {
+            const uint32_t idesc = idesc_f16(TILE_M, C::WIDE && a.terms == 2 ? C::ACC_COLS : BN);
+            const uint32_t a_lo = desc_lo_sw128(astage0), b_lo = desc_lo_sw128(bstage0);
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
+            int bs = 0, bturn = 0, buf = 0, bufturn = 1;
+            for (int u = 0; u < units; u++) {
+    #pragma unroll
+                for (int g = 0; g < KBLOCKS; g++) {
+                    const uint32_t acc = tm + buf * C::ACC_COLS;
+                    // What a K block needs: asked by lanes of the warp at once where its MMAs are so short that the 85 cycles
+                    // of a test count ([5120, 5120] Q8_0 by 48 tokens 24.6 us one by one, 23.1 like this; wider tiles spill).
+                    constexpr bool AT_ONCE = C::STEPS == 4;
+                    if (!AT_ONCE) {
+                        if (g % DRAIN_KB == 0) mbar_wait_parked(accempty0 + 8 * buf, bufturn, a.status, 0x400000u);
+                        mbar_wait_parked(afull0 + 8 * g, u & 1, a.status, 0x1000000u);
+                    }
+    #pragma unroll AT_ONCE ? 2 : 1
+                    for (int p = PASSES - 1; p >= 0; p--) {
+                        if (AT_ONCE) {
+                            uint32_t bar = bfull0 + 8 * bs, phase = bturn;
+                            if (p == PASSES - 1 && (lane & 1)) bar = afull0 + 8 * g, phase = u & 1;
+                            if (p == PASSES - 1 && (lane & 2)) bar = accempty0 + 8 * buf, phase = bufturn;
+                            mbar_wait_all(bar, phase, a.status, 0x800000u);
+                        } else {
+                            mbar_wait_parked(bfull0 + 8 * bs, bturn, a.status, 0x800000u);
+                        }
+                        tc_fence_after();
+                        if (elect_one()) {
+                            // the weights' remainders first: they are too small for the accumulator's rounding to matter
+                            const uint32_t hi = a_lo + g % C::A_STAGES * (C::A_STAGE >> 4), lo = hi + (A_BYTES >> 4), bd = b_lo + bs * (C::B_BYTES >> 4);
+    #pragma unroll
+                            for (int k = 0; k < BK / 16; k++) {
+                                if (g % DRAIN_KB == 0 && k == 0) umma_f16_lo(acc, lo, bd, DESC_HI_SW128, idesc, p != PASSES - 1);
+                                else umma_f16_lo<1>(acc, lo + 2 * k, bd + 2 * k, DESC_HI_SW128, idesc);
+                            }
+    #pragma unroll
+                            for (int k = 0; k < BK / 16; k++) umma_f16_lo<1>(acc, hi + 2 * k, bd + 2 * k, DESC_HI_SW128, idesc);
+                            umma_commit(bempty0 + 8 * bs);
+                            if (p == 0) {
+                                umma_commit(adone0 + 8 * g);
+                                if (g % DRAIN_KB == DRAIN_KB - 1) umma_commit(accfull0 + 8 * buf);
+                            }
+                        }
+                        __syncwarp();
+                        if (++bs == C::B_STAGES) bs = 0, bturn ^= 1;
+                    }
+                    if (g % DRAIN_KB == DRAIN_KB - 1 && ++buf == C::ACC_BUFS) buf = 0, bufturn ^= 1;
+                }
+            }
+        }
     }
-    if (warp > RAW_WARP) regs_dec<DENSE_OTHER_REGS>();      // (the warpgroup takes part as a whole)
     if (warp >= N_WORKERS) {
         __syncwarp();
         if (split_k > 1) {      // the workers' two meetings are the whole cluster's

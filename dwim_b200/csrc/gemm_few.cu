@@ -200,96 +200,9 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     const uint32_t tmem_base = lds32(tmem_slot);
     griddep_launch();
 
-    if (warp == FEW_X_WARP || warp == FEW_X_WARP + 1) {
-        regs_dec<FEW_OTHER_REGS>();
-        griddep_wait();   // the operand comes from the prologue kernel just ahead
-        if (elect_one()) {
-            int turn = 1, row = 0;      // a group's stages are used in turn
-            for (int u0 = 2 * (warp - FEW_X_WARP); u0 < units; u0 += GROUPS) {
-                const int last = min(u0 + 2, units);
-                for (int g = 0; g < KBLOCKS; g += C::STAGE_KB) {
-                    for (int u = u0; u < last; u++) {
-                        const int bs = row * GROUPS + u % GROUPS;
-                        mbar_wait_parked(bempty0 + 8 * bs, turn, a.status, 0x20u);
-                        mbar_expect_tx(bfull0 + 8 * bs, C::TERM_BYTES * a.terms);
-                        tma_load_4d(bstage0 + bs * C::B_BYTES, &tmap_x, 0, 0, KBLOCKS * (ub + u) + g, 0, bfull0 + 8 * bs);
-                    }
-                    if (++row == C::B_STAGES / GROUPS) row = 0, turn ^= 1;
-                }
-            }
-        }
-    } else if (warp == FEW_MEANS_WARP) {
-        regs_dec<FEW_OTHER_REGS>();
-        griddep_wait();
-        if (elect_one()) {
-            for (int u = 0; u < units; u++) {
-                const int ms = u % C::MIN_STAGES;
-                mbar_wait_parked(minempty0 + 8 * ms, ((u / C::MIN_STAGES) & 1) ^ 1, a.status, 0x40u);
-                mbar_expect_tx(minfull0 + 8 * ms, C::MIN_BYTES);
-                tma_load_3d(min0 + ms * C::MIN_BYTES, &tmap_m, 0, 0, (ub + u) * 2, minfull0 + 8 * ms);      // [hi, lo][token][8]
-            }
-        }
-    } else if (warp == FEW_RAW_WARP) {
-        regs_dec<FEW_OTHER_REGS>();
-        if (elect_one()) {
-            int rs = 0, turn = 1;
-            for (int u = 0; u < units; u++) {
-                mbar_wait_parked(rawempty0 + 8 * rs, turn, a.status, 0x10u);
-                mbar_expect_tx(rawfull0 + 8 * rs, TILE_M * 144);
-                tma_load_2d(raw0 + rs * RAW_BYTES, &tmap_w, (ub + u) * 144, row0, rawfull0 + 8 * rs);
-                if (++rs == C::RAW_STAGES) rs = 0, turn ^= 1;
-            }
-        }
-    } else if (warp >= FEW_MMA_WARP && warp < FEW_MMA_WARP + GROUPS) {
-        regs_dec<FEW_OTHER_REGS>();
-        constexpr uint32_t idesc = idesc_f16(TILE_M, N);
-        const int i = __shfl_sync(0xffffffffu, warp, 0) - FEW_MMA_WARP;
-        const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0), b_lo = desc_lo_sw128(bstage0);
-        const uint32_t d = tm + i * N, a0 = tm + C::ACC_COLS + i * C::GROUP_COLS, afull = afull0 + 8 * i * C::SLOTS, aempty = aempty0 + 8 * i * C::SLOTS;
-        int bs = i;
-        uint32_t bturn = 0, turn = 0;
-        // the lanes wait for several barriers at once: lane % 4 chooses
-        auto wait = [&](uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, uint32_t b2, uint32_t p2) {
-            const int l = lane & 3;
-            mbar_wait_all(l == 0 ? b0 : l == 1 ? b1 : b2, l == 0 ? p0 : l == 1 ? p1 : p2, a.status, 0x100u);
-            tc_fence_after();
-        };
-        for (int u = i; u < units; u += GROUPS, turn ^= 1) {
-            const int ms = u % C::MIN_STAGES;
-            // the minimums, terms (hi, hi | lo, lo) against the means' (hi, lo) twice, open the unit's sums
-            wait(accempty0 + 8 * i, turn ^ 1, minfull0 + 8 * ms, (u / C::MIN_STAGES) & 1, mfull0 + 8 * i, turn);
-            if (elect_one()) {
-                const uint32_t at = a0 + C::SLOTS * C::SLOT_COLS;
-                const uint64_t bd = smem_desc_plain(min0 + ms * C::MIN_BYTES, N * 16);
-                umma_ts(d, at, (uint32_t)bd, (uint32_t)(bd >> 32), idesc, false);
-                umma_ts(d, at + 8, (uint32_t)bd, (uint32_t)(bd >> 32), idesc, true);
-                umma_commit(minempty0 + 8 * ms);
-                umma_commit(mempty0 + 8 * i);
-            }
-            __syncwarp();
-#pragma unroll
-            for (int g = 0; g < KBLOCKS; g++) {
-                const uint32_t ab = afull + 8 * (g & 1), bb = bfull0 + 8 * bs, par = g >> 1;      // a slot is used twice a unit
-                if (g % C::STAGE_KB == 0) wait(bb, bturn, bb, bturn, ab, par);
-                else wait(ab, par, ab, par, ab, par);
-                if (elect_one()) {
-                    const uint32_t at = a0 + (g & 1) * C::SLOT_COLS;
-                    const uint32_t bd = b_lo + ((bs * C::B_BYTES + g % C::STAGE_KB * C::TILE_BYTES) >> 4);
-                    if (a.terms == 2) {       // the remainders first
-#pragma unroll
-                        for (int k = 0; k < BK / 16; k++) umma_ts(d, at + 8 * k, bd + (C::TERM_BYTES >> 4) + 2 * k, DESC_HI_SW128, idesc, true);
-                    }
-#pragma unroll
-                    for (int k = 0; k < BK / 16; k++) umma_ts(d, at + 8 * k, bd + 2 * k, DESC_HI_SW128, idesc, true);
-                    umma_commit(aempty + 8 * (g & 1));
-                    if (g % C::STAGE_KB == C::STAGE_KB - 1) umma_commit(bempty0 + 8 * bs);
-                    if (g == KBLOCKS - 1) umma_commit(accfull0 + 8 * i);
-                }
-                __syncwarp();
-                if (g % C::STAGE_KB == C::STAGE_KB - 1 && (bs += GROUPS) >= C::B_STAGES) bs = i, bturn ^= 1;
-            }
-        }
-    } else if (warp < N_WORKERS) {
+    // (A warpgroup's warps trade their registers at one instruction.  The workers' branch first: behind the others' the
+    // compiler made a layer of 16 tokens 125 us of 122.)
+    if (warp < N_WORKERS) {
         regs_inc<FEW_WORKER_REGS>();
         const int quad = warp & 3, i = warp >> 2, rl = quad * 32 + lane;      // i: the group
         const uint32_t lanes = tmem_base + ((uint32_t)(quad * 32) << 16);
@@ -390,6 +303,95 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
                 if (a.epi == EPI_ADD) v += y[j];
                 else if (a.epi == EPI_SWIGLU) v = silu_mul_f(v, y[j]);
                 to.own[c * to.pitch] = v;
+            }
+        }
+    } else if (warp < FEW_X_WARP) {
+        regs_dec<FEW_OTHER_REGS>();
+        constexpr uint32_t idesc = idesc_f16(TILE_M, N);
+        const int i = __shfl_sync(0xffffffffu, warp, 0) - FEW_MMA_WARP;
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0), b_lo = desc_lo_sw128(bstage0);
+        const uint32_t d = tm + i * N, a0 = tm + C::ACC_COLS + i * C::GROUP_COLS, afull = afull0 + 8 * i * C::SLOTS, aempty = aempty0 + 8 * i * C::SLOTS;
+        int bs = i;
+        uint32_t bturn = 0, turn = 0;
+        // the lanes wait for several barriers at once: lane % 4 chooses
+        auto wait = [&](uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, uint32_t b2, uint32_t p2) {
+            const int l = lane & 3;
+            mbar_wait_all(l == 0 ? b0 : l == 1 ? b1 : b2, l == 0 ? p0 : l == 1 ? p1 : p2, a.status, 0x100u);
+            tc_fence_after();
+        };
+        for (int u = i; u < units; u += GROUPS, turn ^= 1) {
+            const int ms = u % C::MIN_STAGES;
+            // the minimums, terms (hi, hi | lo, lo) against the means' (hi, lo) twice, open the unit's sums
+            wait(accempty0 + 8 * i, turn ^ 1, minfull0 + 8 * ms, (u / C::MIN_STAGES) & 1, mfull0 + 8 * i, turn);
+            if (elect_one()) {
+                const uint32_t at = a0 + C::SLOTS * C::SLOT_COLS;
+                const uint64_t bd = smem_desc_plain(min0 + ms * C::MIN_BYTES, N * 16);
+                umma_ts(d, at, (uint32_t)bd, (uint32_t)(bd >> 32), idesc, false);
+                umma_ts(d, at + 8, (uint32_t)bd, (uint32_t)(bd >> 32), idesc, true);
+                umma_commit(minempty0 + 8 * ms);
+                umma_commit(mempty0 + 8 * i);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int g = 0; g < KBLOCKS; g++) {
+                const uint32_t ab = afull + 8 * (g & 1), bb = bfull0 + 8 * bs, par = g >> 1;      // a slot is used twice a unit
+                if (g % C::STAGE_KB == 0) wait(bb, bturn, bb, bturn, ab, par);
+                else wait(ab, par, ab, par, ab, par);
+                if (elect_one()) {
+                    const uint32_t at = a0 + (g & 1) * C::SLOT_COLS;
+                    const uint32_t bd = b_lo + ((bs * C::B_BYTES + g % C::STAGE_KB * C::TILE_BYTES) >> 4);
+                    if (a.terms == 2) {       // the remainders first
+#pragma unroll
+                        for (int k = 0; k < BK / 16; k++) umma_ts(d, at + 8 * k, bd + (C::TERM_BYTES >> 4) + 2 * k, DESC_HI_SW128, idesc, true);
+                    }
+#pragma unroll
+                    for (int k = 0; k < BK / 16; k++) umma_ts(d, at + 8 * k, bd + 2 * k, DESC_HI_SW128, idesc, true);
+                    umma_commit(aempty + 8 * (g & 1));
+                    if (g % C::STAGE_KB == C::STAGE_KB - 1) umma_commit(bempty0 + 8 * bs);
+                    if (g == KBLOCKS - 1) umma_commit(accfull0 + 8 * i);
+                }
+                __syncwarp();
+                if (g % C::STAGE_KB == C::STAGE_KB - 1 && (bs += GROUPS) >= C::B_STAGES) bs = i, bturn ^= 1;
+            }
+        }
+    } else {
+        regs_dec<FEW_OTHER_REGS>();
+        if (warp == FEW_X_WARP || warp == FEW_X_WARP + 1) {
+            griddep_wait();   // the operand comes from the prologue kernel just ahead
+            if (elect_one()) {
+                int turn = 1, row = 0;      // a group's stages are used in turn
+                for (int u0 = 2 * (warp - FEW_X_WARP); u0 < units; u0 += GROUPS) {
+                    const int last = min(u0 + 2, units);
+                    for (int g = 0; g < KBLOCKS; g += C::STAGE_KB) {
+                        for (int u = u0; u < last; u++) {
+                            const int bs = row * GROUPS + u % GROUPS;
+                            mbar_wait_parked(bempty0 + 8 * bs, turn, a.status, 0x20u);
+                            mbar_expect_tx(bfull0 + 8 * bs, C::TERM_BYTES * a.terms);
+                            tma_load_4d(bstage0 + bs * C::B_BYTES, &tmap_x, 0, 0, KBLOCKS * (ub + u) + g, 0, bfull0 + 8 * bs);
+                        }
+                        if (++row == C::B_STAGES / GROUPS) row = 0, turn ^= 1;
+                    }
+                }
+            }
+        } else if (warp == FEW_MEANS_WARP) {
+            griddep_wait();
+            if (elect_one()) {
+                for (int u = 0; u < units; u++) {
+                    const int ms = u % C::MIN_STAGES;
+                    mbar_wait_parked(minempty0 + 8 * ms, ((u / C::MIN_STAGES) & 1) ^ 1, a.status, 0x40u);
+                    mbar_expect_tx(minfull0 + 8 * ms, C::MIN_BYTES);
+                    tma_load_3d(min0 + ms * C::MIN_BYTES, &tmap_m, 0, 0, (ub + u) * 2, minfull0 + 8 * ms);      // [hi, lo][token][8]
+                }
+            }
+        } else if (warp == FEW_RAW_WARP) {
+            if (elect_one()) {
+                int rs = 0, turn = 1;
+                for (int u = 0; u < units; u++) {
+                    mbar_wait_parked(rawempty0 + 8 * rs, turn, a.status, 0x10u);
+                    mbar_expect_tx(rawfull0 + 8 * rs, TILE_M * 144);
+                    tma_load_2d(raw0 + rs * RAW_BYTES, &tmap_w, (ub + u) * 144, row0, rawfull0 + 8 * rs);
+                    if (++rs == C::RAW_STAGES) rs = 0, turn ^= 1;
+                }
             }
         }
     }

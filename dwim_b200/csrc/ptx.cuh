@@ -113,7 +113,8 @@ __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wa
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // A warpgroup gives up registers of its threads', or takes some that others of its block gave up (and waits
-// until they did).  The shares must add up to no more than the block was launched with.
+// until they did).  The shares must add up to no more than the block was launched with, and the warpgroup's four
+// warps execute the same instruction: one in the code, ahead of what tells its warps apart.
 template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 

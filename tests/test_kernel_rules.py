@@ -60,3 +60,27 @@ def test_process_wide_variables_may_be_shared_by_threads(name):
     for m in re.finditer(r"\bstatic\s+((?:[\w:]|<[^<>]*>|\s|\*)+?)\s*\b(\w+)\s*(?:\[[^\]]*\]\s*)*(?:=|;|\{)", source(name)):
         kind = m.group(1)
         assert re.search(r"\b(const|constexpr|thread_local|__device__)\b|\batomic<", kind), f"{name}: static {kind} {m.group(2)}"
+
+
+def test_a_warpgroup_trades_registers_at_one_instruction():
+    """setmaxnreg is for whole warpgroups: all four warps execute the same one.  So it stands first in a branch that
+    parts the warps at a multiple of four, ahead of what tells a warpgroup's warps apart; the workers, who take, first."""
+    text = "\n".join(source(f) for f in HEADERS + SOURCES)
+    numbers = {name: int(value) for name, value in re.findall(r"\b(\w*(?:WARP|WORKERS))\s*=\s*(\d+)\b", text)}
+    traders = 0
+    for name in SOURCES:
+        for function, body in functions(source(name)):
+            trades = list(re.finditer(r"\bregs_(dec|inc)\s*<", body))
+            if not trades:
+                continue
+            traders += 1
+            assert [m.group(1) for m in trades] == ["inc"] + ["dec"] * (len(trades) - 1), function
+            ends = [0]
+            for m in trades:
+                ahead = re.sub(r"if constexpr \(TRADE\)\s*$", "", body[:m.start()]).rstrip()
+                branch = re.search(r"(?:if \(warp < (\w+)\)|else) \{$", ahead)
+                assert branch, f"{function}: regs_{m.group(1)} is not the first of a branch for whole warpgroups"
+                assert bool(branch.group(1)) == (m is not trades[-1]), function
+                ends += [numbers[branch.group(1)]] if branch.group(1) else []
+            assert all(e % 4 == 0 for e in ends) and ends == sorted(set(ends)), f"{function}: branches at warps {ends}"
+    assert traders == 3
