@@ -88,15 +88,18 @@ __device__ __forceinline__ void mbar_wait_parked(uint32_t bar, uint32_t parity, 
         if (i % 1024 == 0 && mbar_gave_up(start, status, code)) return;
     }
 }
-// The whole warp waits until the barriers of all its lanes are through.
+// The whole warp waits until the barriers of all its lanes are through.  A lane has seen its own barrier alone, and a vote
+// orders no memory: the warp meets before one lane goes on with what all of them stand for.
 __device__ __forceinline__ void mbar_wait_all(uint32_t bar, uint32_t parity, uint32_t *status, uint32_t code) {
-    if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return;
-    uint64_t start = 0;
+    if (!__all_sync(0xffffffffu, mbar_try(bar, parity))) {
+        uint64_t start = 0;
 #pragma unroll 1
-    for (uint32_t i = 1;; i++) {
-        if (__all_sync(0xffffffffu, mbar_try_suspend(bar, parity))) return;
-        if (i % 1024 == 0 && __any_sync(0xffffffffu, mbar_gave_up(start, status, code))) return;
+        for (uint32_t i = 1;; i++) {
+            if (__all_sync(0xffffffffu, mbar_try_suspend(bar, parity))) break;
+            if (i % 1024 == 0 && __any_sync(0xffffffffu, mbar_gave_up(start, status, code))) break;
+        }
     }
+    __syncwarp();
 }
 __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, uint32_t *status, uint32_t code) {
 #pragma unroll 1

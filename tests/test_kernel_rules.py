@@ -84,3 +84,10 @@ def test_a_warpgroup_trades_registers_at_one_instruction():
                 ends += [numbers[branch.group(1)]] if branch.group(1) else []
             assert all(e % 4 == 0 for e in ends) and ends == sorted(set(ends)), f"{function}: branches at warps {ends}"
     assert traders == 3
+
+
+def test_lanes_that_waited_for_several_barriers_meet():
+    """A lane that waited for one of several barriers has acquired that one's writes alone, and a warp vote does not order
+    memory among lanes: a wait of the whole warp ends at a __syncwarp, on every path."""
+    body = dict(functions(source("ptx.cuh")))["mbar_wait_all"]
+    assert "return" not in body and re.search(r"__syncwarp\(\);\s*\}$", body)
