@@ -22,7 +22,7 @@ namespace dwim {
 // gemm.cu
 bool gemm_takes(const WeightView &w, size_t n, int terms);
 int gemm_large(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, size_t n, int terms, const OutSpec &out,
-               const float *aux, int epilogue);
+               const float *aux, int epilogue, size_t whole);
 
 int reserve_shadow(dwim_b200_ctx *ctx, dwim_b200_buffer *b, size_t need) {
     if (need <= b->shadow_cap) return 0;
@@ -348,6 +348,8 @@ int dwim_b200_buffer_free(dwim_b200_ctx *ctx, dwim_b200_buffer *buf) {
     if (buf->owned && buf->data) cudaFree(buf->data);
     if (buf->shadow) cudaFree(buf->shadow);
     if (buf->groups) cudaFree(buf->groups);
+    for (void *operand : buf->operands)
+        if (operand) cudaFree(operand);
     delete buf;
     return 0;
 }
@@ -507,52 +509,96 @@ static int ensure_shadow(dwim_b200_ctx *ctx, dwim_b200_buffer *x, int kind, size
 
 constexpr size_t GROUPS_AT_ONCE = 64;
 
-// Room for products of Q6_K and Q8_0 by nine tokens and more: the digit planes of all the groups of eight tokens that
-// `x` can hold, up to GROUPS_AT_ONCE, or its operand for the dense kernel, in one array.  It spares launches or time and
-// no product needs it: it is never made anew at another length of the buffer (a graph captured at one length may still
+// Room for the digit planes of all the groups of eight tokens that `x` can hold, up to GROUPS_AT_ONCE.  It spares launches
+// and no product needs it: it is never made anew at another length of the buffer (a graph captured at one length may still
 // read it), not allocated under a stream capture, and done without when memory is short.
 static void reserve_groups(dwim_b200_ctx *ctx, dwim_b200_buffer *x, size_t cols, size_t group) {
     size_t most = x->cap / cols / I8_MAX_TOKENS;
     if (most > GROUPS_AT_ONCE) most = GROUPS_AT_ONCE;
     if (x->groups_tried || most < 2 || capture_id(ctx)) return;
-    // the dense kernel's: of all the tokens where it takes any number in this way, else of its tile's
-    size_t tokens = x->cap / cols;
-    if (tokens > 64 && cols <= 12288) tokens = 64;
-    const size_t planes = most * group, operand = cols % 256 ? 0 : gemm_operand_bytes(cols, tokens, 1);
     x->groups_tried = true;
-    for (size_t bytes = planes > operand ? planes : operand;; bytes = planes) {
-        if (cudaMalloc(&x->groups, bytes) == cudaSuccess) {
-            x->groups_cap = bytes;
-            return;
-        }
+    if (cudaMalloc(&x->groups, most * group) == cudaSuccess) {
+        x->groups_cap = most * group;
+    } else {
         x->groups = nullptr;
         cudaGetLastError();
-        if (bytes == planes) return;
     }
 }
 
-// The operand of a product that the groups of eight tokens could take as well: in the shadow where it fits, else in the
-// groups' array; null where there is no room.  (The shadow is not made longer for it: graphs captured with the groups'
-// planes in it would read freed memory.  Under a capture the conversion is part of the graph, as the groups' is.)
-static int operand_apart(dwim_b200_ctx *ctx, dwim_b200_buffer *x, size_t cols, size_t n, int split, const __half **operand) {
+// Where the operand of n tokens goes for a product that takes it in pieces if it must: the shadow where it fits (the
+// shadow is not made longer for it: graphs captured with other forms in it would read freed memory), else an array of
+// its own, for whatever the buffer can hold of such rows: DENSE_FEW of the longest that up to DENSE_ROWS activations can
+// be (3.3 MB), or all of longer ones.  That is allocated under a stream capture as well, so that a captured product
+// takes no more launches than another.  When memory is short: the largest array there is, of eight tokens at least.
+static int operand_room(dwim_b200_ctx *ctx, dwim_b200_buffer *x, size_t cols, size_t n, int split, void **place, size_t *bytes) {
     const size_t need = gemm_operand_bytes(cols, n, split);
-    *operand = nullptr;
-    const bool fits = need <= x->shadow_cap;
-    for (int kind : {SHADOW_GEMM, SHADOW_GEMM_APART})
-        if (shadow_holds(ctx, x, kind, cols, split)) {
-            *operand = (const __half *)(kind == SHADOW_GEMM ? x->shadow : x->groups);
-            return 0;
+    const int i = cols > DENSE_ROWS;
+    if (need > x->shadow_cap && !x->operands_tried[i]) {
+        x->operands_tried[i] = true;
+        const size_t most = i || x->cap < DENSE_FEW * DENSE_ROWS ? x->cap : DENSE_FEW * DENSE_ROWS;
+        // (16 bytes more than rows of 256, which have the most tokens, add up to)
+        const size_t want = gemm_operand_bytes(256, most / 256, 1) + 16;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        DWIM_CUDA(ctx, cudaThreadExchangeStreamCaptureMode(&mode));
+        if (cudaMalloc(&x->operands[i], want) == cudaSuccess) {
+            x->operands_cap[i] = want;
+        } else {
+            x->operands[i] = nullptr;
+            cudaGetLastError();
         }
-    if (!fits) {
-        reserve_groups(ctx, x, cols, panel_i8_bytes(cols, I8_MAX_TOKENS));
-        if (need > x->groups_cap) return 0;
+        DWIM_CUDA(ctx, cudaThreadExchangeStreamCaptureMode(&mode));
     }
-    void *place = fits ? x->shadow : x->groups;
-    x->shadow_kind = SHADOW_NONE;
-    int rc = build_gemm_operand(ctx, x->data, n, cols, split, (__half *)place);
+    size_t best = x->shadow_cap;
+    *place = x->shadow;
+    if (need > best)
+        for (int k : {i, 2, 1 - i}) {
+            const size_t cap = k == 2 ? x->groups_cap : x->operands_cap[k];
+            if (best < need && cap > best) best = cap, *place = k == 2 ? x->groups : x->operands[k];
+        }
+    const size_t least = gemm_operand_bytes(cols, capture_id(ctx) ? 1 : n < I8_MAX_TOKENS ? n : I8_MAX_TOKENS, split);
+    if (best < least) {
+        int rc = reserve_shadow(ctx, x, least);
+        if (rc) return rc;
+        best = x->shadow_cap;
+        *place = x->shadow;
+    }
+    *bytes = best;
+    return 0;
+}
+
+// A product that the groups of eight tokens could take as well, by the dense kernel.  Its bits are the same however
+// many pieces the tokens are taken in: a token's sums depend on how many blocks share a tile, and that is chosen for the
+// whole product.
+static int product_apart(dwim_b200_ctx *ctx, const WeightView &v, dwim_b200_buffer *x, size_t n, const OutSpec &out, const float *aux,
+                         int epilogue) {
+    const int split = 1, own = v.cols > DENSE_ROWS;
+    const bool in_shadow = shadow_holds(ctx, x, SHADOW_GEMM, v.cols, split);
+    if (in_shadow || shadow_holds(ctx, x, SHADOW_GEMM_APART, v.cols, split))
+        return gemm_large(ctx, v, (const __half *)(in_shadow ? x->shadow : x->operands[own]), n, 1 + split, out, aux, epilogue, n);
+    void *place;
+    size_t bytes;
+    int rc = operand_room(ctx, x, v.cols, n, split, &place, &bytes);
     if (rc) return rc;
-    shadow_made(ctx, x, fits ? SHADOW_GEMM : SHADOW_GEMM_APART, cols, split);
-    *operand = (const __half *)place;
+    size_t piece = n;
+    if (gemm_operand_bytes(v.cols, n, split) > bytes) {
+        // 16 bytes of alignment at most besides a token's own
+        piece = (bytes - 16) / (gemm_operand_bytes(v.cols, 4, split) / 4);
+        if (piece < 1) piece = 1;
+        if (piece > DENSE_FEW) piece -= piece % DENSE_FEW;      // whole tiles
+    }
+    const bool kept = piece == n && (place == x->shadow || place == x->operands[own]);
+    x->shadow_kind = SHADOW_NONE;
+    if (!kept) shadow_made(ctx, x, SHADOW_NONE, 0, 0);
+    for (size_t t0 = 0; t0 < n; t0 += piece) {
+        const size_t nt = n - t0 < piece ? n - t0 : piece;
+        rc = build_gemm_operand(ctx, x->data + t0 * v.cols, nt, v.cols, split, (__half *)place);
+        if (rc) return rc;
+        if (kept) shadow_made(ctx, x, place == x->shadow ? SHADOW_GEMM : SHADOW_GEMM_APART, v.cols, split);
+        OutSpec to = out;
+        for (int p = 0; p < out.world; p++) to.dst[p] += t0 * out.pitch;
+        rc = gemm_large(ctx, v, (const __half *)place, nt, 1 + split, to, aux ? aux + t0 * v.rows : nullptr, epilogue, n);
+        if (rc) return rc;
+    }
     return 0;
 }
 
@@ -572,16 +618,10 @@ static int product(dwim_b200_ctx *ctx, const OutSpec &out, size_t out_len, const
     // bf16 activations are exact in one f16 term; f32 ones travel as two (value and rounding remainder).
     const int split = x->bf16_exact || ctx->act_f16 ? 0 : 1;
     if (gemm_takes(v, n, 1 + split)) {
-        const __half *operand;
-        int rc;
-        if (v.fmt != Q4_K && split && (n <= 64 || v.cols > 12288)) {
-            rc = operand_apart(ctx, x, v.cols, n, split, &operand);
-        } else {
-            rc = ensure_shadow(ctx, x, SHADOW_GEMM, v.cols, split);
-            operand = (const __half *)x->shadow;
-        }
+        if (v.fmt != Q4_K && split && (n <= DENSE_FEW || v.cols > DENSE_ROWS)) return product_apart(ctx, v, x, n, out, aux, epilogue);
+        int rc = ensure_shadow(ctx, x, SHADOW_GEMM, v.cols, split);
         if (rc) return rc;
-        if (operand) return gemm_large(ctx, v, operand, n, split ? 2 : 1, out, aux, epilogue);
+        return gemm_large(ctx, v, (const __half *)x->shadow, n, 1 + split, out, aux, epilogue, n);
     }
     if (!gemv_takes_i8(v, n < (size_t)I8_MAX_TOKENS ? n : (size_t)I8_MAX_TOKENS))
         return fail(ctx, DWIM_B200_EFORMAT, "%s: no kernel takes format %d with %zu columns", what, v.fmt, v.cols);
@@ -603,8 +643,7 @@ static int product(dwim_b200_ctx *ctx, const OutSpec &out, size_t out_len, const
         if (groups > room) groups = room;
     }
     uint8_t *const panels = (uint8_t *)(groups * group > x->shadow_cap ? x->groups : x->shadow);
-    if (panels == x->shadow || x->shadow_kind == SHADOW_GEMM_APART) shadow_made(ctx, x, SHADOW_NONE, 0, 0);
-    else if (capture_id(ctx)) x->replayed.kind = SHADOW_MIXED;
+    if (panels == x->shadow) shadow_made(ctx, x, SHADOW_NONE, 0, 0);
     for (size_t t0 = 0; t0 < n;) {
         const size_t left = n - t0, g = left < (size_t)I8_MAX_TOKENS ? 1 : left / I8_MAX_TOKENS < groups ? left / I8_MAX_TOKENS : groups;
         const size_t nt = left < (size_t)I8_MAX_TOKENS ? left : (size_t)I8_MAX_TOKENS;

@@ -17,7 +17,7 @@ enum ShadowKind : int {
     SHADOW_NONE = 0,
     SHADOW_GEMM,            // f16 rows, sub-block means and token scales, for the tensor-core kernels
     SHADOW_PANEL_I8,        // int8 digit planes per 256-wide unit, for the small-M kernel
-    SHADOW_GEMM_APART       // as SHADOW_GEMM, in the groups' array
+    SHADOW_GEMM_APART       // as SHADOW_GEMM, in an array of its own (operands)
 };
 
 // What graphs make of a buffer: nothing, one form of its contents, or several (SHADOW_MIXED).
@@ -50,11 +50,16 @@ struct dwim_b200_buffer {
     int shadow_split = 0;        // f16 terms of an activation less one
     unsigned long long shadow_capture = 0;   // the stream capture that the conversion is part of; 0: it was launched
     ShadowForm replayed;         // what captured graphs make there whenever they run
-    // The digit planes of several groups of eight tokens, or the dense kernel's operand (products of Q6_K and Q8_0 by
-    // nine tokens and more), where the shadow holds less.  Allocated once and kept to the buffer's end.
+    // The digit planes of several groups of eight tokens (products of Q6_K and Q8_0 by nine tokens and more), where the
+    // shadow holds fewer.  Allocated once and kept to the buffer's end.
     void *groups = nullptr;
     size_t groups_cap = 0;       // bytes
     bool groups_tried = false;
+    // The dense kernel's operand where the shadow is shorter and must stay as it is (operand_room): of rows of up to
+    // DENSE_ROWS activations, and of longer ones.  Allocated once each and kept to the buffer's end.
+    void *operands[2] = {};
+    size_t operands_cap[2] = {};
+    bool operands_tried[2] = {};
 };
 
 struct dwim_b200_weight {
@@ -207,6 +212,9 @@ int build_panels_i8(dwim_b200_ctx *ctx, const float *x, size_t n, size_t cols, u
 // Tokens above which the tensor-core GEMM takes over from the small-M kernel (for the formats it takes).
 constexpr size_t DWIM_SMALL_M_MAX = I8_MAX_TOKENS;
 size_t gemm_operand_bytes(size_t cols, size_t n, int split);
+// The dense kernel's products that drain every K block: by f32 activations, up to DENSE_FEW tokens, or rows of more
+// than DENSE_ROWS (gemm_takes).
+constexpr size_t DENSE_FEW = 64, DENSE_ROWS = 12288;
 int build_gemm_operand(dwim_b200_ctx *ctx, const float *x, size_t n, size_t cols, int split, __half *out,
                        const float *weight = nullptr, float eps = 0.0f, float *xout = nullptr);
 

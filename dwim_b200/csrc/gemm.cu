@@ -1069,7 +1069,7 @@ template <int FMT, int BN, int MODE> double dense_time(dwim_b200_ctx *ctx, const
 
 template <int FMT, int BN, int MODE>
 int launch_dense(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, size_t n, int terms, const OutSpec &out, const float *aux,
-                 int epi) {
+                 int epi, size_t whole) {
     using C = DenseCfg<FMT, BN, MODE>;
     const size_t units = w.cols / 256;
     CUtensorMap tw, tx;
@@ -1089,7 +1089,7 @@ int launch_dense(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand,
     if ((rc = configure_gemm(ctx, kern, C::SMEM, GEMM_THREADS, 512 * DENSE_WORKER_REGS + 128 * DENSE_OTHER_REGS, configured[ctx->device & 63][shared]))) return rc;
     dim3 grid((unsigned)((w.rows + TILE_M - 1) / TILE_M), (unsigned)((n + BN - 1) / BN));
     if (!shared) {
-        a.split_k = dense_split<FMT, BN, MODE>(ctx, w, n, terms);
+        a.split_k = dense_split<FMT, BN, MODE>(ctx, w, whole, terms);
         grid.x *= a.split_k;
     }
     const bool dependent = !ctx->weights_written;   // see dwim_b200_ctx::weights_written
@@ -1115,12 +1115,13 @@ constexpr size_t DENSE_FROM[2] = {65, 25};      // tokens, by one and two terms
 bool gemm_takes(const WeightView &w, size_t n, int terms) {
     if (w.cols % 256) return false;
     if (w.fmt == Q4_K) return n > (size_t)I8_MAX_TOKENS;
-    return (w.fmt == Q6_K || w.fmt == Q8_0) && n >= DENSE_FROM[terms - 1] && w.cols <= (terms == 2 ? 51200 : 12288);
+    return (w.fmt == Q6_K || w.fmt == Q8_0) && n >= DENSE_FROM[terms - 1] && w.cols <= (terms == 2 ? 51200 : DENSE_ROWS);
 }
 
+// `whole`: the tokens of the product that these are a piece of (the forms drained every K block may be taken in pieces).
 int gemm_large(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, size_t n, int terms, const OutSpec &out,
-               const float *aux, int epilogue) {
-    if (!gemm_takes(w, n, terms)) return fail(ctx, DWIM_B200_EFORMAT, "the tensor-core GEMM does not take format %d, %zu tokens", w.fmt, n);
+               const float *aux, int epilogue, size_t whole) {
+    if (!gemm_takes(w, whole, terms)) return fail(ctx, DWIM_B200_EFORMAT, "the tensor-core GEMM does not take format %d, %zu tokens", w.fmt, whole);
     if (w.fmt == Q4_K) {
         // (at 33 tokens and more a tile of 64 columns: tensor memory holds four groups' sums of 32)
         if (n <= 32 && (out.world == 1 || out.scatter_per)) return gemm_few(ctx, w, operand, n, terms, out, aux, epilogue);
@@ -1143,16 +1144,16 @@ int gemm_large(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, s
     // few tokens, or long rows: drained every K block, for the groups' precision (gemm_takes)
     auto dense = [&](auto fmt) {
         constexpr int F = decltype(fmt)::value;
-        if (n <= 64 || w.cols > 12288)
-            return launch_dense<F, 64, TWO_PASSES>(ctx, w, operand, n, terms, out, aux, epilogue);
-        if (n <= 128) return launch_dense<F, 128, SIDE_BY_SIDE>(ctx, w, operand, n, terms, out, aux, epilogue);
+        if (whole <= DENSE_FEW || w.cols > DENSE_ROWS)
+            return launch_dense<F, 64, TWO_PASSES>(ctx, w, operand, n, terms, out, aux, epilogue, whole);
+        if (n <= 128) return launch_dense<F, 128, SIDE_BY_SIDE>(ctx, w, operand, n, terms, out, aux, epilogue, whole);
         // Tiles of 192 or 256 columns by their waves, as Q4_K's: [12288, 5120] Q6_K by 192 f32 tokens 128 us in tiles of 256,
         // 100 of 192, by 384 206 and 165, by 256 129 and 166; [5120, 5120] Q8_0 by 130 52 and 40, by bf16 ones 31 and 29.
         auto wide = [&](auto mode) {
             constexpr int M = decltype(mode)::value;
             if (0.82 * dense_time<F, 192, M>(ctx, w, n, terms) < dense_time<F, 256, M>(ctx, w, n, terms))
-                return launch_dense<F, 192, M>(ctx, w, operand, n, terms, out, aux, epilogue);
-            return launch_dense<F, 256, M>(ctx, w, operand, n, terms, out, aux, epilogue);
+                return launch_dense<F, 192, M>(ctx, w, operand, n, terms, out, aux, epilogue, whole);
+            return launch_dense<F, 256, M>(ctx, w, operand, n, terms, out, aux, epilogue, whole);
         };
         return terms == 1 ? wide(std::integral_constant<int, ONE_TERM>()) : wide(std::integral_constant<int, TWO_PASSES>());
     };

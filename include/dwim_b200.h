@@ -193,12 +193,17 @@ DWIM_B200_API int dwim_b200_quantize(dwim_b200_ctx *ctx, int fmt, size_t rows, s
  * n = len(x)/cols rows of x; len(out) must be n * rows.
  * The buffer x keeps device memory for the operand form of its contents, from
  * the first product that needs as much: up to 4.3 bytes per activation.  Of
- * Q6_K and Q8_0 products through groups of eight tokens it keeps, besides, as
- * many groups' int8 digit planes as it can hold, up to 64 of them (6624 bytes
- * per group and 256 columns: 3.3 bytes per activation, at most 28 MB at 17408
- * columns): allocated at the first such product outside a stream capture and
- * kept.  Without it -- under a capture, or when memory is short -- the product
- * takes more launches and gives the same bits. */
+ * Q6_K and Q8_0 products by nine tokens and more it keeps, besides, what does
+ * not fit there, each array allocated by the first product that asks and kept:
+ *   - of those through groups of eight tokens, as many groups' int8 digit
+ *     planes as it can hold, up to 64 of them (6624 bytes per group and 256
+ *     columns: 3.3 bytes per activation, at most 28 MB at 17408 columns); not
+ *     allocated under a stream capture;
+ *   - of those by f32 activations of 25 to 64 tokens their f16 operand (at most
+ *     3.3 MB), and of those by f32 rows above 12288 columns theirs (4.2 bytes per
+ *     activation that the buffer can hold: 147 MB for [2048, 17408]).
+ * Without such an array -- under a capture, the first; when memory is short --
+ * the product takes more launches and gives the same bits. */
 DWIM_B200_API int dwim_b200_matmul(dwim_b200_ctx *ctx, dwim_b200_buffer *out,
                                    const dwim_b200_weight *w, dwim_b200_buffer *x);
 /* Device::matmul_add (gpu/mod.rs:256-268): x += w . input.  `scratch` is as

@@ -1147,6 +1147,68 @@ def test_a_captured_conversion_is_not_taken_for_a_made_one(oracle, fmt, n):
         d.close()
 
 
+@pytest.mark.parametrize("fmt", ["q6_k", "q8_0"])
+def test_dense_kernel_gives_its_bits_whatever_memory_there_is(oracle, fmt):
+    """The products that the groups of eight tokens could take as well: captured before any eager one, by a buffer that
+    was read as rows of another length first, and by one whose operand does not fit the device (a buffer of which the
+    caller says that it is longer than any memory; a few rows are used), in as many launches as it takes."""
+    import torch
+    from dwim_b200 import B200, Tensor
+    stream = torch.cuda.Stream()
+    d = B200(0, stream=stream.cuda_stream)
+    try:
+        rng = np.random.default_rng(83)
+        n, short, long = 70, 1024, 12544
+        rows, tokens = {short: 96, long: 300}, {short: 64, long: n}
+        blocks = {c: d.quantize(fmt, (0.02 * rng.standard_normal((rows[c], c))).astype(np.float32)).data for c in rows}
+        weight = {c: d.upload(Tensor(fmt, (rows[c], c), blocks[c])) for c in rows}
+        x = rng.standard_normal(n * long).astype(np.float32)
+
+        def product(xb, c, graph=False):
+            d.resize(xb, tokens[c] * c)
+            d.write(xb, x[:tokens[c] * c])
+            out = d.buffer(rng.standard_normal(tokens[c] * rows[c]).astype(np.float32))
+            launches = d.launches
+            if graph:
+                g = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(g, stream=stream):
+                    d.matmul(out, weight[c], xb)
+                with torch.cuda.stream(stream):
+                    g.replay()
+                    stream.synchronize()
+                del g
+            else:
+                d.matmul(out, weight[c], xb)
+            return d.read(out), d.launches - launches
+
+        want = {c: product(d.alloc(n * long), c)[0] for c in rows}
+        for c in rows:
+            w = oracle.dequantize(fmt, blocks[c], rows[c], c).reshape(rows[c], c).astype(np.float64)
+            y = x[:tokens[c] * c].reshape(-1, c).astype(np.float64) @ w.T
+            assert np.linalg.norm(want[c].reshape(y.shape) - y) <= 3e-7 * np.linalg.norm(y)
+            got, launches = product(d.alloc(n * long), c, graph=True)
+            assert np.array_equal(got, want[c]) and launches == 2, "captured first"
+        for order in ((short, long), (long, short)):
+            xb = d.alloc(n * long)
+            for c in order:
+                got, launches = product(xb, c)
+                assert np.array_equal(got, want[c]) and launches == 2, order
+        with torch.cuda.stream(stream):
+            real = torch.zeros(n * long, device="cuda")
+        xb = d.wrap(real.data_ptr(), 1 << 36)
+        got, launches = product(xb, long)
+        assert np.array_equal(got, want[long]) and launches > 2, "no room for the operand"
+        # an addend and a second product's values in the same pieces
+        res, gated, scratch = d.buffer(want[long]), d.alloc(n * rows[long]), d.alloc(n * rows[long])
+        d.matmul_add(res, weight[long], xb)
+        assert np.array_equal(d.read(res), want[long] + want[long])
+        d.swiglu(gated, weight[long], weight[long], xb, scratch)
+        assert max_rel_err(d.read(gated), silu_times(want[long].astype(np.float64), want[long])) <= 1e-5
+        del xb
+    finally:
+        d.close()
+
+
 @pytest.mark.parametrize("fmt,n", [("q4_k", 16), ("q4_k", 40), ("q4_k", 150), ("q6_k", 40), ("q6_k", 80), ("q6_k", 150), ("q8_0", 40), ("q8_0", 150)])
 def test_gemm_activations_at_the_ends_of_f32(dev, oracle, fmt, n):
     """Rows whose largest activation is near the ends of f32's exponents: the token's power of two reaches both, so that
