@@ -230,17 +230,24 @@ def test_small_m_row_tiles_and_boxes(dev, oracle, fmt, rows, cols):
         assert np.abs(dev.read(out).reshape(n, rows) - silu).max() <= 4 * bar * max(1.0, np.abs(want).max()), n
 
 
+@pytest.mark.parametrize("bf16", [False, True])
 @pytest.mark.parametrize("fmt,rows,cols,n", [("q8_0", 100, 96, 530), ("q8_0", 300, 5120, 64), ("q8_0", 33, 2048, 17), ("q6_k", 2400, 768, 23),
-                                             ("q6_k", 40, 6144, 41), ("q8_0", 16, 32, 9)])
-def test_groups_of_eight_tokens(dev, oracle, fmt, rows, cols, n):
-    """Full groups in one launch (up to 64 of them), the rest in another; every token against the oracle's
-    weights in double precision, 1e-5 of the result's root mean square as for eight tokens."""
+                                             ("q6_k", 40, 6144, 41), ("q8_0", 16, 32, 9), ("q6_k", 48, 12544, 70)])
+def test_groups_of_eight_tokens(dev, oracle, fmt, rows, cols, n, bf16):
+    """Full groups in one launch (up to 64 of them), the rest in another (by f32 activations of 25 tokens and more, rows of
+    whole units: the dense kernel); every token against the oracle's weights in double precision, 1e-5 of the result's
+    root mean square as for eight tokens."""
     rng = np.random.default_rng(rows + n)
     weight, w, _, _ = random_pair(dev, oracle, fmt, rows, cols, rng)
     x = rng.standard_normal((n, cols)).astype(np.float32)
+    xb = dev.buffer(x)
+    if bf16:
+        bits = oracle.to_bf16(x)
+        dev.write_bf16(xb, bits)
+        x = oracle.bf16(bits).reshape(n, cols)
     want = x.astype(np.float64) @ w.T
     res = rng.standard_normal((n, rows)).astype(np.float32)
-    xb, out, acc = dev.buffer(x), dev.alloc(n * rows), dev.buffer(res)
+    out, acc = dev.alloc(n * rows), dev.buffer(res)
     bar = 1e-5 * np.sqrt((want ** 2).mean())
     dev.matmul(out, weight, xb)
     assert np.abs(dev.read(out).reshape(n, rows) - want).max() <= bar
@@ -248,10 +255,12 @@ def test_groups_of_eight_tokens(dev, oracle, fmt, rows, cols, n):
     assert np.abs(dev.read(acc).reshape(n, rows) - (want + res)).max() <= bar + 1e-6
 
 
-def test_groups_under_capture(oracle):
+@pytest.mark.parametrize("bf16", [False, True])
+def test_groups_under_capture(oracle, bf16):
     """A product of more than eight tokens captured into a CUDA graph after a warm-up at another token count
     (the buffer resized between): no allocation is needed there, and none made later takes away what a captured
-    graph reads.  Every token as the eager product gives it."""
+    graph reads.  Every token as the eager product gives it.  (By f32 activations the longer ones are the dense
+    kernel's.)"""
     import torch
     from dwim_b200 import B200, Tensor
     stream = torch.cuda.Stream()
@@ -262,6 +271,8 @@ def test_groups_under_capture(oracle):
         blocks = oracle.quantize("q8_0", (0.02 * rng.standard_normal((rows, cols))).astype(np.float32))
         weight = d.upload(Tensor("q8_0", (rows, cols), blocks))
         x = rng.standard_normal((most, cols)).astype(np.float32)
+        if bf16:
+            x = oracle.bf16(oracle.to_bf16(x)).reshape(most, cols)
         want = oracle.matmul("q8_0", blocks, rows, cols, x).reshape(most, rows)
         xb, out = d.buffer(x), d.alloc(most * rows)
 
@@ -281,12 +292,14 @@ def test_groups_under_capture(oracle):
                 d.matmul(out, weight, xb)
             return graph
 
+        if bf16:
+            d.touch_bf16(xb)
         at(8)
         d.matmul(out, weight, xb)
         assert right(8)
         graphs = {n: captured(n) for n in (most, 16)}
         at(most)
-        d.matmul(out, weight, xb)                       # eager: the planes of all its groups at once
+        d.matmul(out, weight, xb)                       # eager: the planes of all its groups at once, or the operand
         assert right(most)
         graphs[24] = captured(24)
         for n, graph in list(graphs.items()) * 2:
@@ -300,12 +313,13 @@ def test_groups_under_capture(oracle):
 
 
 @pytest.mark.parametrize("bf16", [False, True])
-def test_q4_k_gemm_scale_extremes(dev, oracle, bf16):
+@pytest.mark.parametrize("n", [40, 9, 16, 32, 130])
+def test_q4_k_gemm_scale_extremes(dev, oracle, n, bf16):
     """The tensor-core kernel folds a block's minimums into the same accumulator
     as its quants, scaled by dmin/d: rows whose blocks have d = 0, dmin = 0, either
     sign, or dmin up to 2^40 times d must still match the CPU result."""
     rng = np.random.default_rng(47)
-    rows, cols, n = 256, 1024, 40
+    rows, cols = 256, 1024
     blocks = oracle.quantize("q4_k", (0.02 * rng.standard_normal((rows, cols))).astype(np.float32)).copy()
     regimes = [(1e-3, 2e-3), (0.0, 0.05), (0.05, 0.0), (0.0, 0.0), (1e-3, 0.1), (1e-4, 6.0), (2.4e-7, 30.0),
                (6e-8, 60000.0), (-1e-3, 2e-3), (1e-3, -2e-3), (3e-5, 1.0), (1.0, 6e-8)]
@@ -957,13 +971,14 @@ def test_chunks_and_shards_agree_with_the_whole(dev, oracle, fmt, n, cut):
 
 
 @pytest.mark.parametrize("fmt", ["q6_k", "q8_0"])
-def test_dense_kernel_scale_extremes(dev, oracle, fmt):
+@pytest.mark.parametrize("n", [80, 40, 150])
+def test_dense_kernel_scale_extremes(dev, oracle, fmt, n):
     """Block scales over f16's range within a unit (Q8_0's power of two), sub-scales at both ends (Q6_K's
     13-bit products), zero scales, signed ones: random bit patterns with finite scales, against the decoded
     weights in double precision, per row."""
     from dwim_b200 import Tensor
     rng = np.random.default_rng(5)
-    rows, cols, n = 200, 1024, 80
+    rows, cols = 200, 1024
     size = 34 if fmt == "q8_0" else 210
     blocks = rng.integers(0, 256, (rows, cols // (32 if fmt == "q8_0" else 256), size), dtype=np.uint8)
     exponent = rng.integers(0, 31, blocks.shape[:2])
