@@ -273,6 +273,7 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
         const int quad = warp & 3;
         const int g = warp >> 2;
         const int rl = quad * 32 + lane;                // row within the tile = TMEM lane
+        static_assert(C::DRAINERS == 4 || OUT != 0, "a split tile's blocks meet in every worker");
         const bool drains = g < C::DRAINERS;
         const uint32_t drain_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + g * C::DRAIN_COLS;
         const uint32_t a_row_sw = (astage0 + rl * 128) | ((rl & 7) << 4);
@@ -425,10 +426,6 @@ gemm_q4k_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
                     gemm_emit<SHARED>(to, rows, n, cbase + j, v);
                 }
             }
-        }
-        if (!drains && split_k > 1) {
-            cluster_sync();
-            cluster_sync();
         }
     } else {
         if constexpr (TRADE) regs_dec<OTHER_REGS>();      // (a warpgroup's warps at one instruction)
