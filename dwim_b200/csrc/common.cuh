@@ -83,7 +83,7 @@ struct dwim_b200_ctx {
     // (an upload's repack): that launch must be an ordinary one, because a
     // programmatic dependent streams weights before it waits for the kernels ahead.
     bool weights_written = false;
-    // 1: f32 activations go to the tensor-core kernels as one f16 column (dwim_b200_activation_precision)
+    // 1: f32 activations go to the tensor-core kernels as one f16 term (dwim_b200_activation_precision)
     int act_f16 = 0;
     // argmax's keys, a block's each (pinned host memory the kernel writes; neighbours.cu), created on request
     unsigned long long *argmax_host = nullptr;

@@ -13,7 +13,7 @@
 // is applied by CUDA cores in fp32.  The first sum's products are exact; the
 // second's factors travel as f16 value + rounding remainder on both sides (22
 // bits each), and a power of two moves between d and the operands when dmin/d
-// is large (q4k_fold below).  The reference's tile kernel rounds every
+// is large (q4k_fold, gemm.cuh).  The reference's tile kernel rounds every
 // dequantized weight to f16 instead (matmul_tile.cu:66-74): 2e-4 of rms error
 // against 5e-7 here.  An f32 activation travels as two f16 terms, value and
 // rounding remainder; a bf16 one is exact in one.  The terms share a token's
@@ -46,8 +46,8 @@
 //                 blocks [128 rows][144 B] from HBM into the raw ring.
 // Where the tiles do not fill the chip, a cluster's blocks share a tile's K and add up
 // through each other's shared memory (pick_split).
-// Warp 19 makes whole warpgroups of them, which trade registers: 96 a thread at launch,
-// 104 for a worker then.  (At 96 the 256-column form spilled in its main loop: [17408,
+// Warp 19 makes whole warpgroups of them, which trade registers at 256 columns: 96 a thread
+// at launch, 104 for a worker then.  (At 96 the 256-column form spilled in its main loop: [17408,
 // 5120] by 2048 bf16 tokens 391 us, 375 like this; with 100 bytes of spills 442.)
 // Every mbarrier wait is bounded (ptx.cuh); a kernel that gave up says so in
 // the context's status word.
@@ -753,7 +753,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 const uint4 sc = fetch(u);
                 const int r = C::RAW_STEPS == 2 ? 2 * u + (g >> 1) : u, rs = r % C::RAW_STAGES;
                 mbar_wait_parked(rawfull0 + 8 * rs, (r / C::RAW_STAGES) & 1, a.status, 0x4000000u);
-    // the stage's last user is done: the K block of the unit before, or with two stages (this warp has waited for
+                // the stage's last user is done: the K block of the unit before, or with two stages (this warp has waited for
                 // the use before that one) the one two K blocks back
                 if (C::A_STAGES == KBLOCKS) mbar_wait_parked(adone0 + 8 * g, (u & 1) ^ 1, a.status, 0x8000000u);
                 else mbar_wait_parked(adone0 + 8 * (g ^ 2), (u & 1) ^ (g < 2 ? 1 : 0), a.status, 0x8000000u);
@@ -980,8 +980,8 @@ template <int BN, int MODE>
 int gemm_split(dwim_b200_ctx *ctx, const WeightView &w, size_t n, int terms, double *time = nullptr) {
     static std::atomic<int> known[64][MAX_SPLIT + 1] = {};
     const long tiles = (long)((w.rows + TILE_M - 1) / TILE_M) * (long)((n + BN - 1) / BN);
-    return pick_split(ctx, gemm_q4k_kernel<BN, 0, MODE>, GEMM_THREADS, (size_t)Cfg<BN, MODE>::SMEM, Cfg<BN, MODE>::split_fits, SplitCost{3.0, 6.5}, known, tiles,
-                      (int)(w.cols / 256), q4k_unit(BN, terms), time);
+    return pick_split(ctx, gemm_q4k_kernel<BN, 0, MODE>, GEMM_THREADS, (size_t)Cfg<BN, MODE>::SMEM, Cfg<BN, MODE>::split_fits,
+                      SplitCost{3.0, 6.5}, known, tiles, (int)(w.cols / 256), q4k_unit(BN, terms), time);
 }
 template <int BN, int MODE> double gemm_time(dwim_b200_ctx *ctx, const WeightView &w, size_t n, int terms) {
     double t = 0;
@@ -1034,7 +1034,8 @@ int launch_gemm(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, 
         if (shared == 1) kern = gemm_q4k_kernel<BN, 1, MODE>;
     }
     static std::atomic<bool> configured[64][3] = {};
-    if ((rc = configure_gemm(ctx, kern, C::SMEM, GEMM_THREADS, C::TRADE ? 512 * WORKER_REGS + 128 * OTHER_REGS : 0, configured[ctx->device & 63][shared]))) return rc;
+    constexpr int SHARES = C::TRADE ? 512 * WORKER_REGS + 128 * OTHER_REGS : 0;
+    if ((rc = configure_gemm(ctx, kern, C::SMEM, GEMM_THREADS, SHARES, configured[ctx->device & 63][shared]))) return rc;
     dim3 grid((unsigned)((w.rows + TILE_M - 1) / TILE_M), (unsigned)((n + BN - 1) / BN));
     if constexpr (ONE) {
         if (!shared) {
@@ -1083,7 +1084,8 @@ int launch_dense(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand,
     const bool shared = out.world > 1 && !out.scatter_per;
     auto kern = shared ? gemm_dense_kernel<FMT, BN, MODE, true> : gemm_dense_kernel<FMT, BN, MODE, false>;
     static std::atomic<bool> configured[64][2] = {};
-    if ((rc = configure_gemm(ctx, kern, C::SMEM, GEMM_THREADS, 512 * DENSE_WORKER_REGS + 128 * DENSE_OTHER_REGS, configured[ctx->device & 63][shared]))) return rc;
+    constexpr int SHARES = 512 * DENSE_WORKER_REGS + 128 * DENSE_OTHER_REGS;
+    if ((rc = configure_gemm(ctx, kern, C::SMEM, GEMM_THREADS, SHARES, configured[ctx->device & 63][shared]))) return rc;
     dim3 grid((unsigned)((w.rows + TILE_M - 1) / TILE_M), (unsigned)((n + BN - 1) / BN));
     if (!shared) {
         a.split_k = dense_split<FMT, BN, MODE>(ctx, w, whole, terms);

@@ -203,9 +203,9 @@ __device__ __forceinline__ void mins_q4k_terms(const uint4 &hdr, int part, float
 // Blocks that share a tile's K.  A block is alone on its SM, so tiles run in waves of as many
 // clusters as the device holds; a wave lasts a block's units and what a tile costs besides, in units:
 // three for ramp and epilogue, six and a half with the exchange (fitted to every split from 1 to 8 of
-// six shapes by 16 to 2048 tokens; the choice is within 3 % of the best of them but for [1024, 5120] by
-// 2048).  Without it 40 tiles left 108 of 148 SMs idle: [5120, 17408] by 16 tokens 85 us, 39 with three
-// blocks a tile; by 131 bf16 tokens 134 and 67; by 512 f32 tokens (160 tiles) 299 and 236.
+// six shapes by 48 to 2048 tokens; the choice is within 3 % of the best of them but for [1024, 5120] by
+// 2048).  Without it 40 tiles left 108 of 148 SMs idle: [5120, 17408] by 131 bf16 tokens 134 us, 67 with three
+// blocks a tile; by 512 f32 tokens (160 tiles) 299 and 236.  The few-token kernel's use of it: gemm_few.cu.
 // The dense kernel's units are twice as long, so a tile's other costs are fewer of them: two, and four and
 // a half with the exchange.  Over every split of twelve products (rows 1024 to 17408, K 5120 and 12288, 80 to 2048
 // tokens) the choice is within 3 % of the best, but for [5120, 5120] by 131 f32 tokens (63.6 us alone, 60.4 by three).

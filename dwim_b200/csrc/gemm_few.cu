@@ -432,9 +432,14 @@ int launch_few(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, s
     FewArgs a{w.rows, n, units, terms, epi, 1, out, tok_scale, aux, ctx->status};
     auto kern = gemm_few_kernel<N>;
     static std::atomic<bool> configured[64] = {};
-    if ((rc = configure_gemm(ctx, kern, C::SMEM, FEW_THREADS, 512 * FEW_WORKER_REGS + 256 * FEW_OTHER_REGS, configured[ctx->device & 63]))) return rc;
+    constexpr int SHARES = 512 * FEW_WORKER_REGS + 256 * FEW_OTHER_REGS;
+    if ((rc = configure_gemm(ctx, kern, C::SMEM, FEW_THREADS, SHARES, configured[ctx->device & 63]))) return rc;
     static std::atomic<int> known[64][MAX_SPLIT + 1] = {};
     const long tiles = (long)((w.rows + TILE_M - 1) / TILE_M);
+    // The prices of gemm.cu's kernel hold for this one: of the splits from 1 to 8 of ten shapes, by 9, 16 and 32 tokens in
+    // one and two terms, the choice is within 2 % of the best for eight ([10240, 5120] by 16 17.1 us alone, 23.8 by two
+    // blocks; [6144, 5120] 15.8 and 12.7; [5120, 17408] 43.4, 26.4 and 20.9 by three), and a block too far where the
+    // tiles are few: [1024, 5120] takes seven for 7.7 us where five and six take 7.0, [3000, 2048] four for 7.8, two 7.5.
     a.split_k = pick_split(ctx, kern, FEW_THREADS, (size_t)C::SMEM, C::split_fits, SplitCost{3.0, 6.5}, known, tiles, (int)units, 1.0);
     const bool dependent = !ctx->weights_written;   // see dwim_b200_ctx::weights_written
     DWIM_CUDA(ctx, launch_clustered(dependent, (unsigned)a.split_k, kern, dim3((unsigned)(tiles * a.split_k)), dim3(FEW_THREADS),

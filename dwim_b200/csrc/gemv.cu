@@ -315,7 +315,7 @@ __device__ __forceinline__ void unit_q8_i8(const Lane &L, const I8Cols X, int ul
 // the four sets of four groups, from which nine instructions a set make the groups' bytes,
 // 4 * q each (formats.cuh); d takes the 4 back.  (Bound by issue: with the file's nibbles and bit pairs, twelve
 // 32-bit loads and sixteen instructions, the [151936, 5120] product took 108 us at one token, 131 at two and 201 at
-// eight; 100, 118 and 194 like this.)
+// eight; 100, 118 and 194 like this, 101, 110 and 168 to 174 with launch_shape's row tiles.)
 __device__ __forceinline__ uint32_t word_of(const uint4 &v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 template <int NTILE, bool ONE>
 __device__ __forceinline__ void unit_q6k_i8(const Lane &L, const I8Cols X, int ul, int xu, int d_index, float (&acc)[NTILE == 2 ? 8 : 4]) {
@@ -866,8 +866,8 @@ static int launch_shape(dwim_b200_ctx *ctx, GemvArgs &a) {
     //   Q4_K, one token: [17408, 5120] 15.7 13.4 12.6 12.5, [10240, 5120] 11.1 10.4 8.8 10.2, [6144, 5120] 7.5 7.0 6.8
     //   7.2, [5120, 6144] 7.3 7.9 7.2 8.3, [1024, 5120] 3.4 4.2 5.1 5.8, [5120, 17408] 15.7 19.5 14.6 16.7; five tokens
     //   [17408, 5120] 22.5 19.2 18.6 18.4, [10240, 5120] 14.9 14.0 13.3 16.9, [5120, 17408] 24.6 24.0 16.8 21.5
-    //   Q6_K: the [151936, 5120] head by one 116 106 107 114, by five 232 168 173 156, by eight 230 209 197 180;
-    //   [12288, 5120] by one 12.3 12.1 11.4 13.2, by five 22.8 18.2 18.1 19.3
+    //   Q6_K: the [151936, 5120] head by one 107 99 101, by two 125 112 112, by five 251 171 167 147, by eight 234 211 186
+    //   168; [12288, 5120] by one 12.4 12.3 11.5, by five 22.9 18.4 18.5 19.4
     //   Q8_0: [17408, 2048] by one 12.6 9.5 9.4 8.8, by eight 16.5 11.8 13.8 11.9; [5120, 5120] by eight 14.3 14.7 10.3
     // (with c = 0.3 throughout, [10240, 5120] took one row tile and [17408, 2048] whole rows of one).  Four K-split warps
     // leave a thread more registers than five: Q4_K by one token with three row tiles [10240, 5120] 9.3 us with five,

@@ -134,7 +134,8 @@ __global__ void __launch_bounds__(256) matmul_bf16_kernel(const __grid_constant_
 // tokens 10.6, 10.6, 16, 22 and 24 us; 14, 14, 18, 33 and 41 with one chunk ahead in registers, one
 // group and two barriers a chunk; 10.7, 16, 18, 18 and 33 with four groups; 15, 15, 23, 26 and 27 in
 // tiles of 64 tokens.  (A warp per row and eight tokens took 306 us by 512.)
-constexpr int BT_ROWS = 32, BT_TOK = 32, BT_K = 64, BT_PITCH = BT_K + 4, BT_WPITCH = BT_K + 8, BT_SPLIT = 8, BT_STAGES = 4, BT_GROUPS = 2, BT_THREADS = 128 * BT_GROUPS;
+constexpr int BT_ROWS = 32, BT_TOK = 32, BT_K = 64, BT_PITCH = BT_K + 4, BT_WPITCH = BT_K + 8, BT_SPLIT = 8;
+constexpr int BT_STAGES = 4, BT_GROUPS = 2, BT_THREADS = 128 * BT_GROUPS;
 constexpr int BT_X = BT_TOK * BT_PITCH * 4, BT_W = BT_ROWS * BT_WPITCH * 2, BT_SMEM = BT_STAGES * (BT_X + BT_W);      // a stage's bytes; all
 static_assert(BT_GROUPS * BT_ROWS * BT_TOK * 4 <= BT_STAGES * BT_X, "the partial tiles take the activations' place");
 __device__ __forceinline__ void ffma2_n(uint64_t &d, uint64_t a, uint64_t b) {
@@ -157,7 +158,7 @@ __global__ void __cluster_dims__(BT_SPLIT, 1, 1) __launch_bounds__(BT_THREADS) m
     const size_t chunks = (a.cols + BT_K - 1) / BT_K;
     const size_t c0 = chunks * rank / BT_SPLIT;
     const int n_chunks = (int)(chunks * (rank + 1) / BT_SPLIT - c0);
-    const int rg = tid & 7, tg = (tid >> 3) & 15, kg = tid >> 7;      // rows rg + 8 i, tokens tg + 16 j, quarter kg of a chunk
+    const int rg = tid & 7, tg = (tid >> 3) & 15, kg = tid >> 7;      // rows rg + 8 i, tokens tg + 16 j, half kg of a chunk
     constexpr int TJ = BT_TOK / 16;
     uint64_t acc[4][TJ];
 #pragma unroll
@@ -331,7 +332,7 @@ extern "C" int dwim_b200_normalize(dwim_b200_ctx *ctx, dwim_b200_buffer *out, co
     const size_t n = len / dim;
     if (dim % 256 == 0 && n > DWIM_SMALL_M_MAX && n <= 65535) {
         // more tokens than the small-M kernel takes: the next product is the tensor-core GEMM, whose
-        // operand (f16 value and remainder columns, sub-block means, the token's scale) this launch writes
+        // operand (f16 value and remainder terms, sub-block means, the token's scale) this launch writes
         const int split = ctx->act_f16 ? 0 : 1;
         int rc = reserve_shadow(ctx, out, gemm_operand_bytes(dim, n, split));
         if (rc) return rc;

@@ -178,8 +178,8 @@ int build_panels_i8(dwim_b200_ctx *ctx, const float *x, size_t n, size_t cols, u
     return 0;
 }
 
-// Bytes of the GEMM's operand for n tokens (ncols = n, or 2n when an f32 activation travels as two
-// columns): the f16 rows, the sub-block means, and one f32 scale per token.
+// Bytes of the GEMM's operand for n tokens (one f16 term an activation, or two when an f32 one travels as value and
+// remainder): the f16 rows, the sub-block means, and one f32 scale per token.
 size_t gemm_operand_bytes(size_t cols, size_t n, int split) {
     const size_t terms = split ? 2 : 1;
     return (terms * cols + cols / 256 * 16) * n * sizeof(__half) + ((n * sizeof(float) + 15) & ~size_t(15));
@@ -268,7 +268,9 @@ __device__ __noinline__ Terms terms_clamped(float f0, float f1, float f2, float 
 }
 
 // A block per token row, or a cluster of up to eight; the row in chunks of THREADS * 4 activations (four a
-// thread), dealt to the blocks in turn, R of them a block, and held in registers until its largest magnitude is known.
+// thread), dealt to the blocks in turn, R of them a block, and held in registers until its largest magnitude is known
+// (all but a few of the longer forms': R = 9, rows of 17408, spills 144 bytes a thread, 232 to 240 with the norm; R = 5,
+// rows of 5120, 24 to 48).
 //   NORM: the row is first normalized by its root mean square and multiplied
 //   by `weight` (Cpu::rmsnorm, gpu/cpu.rs:157-166: v * (scale * w) with
 //   scale = 1 / sqrt(sum(v^2) / dim + eps)); the f32 result goes to `xout`.
@@ -282,10 +284,9 @@ __device__ __noinline__ Terms terms_clamped(float f0, float f1, float f2, float 
 // maximum, was measured to slow the tensor-core kernel by half: the same
 // kernel on larger operand magnitudes runs into the power limit earlier.)
 template <bool NORM, bool SPLIT, int THREADS, int R>
-__global__ void __launch_bounds__(THREADS, THREADS == 512 ? (R > 9 ? 1 : 2) : R > 3 ? 5 : 6) gemm_operand_kernel(const float *x, const float *__restrict__ weight, float eps, float *xout,
-                                                               size_t cols, size_t units, int cluster, size_t n,
-                                                               __half *__restrict__ x16, __half *__restrict__ means,
-                                                               float *__restrict__ tok_scale) {
+__global__ void __launch_bounds__(THREADS, THREADS == 512 ? (R > 9 ? 1 : 2) : R > 3 ? 5 : 6)
+gemm_operand_kernel(const float *x, const float *__restrict__ weight, float eps, float *xout, size_t cols, size_t units, int cluster, size_t n,
+                    __half *__restrict__ x16, __half *__restrict__ means, float *__restrict__ tok_scale) {
     if (cluster > 1) cluster_arrive();
     // as the small-M prologues: let the product's kernel begin (it streams weights first),
     // wait for the kernel ahead, which may still read the operand or write x
@@ -304,7 +305,8 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? (R > 9 ? 1 : 2) : R 
         float4 w[R];      // (fetched ahead of the sum where the registers last)
         constexpr bool AHEAD = R <= 3;
 #pragma unroll
-        for (int r = 0; r < R && AHEAD; r++) w[r] = place(r) < cols ? *reinterpret_cast<const float4 *>(weight + place(r)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int r = 0; r < R && AHEAD; r++)
+            w[r] = place(r) < cols ? *reinterpret_cast<const float4 *>(weight + place(r)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         float ssq = 0.0f;
 #pragma unroll
         for (int r = 0; r < R; r++) ssq += (v[r].x * v[r].x + v[r].y * v[r].y) + (v[r].z * v[r].z + v[r].w * v[r].w);

@@ -140,7 +140,7 @@ DWIM_B200_API int dwim_b200_touch_bf16(dwim_b200_ctx *ctx, dwim_b200_buffer *buf
  * eight tokens; the small-M kernel's digit planes are exact either way).
  * EXACT, the default: a token travels as two f16 terms, value and rounding
  * remainder, and the product's error stays near 2e-6 of its rms; twice the
- * tensor-core work of a bf16-exact buffer.  F16: one column, the activation
+ * tensor-core work of a bf16-exact buffer.  F16: one term, the activation
  * rounded to f16 after the token's power-of-two scaling, which is the
  * precision of the reference's own CUDA device (`halves`,
  * gpu/cuda/mod.rs:313-384): rms error about 3e-4 of the result's magnitude,

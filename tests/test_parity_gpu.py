@@ -701,7 +701,7 @@ def test_bf16_matmul_matches_cpu(dev, oracle):
 @pytest.mark.parametrize("rows,cols,n", [(1, 8, 1), (33, 2048, 3), (5, 2056, 8), (96, 5120, 16), (3, 8, 17), (33, 520, 64), (31, 72, 65), (33, 136, 128),
                                          (96, 5120, 129)])
 def test_bf16_matmul_edges(dev, oracle, rows, cols, n):
-    """Both kernels at the edges of their tiles (rows of 32, tokens of 32 or 64, K of 64 dealt to eight
+    """Both kernels at the edges of their tiles (rows of 32, tokens of 32, K of 64 dealt to eight
     blocks), with the three epilogues.  fp32 sums of at most 5120 products: 1e-5 of the result's
     root mean square is sixteen times 2^-24 * sqrt(5120)."""
     from dwim_b200 import Tensor
@@ -844,7 +844,7 @@ def test_config2_gemm_full_size(dev, oracle, rows, cols, n):
 
 @pytest.mark.parametrize("n", [17, 33, 130, 300])
 def test_gemm_bf16_token_counts(dev, oracle, n):
-    """bf16 activations (one f16 column per token) in tiles of 32, 64 and 192 or
+    """bf16 activations (one f16 term) in tiles of 32, 64 and 192 or
     256 columns of the tensor-core kernel, ragged against each."""
     rng = np.random.default_rng(3000 + n)
     rows, cols = 1000, 5120
@@ -1246,8 +1246,8 @@ def test_gemm_activations_at_the_ends_of_f32(dev, oracle, fmt, n):
 
 @pytest.mark.parametrize("bf16", [True, False])
 def test_gemm_fused_epilogues_at_256_columns(dev, oracle, bf16):
-    """matmul_add and swiglu through the 256-column kernel (300 tokens of bf16
-    input, or 150 of f32 travelling as two columns each)."""
+    """matmul_add and swiglu of 300 tokens of bf16 input, or 150 of f32 in two terms (in tiles of 192 columns, whose wave is
+    the shorter one here; of 256: test_tiles_of_256_columns)."""
     rng = np.random.default_rng(3100 + bf16)
     rows, cols, n = 1030, 5120, 300 if bf16 else 150
     gate = oracle.quantize("q4_k", (0.02 * rng.standard_normal((rows, cols))).astype(np.float32))
@@ -1270,12 +1270,39 @@ def test_gemm_fused_epilogues_at_256_columns(dev, oracle, bf16):
     assert max_rel_err(got - res, want - res) <= 1e-4
 
 
+@pytest.mark.parametrize("fmt", FORMATS)
+@pytest.mark.parametrize("bf16", [True, False])
+def test_tiles_of_256_columns(dev, oracle, fmt, bf16):
+    """76 row tiles by 255 tokens: one wave in tiles of 256 columns and two of 192, so these take it; the three epilogues,
+    ragged rows and tokens.  2e-5 of the result's root mean square, as for the narrower tiles."""
+    rng = np.random.default_rng(3200 + bf16)
+    rows, cols, n = 9601, 512, 255
+    weight, w, other, w2 = random_pair(dev, oracle, fmt, rows, cols, rng)
+    x = rng.standard_normal((n, cols)).astype(np.float32)
+    xb = dev.buffer(x)
+    if bf16:
+        bits = oracle.to_bf16(x)
+        dev.write_bf16(xb, bits)
+        x = oracle.bf16(bits).reshape(n, cols)
+    want = x.astype(np.float64) @ w.T
+    bar = 2e-5 * np.sqrt((want ** 2).mean())
+    out, scratch, res = dev.alloc(n * rows), dev.alloc(n * rows), rng.standard_normal((n, rows)).astype(np.float32)
+    acc = dev.buffer(res)
+    dev.matmul(out, weight, xb)
+    assert np.abs(dev.read(out).reshape(n, rows) - want).max() <= bar
+    dev.matmul_add(acc, weight, xb)
+    assert np.abs(dev.read(acc).reshape(n, rows) - (want + res)).max() <= bar + 1e-6
+    dev.swiglu(out, weight, other, xb, scratch)
+    silu = silu_times(want, x.astype(np.float64) @ w2.T)
+    assert np.abs(dev.read(out).reshape(n, rows) - silu).max() <= 4 * bar * max(1.0, np.abs(want).max())
+
+
 @pytest.mark.parametrize("fmt", ["q6_k", "q8_0"])
 @pytest.mark.parametrize("n,bf16", [(12, False), (33, False), (65, True), (130, False), (300, True)])
 def test_dense_pair_gemm_for_q6_k_and_q8_0(dev, oracle, fmt, n, bf16):
     """Above the small-M kernel's eight tokens Q6_K and Q8_0 go in groups of eight
-    (up to 64 tokens) and then through the dense kernel, whose weights are pairs of
-    f16 terms: both tile widths, ragged rows, both activation forms, fused epilogues.
+    (up to 24 tokens by f32 activations, 64 by bf16) and then through the dense kernel, whose weights are pairs of
+    f16 terms: its narrower tiles, ragged rows, both activation forms, fused epilogues.
     Against the oracle's fp32 sums: 2e-5 for either path (4.2e-6 of the result's root
     mean square is the most the dense kernel was measured to be off, at any K)."""
     rng = np.random.default_rng(4000 + n)
@@ -1424,7 +1451,7 @@ def test_shared_result_of_two_ranks_on_one_gpu(dev, oracle):
 
 
 def test_activation_precision_f16(dev, oracle):
-    """f32 activations as one f16 column on request (the reference device's own precision, `halves`,
+    """f32 activations as one f16 term on request (the reference device's own precision, `halves`,
     gpu/cuda/mod.rs:313-384): it passes the reference's gate for that device (rms error below 1e-3 of
     the typical magnitude and the worst below 1e-2, gpu/tests.rs:198-211), not this library's 1e-3
     on the worst element, and is really another path than the exact one."""
