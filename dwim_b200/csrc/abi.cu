@@ -24,15 +24,29 @@ bool gemm_takes(const WeightView &w, size_t n, int terms);
 int gemm_large(dwim_b200_ctx *ctx, const WeightView &w, const __half *operand, size_t n, int terms, const OutSpec &out,
                const float *aux, int epilogue, size_t whole);
 
+// Graphs that were captured with the shadow read and write it wherever they run: a longer one leaves it to them then, and
+// is twice as long at least, so that there are few of them.
 int reserve_shadow(dwim_b200_ctx *ctx, dwim_b200_buffer *b, size_t need) {
     if (need <= b->shadow_cap) return 0;
-    if (b->shadow) {
+    b->shadow_kind = SHADOW_NONE;
+    if (b->shadow && b->replayed.kind == SHADOW_NONE) {
         DWIM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         cudaFree(b->shadow);
         b->shadow = nullptr;
         b->shadow_cap = 0;
     }
-    DWIM_CUDA(ctx, cudaMalloc(&b->shadow, need));
+    if (b->shadow && need < 2 * b->shadow_cap) need = 2 * b->shadow_cap;
+    void *longer = nullptr;
+    DWIM_CUDA(ctx, cudaMalloc(&longer, need));
+    if (b->shadow) {
+        ReplayedShadow *left = new (std::nothrow) ReplayedShadow{b->shadow, b->left};
+        if (!left) {
+            cudaFree(longer);
+            return fail(ctx, DWIM_B200_ENOMEM, "out of host memory");
+        }
+        b->left = left;
+    }
+    b->shadow = longer;
     b->shadow_cap = need;
     return 0;
 }
@@ -347,6 +361,11 @@ int dwim_b200_buffer_free(dwim_b200_ctx *ctx, dwim_b200_buffer *buf) {
     if (buf->sh_world) shared_release(buf);
     if (buf->owned && buf->data) cudaFree(buf->data);
     if (buf->shadow) cudaFree(buf->shadow);
+    while (ReplayedShadow *left = buf->left) {
+        cudaFree(left->array);
+        buf->left = left->next;
+        delete left;
+    }
     if (buf->groups) cudaFree(buf->groups);
     for (void *operand : buf->operands)
         if (operand) cudaFree(operand);

@@ -27,6 +27,11 @@ struct ShadowForm {
     size_t cols = 0, len = 0;
 };
 
+struct ReplayedShadow {
+    void *array;
+    ReplayedShadow *next;
+};
+
 constexpr int DWIM_MAX_WORLD = 8;
 
 struct dwim_b200_buffer {
@@ -50,6 +55,7 @@ struct dwim_b200_buffer {
     int shadow_split = 0;        // f16 terms of an activation less one
     unsigned long long shadow_capture = 0;   // the stream capture that the conversion is part of; 0: it was launched
     ShadowForm replayed;         // what captured graphs make there whenever they run
+    ReplayedShadow *left = nullptr;      // shorter shadows that graphs were captured with, kept to the buffer's end
     // The digit planes of several groups of eight tokens (products of Q6_K and Q8_0 by nine tokens and more), where the
     // shadow holds fewer.  Allocated once and kept to the buffer's end.
     void *groups = nullptr;

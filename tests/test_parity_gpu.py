@@ -1162,6 +1162,57 @@ def test_a_captured_conversion_is_not_taken_for_a_made_one(oracle, fmt, n):
         d.close()
 
 
+@pytest.mark.parametrize("fmt", FORMATS)
+@pytest.mark.parametrize("n", [3, 16])
+def test_a_graph_keeps_the_operand_that_it_reads(oracle, fmt, n):
+    """A product captured at a few tokens, then eager ones of more and more, whose operand is longer: the graph's own stays
+    where it is, whatever is allocated after it."""
+    import torch
+    from dwim_b200 import B200, Tensor
+    stream = torch.cuda.Stream()
+    d = B200(0, stream=stream.cuda_stream)
+    try:
+        rng = np.random.default_rng(89)
+        rows, cols, most = 96, 2048, 300
+        blocks = oracle.quantize(fmt, (0.02 * rng.standard_normal((rows, cols))).astype(np.float32))
+        weight = d.upload(Tensor(fmt, (rows, cols), blocks))
+        x = rng.standard_normal((most, cols)).astype(np.float32)
+        want = oracle.matmul(fmt, blocks, rows, cols, x).reshape(most, rows)
+        xb, out = d.buffer(x), d.alloc(most * rows)
+
+        def at(tokens):
+            d.resize(xb, tokens * cols)
+            d.resize(out, tokens * rows)
+
+        def right(tokens):
+            got = d.read(out).reshape(tokens, rows)
+            d.write(out, np.zeros(tokens * rows, np.float32))
+            return max_rel_err(got, want[:tokens]) <= 2e-5
+
+        at(n)
+        d.matmul(out, weight, xb)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            d.matmul(out, weight, xb)
+        others = []
+        for tokens in (n + 6, 100, most):
+            at(tokens)
+            d.matmul(out, weight, xb)
+            assert right(tokens)
+            others += [d.buffer(np.full(1 << k, 7.0, np.float32)) for k in range(12, 20)]
+            at(n)
+            with torch.cuda.stream(stream):
+                graph.replay()
+            assert right(n), tokens
+            at(tokens)
+            d.matmul(out, weight, xb)
+            assert right(tokens)
+        assert all((d.read(o) == 7.0).all() for o in others)
+        del graph
+    finally:
+        d.close()
+
+
 @pytest.mark.parametrize("fmt", ["q6_k", "q8_0"])
 def test_dense_kernel_gives_its_bits_whatever_memory_there_is(oracle, fmt):
     """The products that the groups of eight tokens could take as well: captured before any eager one, by a buffer that
